@@ -1,0 +1,36 @@
+"""Lists around the lengths at which the passes change how they walk them:
+the backward takes a list in stretches of 128 entries, each from the state
+the forward left there, so lists one entry short of, at and past whole
+stretches are compared with the oracle's adjoint, with pixels that end before,
+inside and after a stretch."""
+import numpy as np
+import pytest
+
+from radiance_meshes_b200.camera import pinhole_tcam
+from test_gpu_backward import _run
+
+pytestmark = pytest.mark.gpu
+
+
+def _stack(n, density, seed):
+    """n thin tets one behind the other along the view axis, wider than most
+    of the image, each shifted sideways a little."""
+    rng = np.random.default_rng(seed)
+    z = 2.0 + 0.02 * np.arange(n)[:, None]
+    s = z * rng.uniform(0.3, 1.2, size=(n, 1))
+    cx, cy = (z * rng.uniform(-0.2, 0.2, size=(n, 1)) for _ in range(2))
+    corners = [(-1, -1, 0.0), (1, -1, 0.0), (0, 1.2, 0.0), (0.0, 0.0, 0.015)]
+    verts = np.concatenate([np.concatenate([cx + a * s, cy + b * s, z + dz], 1)[:, None] for a, b, dz in corners], 1)
+    idx = np.arange(4 * n, dtype=np.int32).reshape(n, 4)[:, [1, 0, 2, 3]]
+    cv = np.concatenate([density * rng.uniform(0.5, 1.5, (n, 1)), rng.uniform(0, 1, (n, 3)),
+                         rng.normal(0, 0.1, (n, 3))], 1)
+    return verts.reshape(-1, 3).astype(np.float32), np.ascontiguousarray(idx), cv.astype(np.float32)
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 256, 257, 400])
+@pytest.mark.parametrize("density", [0.3, 6.0])  # every pixel reaches the end; most end on the way
+def test_backward_over_stretches(cuda, n, density):
+    verts, idx, cv = _stack(n, density, n)
+    tcam = pinhole_tcam((0.0, 0.0, 0.0), (0.0, 0.0, 1.0), 11, 13, 30.0, tile_size=8)
+    jitter = np.random.default_rng(n).uniform(0, 1, (11, 13, 2)).astype(np.float32)
+    _run(verts, idx, cv, tcam, jitter, "linear", seed=n, check_f64=False, hit_masks=True)
