@@ -107,6 +107,34 @@ template <bool PLANES>
 __device__ __forceinline__ Isect intersect(const float4* __restrict__ q, f3 o, f3 d) {
     const f3 a0 = xyz(q[4]) - o;
     const f3 a1 = xyz(q[5]) - o;
+    if (!PLANES) {
+        // No plane index wanted: with no plane nearly parallel to the ray
+        // (the common case) the updates are one maximum or minimum per plane.
+        float dist[4], den[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const f3 n = xyz(q[i]);
+            dist[i] = -dot3(n, i == 3 ? a1 : a0);
+            den[i] = dot3(n, d);
+        }
+        const float least = fminf(fminf(fabsf(den[0]), fabsf(den[1])), fminf(fabsf(den[2]), fabsf(den[3])));
+        if (!(least < 1e-10f)) {
+            float te = -1e30f, tx = 1e30f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float tp = -dist[i] / den[i];
+                te = fmaxf(te, den[i] < 0.f ? tp : -1e30f);
+                tx = fminf(tx, den[i] < 0.f ? 1e30f : tp);
+            }
+            Isect r;
+            r.te = te;
+            r.tx = tx;
+            r.geo = !(te > tx) && !(tx <= 0.f);
+            r.enter = fmaxf(te, 0.f);
+            r.exit = fmaxf(tx, r.enter);
+            return r;
+        }
+    }
     float te = -1e30f, tx = 1e30f, dene = 1.f, denx = 1.f;
     int ie = -1, ix = -1;
     bool miss = false;
@@ -158,11 +186,11 @@ __device__ __forceinline__ Weights seg_weights(float x) {
     w.alpha = __expf(-x);
     if (x < 0.25f) {
         // w1 = x/2 - x^2/6 + x^3/24 - x^4/120 + x^5/720 - x^6/5040 + x^7/40320
-        w.w1 = x * (0.5f + x * (-1.0f / 6.0f + x * (1.0f / 24.0f + x * (-1.0f / 120.0f + x * (1.0f / 720.0f +
-                 x * (-1.0f / 5040.0f + x * (1.0f / 40320.0f)))))));
+        w.w1 = x * fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, 1.0f / 40320.0f, -1.0f / 5040.0f), 1.0f / 720.0f),
+                                            -1.0f / 120.0f), 1.0f / 24.0f), -1.0f / 6.0f), 0.5f);
         // w0 = x/2 - x^2/3 + x^3/8 - x^4/30 + x^5/144 - x^6/840 + x^7/5760
-        w.w0 = x * (0.5f + x * (-1.0f / 3.0f + x * (0.125f + x * (-1.0f / 30.0f + x * (1.0f / 144.0f +
-                 x * (-1.0f / 840.0f + x * (1.0f / 5760.0f)))))));
+        w.w0 = x * fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, 1.0f / 5760.0f, -1.0f / 840.0f), 1.0f / 144.0f),
+                                            -1.0f / 30.0f), 0.125f), -1.0f / 3.0f), 0.5f);
     } else {
         const float phi = __fdividef(1.0f - w.alpha, x);
         w.w0 = phi - w.alpha;
@@ -463,6 +491,16 @@ struct EntryResult {
     float rgb[3];
 };
 
+// x / 3 correctly rounded for every x >= 0 (one residual correction of the
+// product with the rounded reciprocal; equal to the division on all
+// non-negative floats, checked exhaustively), a third of its instructions.
+__device__ __forceinline__ float third(float x) {
+    const float r3 = 1.0f / 3.0f;
+    const float q = x * r3;
+    const float y = fmaf(fmaf(-3.0f, q, x), r3, q);
+    return x <= 3.402823466e38f ? y : x;
+}
+
 __device__ __forceinline__ EntryResult eval_entry(const float4* __restrict__ q, f3 o, f3 d) {
     EntryResult r;
     const Isect is = intersect<false>(q, o, d);
@@ -478,7 +516,7 @@ __device__ __forceinline__ EntryResult eval_entry(const float4* __restrict__ q, 
         integrate(q, o, d, is.enter, is.exit, s);
         r.a = s.a;
         r.m1 = density * (is.exit + is.enter) / 2.0f;
-        r.d4 = density * density * s.dt / 3.0f;
+        r.d4 = third(density * density * s.dt);
 #pragma unroll
         for (int k = 0; k < 3; ++k) r.rgb[k] = s.rgb[k];
     }
@@ -553,26 +591,110 @@ __device__ __forceinline__ void fwd_dense_item(int tile, int sub, const int32_t*
     }
 }
 
+// A bundle of rays from one point: every ray direction is a positive multiple
+// of u * r0 + v * r1 + r2 for the camera axes r0, r1, r2, with (u, v) inside
+// the box.
+struct Bundle {
+    float u0, u1, v0, v1;
+};
+
+// Whether a list entry can be hit by a ray of the bundle.  Seen from the
+// camera position c, a hit ray d satisfies, for each face i that c lies
+// outside of and each face j that c lies inside of (the silhouette),
+//     g = dot(dist_j n_i - dist_i n_j, d) >= 0,  dist = dot(n, c - v):
+// the quotients of eval_entry order as te <= tx exactly when every such g is
+// not negative, and moving the ray's start along d leaves g alone.  g is
+// linear in d, so its largest value over the box decides.  The margin covers
+// the rounding of dist, n.d and of the ray origin in eval_entry (below 60
+// units of 2^-24 of |n_i| |n_j| times the distance scale A), planes it skips
+// as parallel (|n.d| < 1e-10) and axes orthonormal to 2e-6 only; faces whose
+// side of c is within rounding take no part.  So an entry that is dropped is
+// one for which eval_entry returns a miss for every ray of the bundle.
+// r: the entry's record; inv_z: 1 / the least d.r2 of the unit directions.
+__device__ __forceinline__ bool entry_reaches(const float4* __restrict__ r, const rm_camera& cam, const Bundle& bd,
+                                              float inv_z) {
+    const f3 c = {cam.cam_pos[0], cam.cam_pos[1], cam.cam_pos[2]};
+    const float* M = cam.world_view;
+    const f3 a0 = xyz(__ldg(r + 4)) - c, a1 = xyz(__ldg(r + 5)) - c;
+    const float A = fmaxf(fabsf(a0.x) + fabsf(a0.y) + fabsf(a0.z), fabsf(a1.x) + fabsf(a1.y) + fabsf(a1.z)) +
+                    (fabsf(c.x) + fabsf(c.y) + fabsf(c.z)) + cam.min_t;
+    float dist[4], N[4];
+    f3 m[4];
+    uint32_t outside = 0, inside = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const f3 n = xyz(__ldg(r + i));
+        dist[i] = -dot3(n, i == 3 ? a1 : a0);
+        N[i] = fabsf(n.x) + fabsf(n.y) + fabsf(n.z);
+        const float sure = fmaf(2e-6f * N[i], A, 1e-9f * (1.0f + cam.min_t));
+        outside |= dist[i] > sure ? 1u << i : 0u;
+        inside |= dist[i] < -sure ? 1u << i : 0u;
+        m[i] = {dot3(mk3(M[0], M[1], M[2]), n), dot3(mk3(M[4], M[5], M[6]), n), dot3(mk3(M[8], M[9], M[10]), n)};
+    }
+    bool reach = true;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+#pragma unroll
+        for (int j = i + 1; j < 4; ++j) {
+            const bool ij = ((outside >> i) & (inside >> j) & 1u) != 0u, ji = ((outside >> j) & (inside >> i) & 1u) != 0u;
+            if (!ij && !ji) continue;
+            const float di = ij ? dist[i] : -dist[i], dj = ij ? dist[j] : -dist[j];
+            const f3 e = {fmaf(dj, m[i].x, -(di * m[j].x)), fmaf(dj, m[i].y, -(di * m[j].y)),
+                          fmaf(dj, m[i].z, -(di * m[j].z))};
+            const float P = N[i] * N[j] * A;
+            const float margin = fmaf(8e-6f, P, fmaf(1e-5f, fabsf(e.x) + fabsf(e.y) + fabsf(e.z),
+                                                     2e-10f * A * (N[i] + N[j])));
+            const float g = e.z + fmaxf(e.x * bd.u0, e.x * bd.u1) + fmaxf(e.y * bd.v0, e.y * bd.v1);
+            if (P > 1e-25f && P < 1e30f && fmaf(margin, inv_z, g) < 0.f) reach = false;
+        }
+    }
+    return reach;
+}
+
 // Pair forward item: a strip of PX pixels (PX / tile_width rows of one tile)
-// handled by NT >= PX threads.  Threads 0..PX-1 own one pixel each.  Per batch
-// of B list entries the records are staged in shared memory, the still-active
-// pixels are compacted into slots, and all NT threads evaluate the
-// (entry, slot) pairs -- a warp takes one entry at a time (its record is read
-// as a broadcast) and its lanes take the slots -- writing each pair's a, m1,
-// D4 increment and colour to shared memory.  Each owner then folds its
-// pixel's results in list order: this sequential part is a handful of adds
-// per entry, so a pixel whose ray crosses thousands of tets no longer runs
-// the whole intersection/integration chain on one thread.  The fold uses
-// exactly the arithmetic of the one-thread-per-pixel walk, so n_contributors,
-// log T and the distortion moments are unchanged bit for bit.
+// handled by NT >= PX threads, or (quarter >= 0) one 4x4-pixel quarter of an
+// 8x8 strip.  The first threads own one pixel each.
+//
+// The list is taken in blocks of RB entries.  A staging warp loads a block,
+// one entry per lane, drops the entries that no ray of the strip can hit
+// (entry_reaches, and those of zero density) and writes the records of the
+// rest to shared memory, as many blocks per batch as fill the B records.  The
+// still-active pixels are compacted into slots and all NT threads evaluate
+// the (entry, slot) pairs -- a warp takes one entry at a time (its record is
+// read as a broadcast) and its lanes take 32 slots, or groups of lanes take
+// entries of their own where fewer are active -- writing each pair's a, m1,
+// D4 increment and colour to shared memory (zeros for a miss).  Each owner
+// then folds its pixel's results in list order while the other warps stage
+// the next batch.  The fold is exactly the arithmetic of the
+// one-thread-per-pixel walk (adding a miss's zeros changes no bit), so
+// n_contributors, log T and the distortion moments are unchanged bit for bit.
+//
+// Bound: instruction issue in the evaluation (about 200 instructions for 32
+// pairs); for the few lists of thousands of entries the chain of batches,
+// hence the quarters and a fold whose only serial part is one add per entry.
+template <int PX, int NT, int B>
+struct PairShape {
+    static constexpr int kOwnWarps = (PX + 31) / 32;
+    static constexpr int kWarps = NT / 32;
+    static constexpr int kStageWarps = kWarps - kOwnWarps;
+    static constexpr int RB = B < 32 ? B : 32;
+};
+
 template <int PX, int B>
 struct FwdPairSmem {
-    float4 srec[B][kRecFloat4];
-    float dens[2][B];      // densities of the batch being folded and of the one being staged
-    float ray[6][PX];      // o, d of each slot (structure of arrays)
+    static constexpr int kMaxStage = 6;
+    float4 srec[B][kRecFloat4 + 1];  // padded: a warp writes whole records, one per lane
     float res[6][B][PX];   // a (0: miss), m1, d4, r, g, b per (entry, slot)
+    float ray[6][PX];      // o, d of each slot (structure of arrays)
+    float dens[2][B];      // densities of the batch being folded and of the one being staged
+    uint8_t pos[2][B];     // list offset of each record inside its block
+    uint32_t bal[kMaxStage];           // entries kept of the blocks a staging round looked at
+    int32_t start[2][kMaxStage + 1];   // first record of each block of the batch; [n_blk]: their count
+    int32_t n_blk[2];
+    float bnd[2][(PX + 31) / 32][4];   // (min u, max u, min v, max v) of each owner warp's active pixels
+    float z_min[(PX + 31) / 32];
+    float uv[2][PX];       // each owner's (u, v), by owner thread
     int32_t warp_base[(PX + 31) / 32];
-    float pray[6][PX];     // each owner's own ray, by owner thread (kept out of registers)
 };
 
 template <int PX, int B>
@@ -585,141 +707,274 @@ __device__ __forceinline__ void store_result(FwdPairSmem<PX, B>& S, int j, int s
     S.res[5][j][sl] = r.rgb[2];
 }
 
-// Stages batch [base, base + n) into srec (and its densities into dens[buf])
-// with threads t, t + nt, ...: one float4 of one record each, the thread
-// loading the entry's id itself.
-template <int PX, int B>
-__device__ __forceinline__ void stage_pair_batch(FwdPairSmem<PX, B>& S, int buf, int base, int n,
+// Stages a batch from block `blk` of the list [x, y) on with the staging
+// warps (sw: this warp's number among them): looks at up to `tries` blocks,
+// one per warp, and keeps as many as fit in B records (at least one).
+template <int PX, int NT, int B>
+__device__ __forceinline__ void stage_pair_batch(FwdPairSmem<PX, B>& S, int buf, int rd, int blk, int tries, int x, int y,
                                                  const int32_t* __restrict__ ids, const float4* __restrict__ recs,
-                                                 const Queue& lq, int t, int nt) {
-    for (int k = t; k < n * kRecFloat4; k += nt) {
-        const int j = k >> 3, c = k & 7;
-        const float4 r = record_part(recs, list_id(ids, base + j, lq), c);
-        S.srec[j][c] = r;
-        if (c == 0) S.dens[buf][j] = r.w;
+                                                 const rm_camera& cam, float inv_z, const Queue& lq, int sw, int lane) {
+    using Sh = PairShape<PX, NT, B>;
+    tries = min(tries, (y - x - blk * Sh::RB + Sh::RB - 1) / Sh::RB);
+    bool keep = false;
+    uint32_t bal = 0;
+    const float4* r = recs;
+    if (sw < tries) {
+        const int e = x + (blk + sw) * Sh::RB + lane;
+        int32_t g = -1;
+        if (lane < Sh::RB && e < y) g = list_id(ids, e, lq);
+        if (g >= 0) {
+            r = recs + (int64_t)kRecFloat4 * g;
+            keep = __ldg(&r[0].w) > 0.f;  // a density of zero hits nothing
+            if (keep && inv_z > 0.f) {
+                Bundle bd = {S.bnd[rd][0][0], S.bnd[rd][0][1], S.bnd[rd][0][2], S.bnd[rd][0][3]};
+#pragma unroll
+                for (int w = 1; w < Sh::kOwnWarps; ++w)
+                    bd = {fminf(bd.u0, S.bnd[rd][w][0]), fmaxf(bd.u1, S.bnd[rd][w][1]), fminf(bd.v0, S.bnd[rd][w][2]),
+                          fmaxf(bd.v1, S.bnd[rd][w][3])};
+                keep = entry_reaches(r, cam, bd, inv_z);
+            }
+        }
+        bal = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) S.bal[sw] = bal;
+    }
+    if (Sh::kStageWarps > 1)
+        asm volatile("bar.sync 1, %0;" ::"r"(Sh::kStageWarps * 32) : "memory");
+    else
+        __syncwarp();
+    // how many blocks fit, and this warp's first record
+    int m = 0, n = 0, mine = 0;
+    for (; m < tries; ++m) {
+        const int k = __popc(S.bal[m]);
+        if (n + k > B) break;
+        if (m == sw) mine = n;
+        if (sw == 0 && lane == 0) S.start[buf][m] = n;
+        n += k;
+    }
+    if (sw == 0 && lane == 0) {
+        S.start[buf][m] = n;
+        S.n_blk[buf] = m;
+    }
+    if (sw < m && keep) {
+        const int j = mine + __popc(bal & ((1u << lane) - 1u));
+#pragma unroll
+        for (int c = 0; c < kRecFloat4; ++c) S.srec[j][c] = __ldg(r + c);
+        S.dens[buf][j] = __ldg(&r[0].w);
+        S.pos[buf][j] = (uint8_t)lane;
     }
 }
 
+// One entry of the fold, hit or miss (a = 0, every increment zero).
+__device__ __forceinline__ void fold_any(PixelState& st, float a, float m0, float m1, float d4, float r, float g,
+                                         float b) {
+    const float T = __expf(st.logT);
+    st.c[0] = fmaf(r, T, st.c[0]);
+    st.c[1] = fmaf(g, T, st.c[1]);
+    st.c[2] = fmaf(b, T, st.c[2]);
+    st.logT = st.logT - a;
+    const float D2 = st.D[2], D3 = st.D[3];
+    st.D[0] = fmaf(2.0f * m1, D2, st.D[0]);
+    st.D[1] = fmaf(2.0f * m0, D3, st.D[1]);
+    st.D[2] = D2 + m0;
+    st.D[3] = D3 + m1;
+    st.D[4] = st.D[4] + d4;
+}
+
 template <int PX, int NT, int B>
-__device__ __forceinline__ void fwd_pair_item(int tile, int sub, const int32_t* __restrict__ ids,
+__device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, const int32_t* __restrict__ ids,
                                          const int2* __restrict__ ranges, const float4* __restrict__ recs,
                                          const float2* __restrict__ jitter, const rm_camera& cam,
                                          float4* __restrict__ out_img, float* __restrict__ out_dist,
                                          int32_t* __restrict__ out_nc, FwdPairSmem<PX, B>& S,
                                          const HitMasks& hm, int subs, int gtile, const Queue& lq) {
-    static_assert(PX <= 64 && NT >= 64, "a lane evaluates at most two slots");
+    using Sh = PairShape<PX, NT, B>;
+    static_assert(PX <= 64 && NT >= 64, "two owner warps at most");
+    static_assert(Sh::kStageWarps >= 1 && Sh::kStageWarps <= FwdPairSmem<PX, B>::kMaxStage, "staging warps");
     constexpr bool kMasks = PX == 64 && B % 32 == 0;
-    constexpr unsigned kOwnMask = WarpShape<PX>::kMask;
-    constexpr int kWarps = NT / 32;
-    constexpr int kOwnThreads = (PX + 31) / 32 * 32;  // the owners' warps; the rest stage during the fold
-    static_assert(NT > kOwnThreads, "staging needs warps besides the owners'");
+    constexpr int RB = Sh::RB;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const bool owner = tid < PX;
+    const bool own_warp = warp < Sh::kOwnWarps;
+    const bool owner = tid < (quarter >= 0 ? 16 : PX);
+    const int2 rg = __ldg(ranges + tile);
+    // the owner's pixel of the strip
+    const int p = quarter < 0 ? tid : ((quarter >> 1) * 4 + (tid >> 2)) * 8 + (quarter & 1) * 4 + (tid & 3);
     const int tx = tile % cam.grid_width, ty = tile / cam.grid_width;
     int lx, ly;
-    strip_pixel<PX>(cam, sub, tid, lx, ly);
+    strip_pixel<PX>(cam, sub, p, lx, ly);
     const int px = tx * cam.tile_width + lx, py = ty * cam.tile_height + ly;
     const bool inside = owner && px < cam.image_width && py < cam.image_height;
     const int64_t pix = (int64_t)py * cam.image_width + px;
-    f3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f};
-    if (inside) {
-        const float2 j = __ldg(jitter + pix);
-        make_ray(cam, px, py, j.x, j.y, o, d);
-    }
-    if (owner) {
-        S.pray[0][tid] = o.x; S.pray[1][tid] = o.y; S.pray[2][tid] = o.z;
-        S.pray[3][tid] = d.x; S.pray[4][tid] = d.y; S.pray[5][tid] = d.z;
-    }
-    const int2 rg = __ldg(ranges + tile);
     PixelState st = {{0.f, 0.f, 0.f}, 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}};
-    int32_t nc = 0;
-    bool active = inside;
-    // The first batch is staged by all threads; each later one by the
-    // non-owner warps while the owners fold the batch before it (srec is no
-    // longer read by then: the fold reads the densities kept in dens[cur]).
-    stage_pair_batch(S, 0, rg.x, min(B, rg.y - rg.x), ids, recs, lq, tid, NT);
-    int rank = 0;  // the owner's rank among the active pixels of its warp
-    if (owner) {
-        const unsigned bal = __ballot_sync(kOwnMask, active);
+    int32_t nc = rg.y - rg.x;  // entries walked: all of them unless log T runs out
+    bool active = inside && nc > 0;
+    int rank = 0, slot = tid;  // rank among the warp's active pixels; where the pixel's ray and results lie
+    const float* M = cam.world_view;
+    // Box of the active pixels' (u, v), per owner warp.
+    auto bounds = [&](int buf, bool in) {
+        const float u = in ? S.uv[0][tid] : 0.f, v = in ? S.uv[1][tid] : 0.f;
+        float u0 = in ? u : 3e38f, u1 = in ? u : -3e38f, v0 = in ? v : 3e38f, v1 = in ? v : -3e38f;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            u0 = fminf(u0, __shfl_xor_sync(0xffffffffu, u0, o));
+            u1 = fmaxf(u1, __shfl_xor_sync(0xffffffffu, u1, o));
+            v0 = fminf(v0, __shfl_xor_sync(0xffffffffu, v0, o));
+            v1 = fmaxf(v1, __shfl_xor_sync(0xffffffffu, v1, o));
+        }
+        if (lane == 0) {
+            S.bnd[buf][warp][0] = u0;
+            S.bnd[buf][warp][1] = u1;
+            S.bnd[buf][warp][2] = v0;
+            S.bnd[buf][warp][3] = v1;
+        }
+    };
+    auto rank_active = [&]() {
+        const unsigned bal = __ballot_sync(0xffffffffu, active);
         if (lane == 0) S.warp_base[warp] = __popc(bal);
-        rank = __popc(bal & ((1u << lane) - 1u));
+        return __popc(bal & ((1u << lane) - 1u));
+    };
+    if (own_warp) {
+        f3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f};
+        float z = 3e38f;
+        rank = rank_active();
+        if (active) {
+            const float2 j = __ldg(jitter + pix);
+            make_ray(cam, px, py, j.x, j.y, o, d);
+            z = dot3(mk3(M[8], M[9], M[10]), d);
+            S.uv[0][tid] = dot3(mk3(M[0], M[1], M[2]), d) / z;
+            S.uv[1][tid] = dot3(mk3(M[4], M[5], M[6]), d) / z;
+            S.ray[0][tid] = o.x; S.ray[1][tid] = o.y; S.ray[2][tid] = o.z;
+            S.ray[3][tid] = d.x; S.ray[4][tid] = d.y; S.ray[5][tid] = d.z;
+        }
+        bounds(0, active);
+#pragma unroll
+        for (int off = 16; off; off >>= 1) z = fminf(z, __shfl_xor_sync(0xffffffffu, z, off));
+        if (lane == 0) S.z_min[warp] = z;
     }
     int n_active = __syncthreads_count(active);
-    int cur = 0;
-    for (int base = rg.x; base < rg.y && n_active > 0; base += B) {
-        const int n = min(B, rg.y - base);
-        int slot = rank;
-        if (active) {
-            if (kMasks) write_checkpoint(hm, st, rg.x, base, sub, subs, tid);
-            for (int w = 0; w < warp; ++w) slot += S.warp_base[w];
+    // 1 / (least z), 0: the bundle test is off (rays starting behind the
+    // camera position, axes that are no rotation, rays far off the axis)
+    float inv_z = 0.f;
+    if (!own_warp) {
+        float z = S.z_min[0];
 #pragma unroll
-            for (int k = 0; k < 6; ++k) S.ray[k][slot] = S.pray[k][tid];
+        for (int w = 1; w < Sh::kOwnWarps; ++w) z = fminf(z, S.z_min[w]);
+        const f3 r0 = mk3(M[0], M[1], M[2]), r1 = mk3(M[4], M[5], M[6]), r2 = mk3(M[8], M[9], M[10]);
+        const float skew = fmaxf(fmaxf(fmaxf(fabsf(dot3(r0, r1)), fabsf(dot3(r0, r2))), fabsf(dot3(r1, r2))),
+                                 fmaxf(fmaxf(fabsf(dot3(r0, r0) - 1.f), fabsf(dot3(r1, r1) - 1.f)),
+                                       fabsf(dot3(r2, r2) - 1.f)));
+        if (cam.min_t >= 0.f && skew < 2e-6f && z > 0.05f) inv_z = 1.0f / z;
+    }
+    if (!own_warp && n_active > 0)
+        stage_pair_batch<PX, NT, B>(S, 0, 0, 0, 1, rg.x, rg.y, ids, recs, cam, inv_z, lq, warp - Sh::kOwnWarps, lane);
+    int shape_of = -1;  // the active count that slots and rays are laid out for
+    int cur = 0, blk = 0;
+    __syncthreads();
+    while (n_active > 0 && blk * RB < rg.y - rg.x) {
+        const int m = S.n_blk[cur], n = S.start[cur][m];
+        if (n_active != shape_of) {  // some pixel ended: close the gaps it left
+            float ray[6];
+            if (active) {
+                for (int w = 0; w < warp; ++w) rank += S.warp_base[w];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) ray[k] = S.ray[k][slot];
+            }
+            __syncthreads();
+            if (active) {
+#pragma unroll
+                for (int k = 0; k < 6; ++k) S.ray[k][rank] = ray[k];
+                slot = rank;
+            }
+            shape_of = n_active;
+            __syncthreads();
         }
-        __syncthreads();
-        // Evaluate.  Rays stay in registers for the whole batch.  With more than
-        // 32 active slots a lane takes slots lane and lane + 32 of each entry the
-        // warp takes; with fewer, the warp splits into groups of `span` lanes
-        // (the next power of two >= n_active, at least 4), each group taking
-        // its own entry, so lanes do not idle when most pixels have terminated.
-        if (n_active > 32) {
-            const bool has1 = lane + 32 < n_active;
-            const f3 o0 = {S.ray[0][lane], S.ray[1][lane], S.ray[2][lane]};
-            const f3 d0 = {S.ray[3][lane], S.ray[4][lane], S.ray[5][lane]};
-            f3 o1 = o0, d1 = d0;
-            if (has1) {
-                o1 = {S.ray[0][lane + 32], S.ray[1][lane + 32], S.ray[2][lane + 32]};
-                d1 = {S.ray[3][lane + 32], S.ray[4][lane + 32], S.ray[5][lane + 32]};
-            }
-            for (int j = warp; j < n; j += kWarps) {
-                store_result(S, j, lane, eval_entry(S.srec[j], o0, d0));
-                if (has1) store_result(S, j, lane + 32, eval_entry(S.srec[j], o1, d1));
-            }
-        } else {
-            const int span = n_active <= 4 ? 4 : n_active <= 8 ? 8 : n_active <= 16 ? 16 : 32;
-            const int groups = 32 / span;
-            const int sl = lane & (span - 1);
-            const bool has = sl < n_active;
-            f3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f};
-            if (has) {
-                o = {S.ray[0][sl], S.ray[1][sl], S.ray[2][sl]};
-                d = {S.ray[3][sl], S.ray[4][sl], S.ray[5][sl]};
-            }
-            for (int j = warp * groups + lane / span; j < n; j += kWarps * groups)
-                if (has) store_result(S, j, sl, eval_entry(S.srec[j], o, d));
-        }
-        __syncthreads();
-        if (tid >= kOwnThreads) {
-            if (base + B < rg.y)
-                stage_pair_batch(S, cur ^ 1, base + B, min(B, rg.y - base - B), ids, recs, lq, tid - kOwnThreads,
-                                 NT - kOwnThreads);
-        } else {
-            // Fold in list order; the hit tests of four entries are read ahead.
-            uint64_t hb = 0;  // bit j: entry j of the batch was a hit for this owner's pixel
-            for (int j0 = 0; active && j0 < n; j0 += 4) {
-                float a4[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) a4[u] = j0 + u < n ? S.res[0][j0 + u][slot] : 0.f;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int j = j0 + u;
-                    if (!active || j >= n) break;
-                    ++nc;
-                    if (a4[u] > 0.f) {
-                        hb |= 1ull << j;
-                        const float rgb[3] = {S.res[3][j][slot], S.res[4][j][slot], S.res[5][j][slot]};
-                        fold_hit(st, a4[u], S.dens[cur][j], S.res[1][j][slot], S.res[2][j][slot], rgb);
-                        if (st.logT < kTermLogT) active = false;
-                    }
+        if (n > 0) {
+            // Evaluate.  With more than 32 active slots the warps form two
+            // teams, one per half of the slots, sized by the work; a team with
+            // few slots splits its warps into groups of `span` lanes (a power
+            // of two, at least 4), each group taking its own entry.
+            int first = 0, cnt = n_active, team = Sh::kWarps, member = warp;
+            if (PX > 32 && n_active > 32) {
+                const int rest = n_active - 32;
+                const int w1 = rest > 16 ? Sh::kWarps / 2 : rest > 8 ? Sh::kWarps * 3 / 8 : rest > 4 ? Sh::kWarps / 4
+                                                                                                    : Sh::kWarps / 8;
+                cnt = 32;
+                team = Sh::kWarps - w1;
+                if (warp >= team) {
+                    member = warp - team;
+                    first = 32;
+                    cnt = rest;
+                    team = w1;
                 }
             }
-            if (kMasks && owner && hm.words) write_masks(hm, hb, gtile, rg.x, base, n, sub, subs, tid);
-            // the next batch's slots: the pixels still active
-            if (owner) {
-                const unsigned bal = __ballot_sync(kOwnMask, active);
-                if (lane == 0) S.warp_base[warp] = __popc(bal);
-                rank = __popc(bal & ((1u << lane) - 1u));
+            const int span = cnt <= 4 ? 4 : cnt <= 8 ? 8 : cnt <= 16 ? 16 : 32;
+            const int groups = 32 / span;
+            const int sl = first + (lane & (span - 1));
+            if ((lane & (span - 1)) < cnt) {
+                const f3 o = {S.ray[0][sl], S.ray[1][sl], S.ray[2][sl]};
+                const f3 d = {S.ray[3][sl], S.ray[4][sl], S.ray[5][sl]};
+                for (int j = member * groups + lane / span; j < n; j += team * groups)
+                    store_result(S, j, sl, eval_entry(S.srec[j], o, d));
             }
+            __syncthreads();
         }
+        if (!own_warp) {
+            const int next = blk + m;
+            // blocks to look at: as many as the last batch's yield would need to fill B records
+            const int tries = min(Sh::kStageWarps, max(1, B * m / max(n, 1)));
+            if (next * RB < rg.y - rg.x)
+                stage_pair_batch<PX, NT, B>(S, cur ^ 1, cur, next, tries, rg.x, rg.y, ids, recs, cam, inv_z, lq,
+                                            warp - Sh::kOwnWarps, lane);
+        } else {
+            const bool was = active;
+            for (int w = 0; w < m; ++w) {
+                const int j1 = S.start[cur][w + 1];
+                uint32_t hb = 0;  // bit k: entry k of the block was a hit for this owner's pixel
+                if (kMasks && active) write_checkpoint(hm, st, rg.x, rg.x + (blk + w) * RB, sub, subs, p);
+                for (int j = S.start[cur][w]; j < j1 && active; j += 4) {
+                    float a[4];
+                    float logT = st.logT;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        a[k] = j + k < j1 ? S.res[0][min(j + k, B - 1)][slot] : 0.f;
+                        logT = logT - a[k];
+                    }
+                    if (j + 4 <= j1 && !(logT < kTermLogT)) {  // log T never rises: none of the four ends the walk
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const bool hit = a[k] > 0.f;
+                            hb |= hit ? 1u << S.pos[cur][j + k] : 0u;
+                            fold_any(st, a[k], hit ? S.dens[cur][j + k] : 0.f, S.res[1][j + k][slot],
+                                     S.res[2][j + k][slot], S.res[3][j + k][slot], S.res[4][j + k][slot],
+                                     S.res[5][j + k][slot]);
+                        }
+                    } else {
+                        for (int k = 0; k < 4 && j + k < j1; ++k) {
+                            const float ak = S.res[0][j + k][slot];
+                            if (!(ak > 0.f)) continue;
+                            const int at = S.pos[cur][j + k];
+                            hb |= 1u << at;
+                            fold_any(st, ak, S.dens[cur][j + k], S.res[1][j + k][slot], S.res[2][j + k][slot],
+                                     S.res[3][j + k][slot], S.res[4][j + k][slot], S.res[5][j + k][slot]);
+                            if (st.logT < kTermLogT) {
+                                active = false;
+                                nc = (blk + w) * RB + at + 1;
+                                break;
+                            }
+                        }
+                    }
+                }
+                if (kMasks && owner && hm.words) {
+                    const int64_t i = mask_word(gtile, rg.x, blk + w, sub, subs, p);
+                    if (i < hm.cap) __stcg(hm.words + i, hb);
+                }
+            }
+            if (__any_sync(0xffffffffu, was != active))
+                bounds(cur ^ 1, active);
+            else if (lane < 4)
+                S.bnd[cur ^ 1][warp][lane] = S.bnd[cur][warp][lane];
+            rank = rank_active();
+        }
+        blk += m;
         cur ^= 1;
         n_active = __syncthreads_count(active);
     }
@@ -763,15 +1018,26 @@ __global__ void __launch_bounds__(NT, MINB) blend_fwd_pair_kernel(
     FwdPairSmem<PX, B>& S = *reinterpret_cast<FwdPairSmem<PX, B>*>(fwd_smem_raw);
     __shared__ int s_item;
     __shared__ HitMasks hm;  // read once per batch: kept out of the registers
-    const int n_items = queue_items(q);
+    // the first info[1] tiles of the order go by quarters of their strips
+    const int nq = PX == 64 ? __ldg(q.info + 1) : 0;
+    const int q_items = nq * q.subs * 4;
+    const int n_items = q_items + (__ldg(q.info) - nq) * q.subs;
     if (threadIdx.x == 0) hm = live_masks(q.hm, q.subs);  // seen after next_item's barriers
     for (;;) {
-        const int item = next_item(q, &s_item);
+        int item = next_item(q, &s_item);
         if (item >= n_items) return;
-        const int t = queue_tile(q, item), v = views.find(t);
+        int quarter = -1, at = 0;
+        if (item < q_items) {
+            quarter = item & 3;
+            item >>= 2;
+        } else {
+            item -= q_items;
+            at = nq;
+        }
+        const int t = __ldg(q.order + at + item / q.subs), v = views.find(t);
         const int tb = views.tile_base(v);
         const int64_t pb = views.pixel_base(v);
-        fwd_pair_item<PX, NT, B>(t - tb, item % q.subs, ids, ranges + tb, recs, jitter + pb, views.camera(v),
+        fwd_pair_item<PX, NT, B>(t - tb, item % q.subs, quarter, ids, ranges + tb, recs, jitter + pb, views.camera(v),
                                  out_img + pb, out_dist + 5 * pb, out_nc + pb, S, hm, q.subs, t, q);
     }
 }
@@ -783,7 +1049,8 @@ __global__ void __launch_bounds__(NT, MINB) blend_fwd_pair_kernel(
 __global__ void __launch_bounds__(1024) order_kernel(const int2* __restrict__ ranges, int G,
                                                      int32_t* __restrict__ order, int32_t* info,
                                                      uint32_t* tickets, int heavy_shift, uint32_t* mask_header,
-                                                     const MaskHeader mh, const uint32_t* seg_header) {
+                                                     const MaskHeader mh, const uint32_t* seg_header,
+                                                     int quarter_slots) {
     // Warp-aggregated counting: lanes that share a bucket elect one leader
     // (match_any) for the shared atomic, and the list-length sum and the
     // non-empty count are reduced per warp before one shared update each.
@@ -838,6 +1105,15 @@ __global__ void __launch_bounds__(1024) order_kernel(const int2* __restrict__ ra
         int heavy = 0;
         for (int b = 32; b >= b_thr; --b) heavy += (int)cnt[b];
         info[0] = heavy;
+        // Tiles whose list is longer than one resident CTA's share of all
+        // entries go by quarters: walked by one CTA each, they would outlast
+        // the launch.  A launch with fewer strips than CTAs splits most.
+        int quarters = 0;
+        if (quarter_slots > 0) {
+            const unsigned long long share = sum / quarter_slots;
+            for (int b = 32; b > 0 && (1ull << (b - 1)) >= share; --b) quarters += (int)cnt[b];
+        }
+        info[1] = min(quarters, heavy);
         for (int k = 0; k < 4; ++k) tickets[k] = 0u;
         if (mask_header) {
             mask_header[0] = mh.state;
@@ -1161,6 +1437,11 @@ __device__ __forceinline__ void seed_segment(const HitMasks& hm, int x, int s1, 
     dS_logT = fmaf(dS_c[2], final_c.z - __ldcg(c + 5 * 64), dS_logT);
 }
 
+// The lowest n bits of w (none for n <= 0).
+__device__ __forceinline__ uint32_t bits_below(uint32_t w, int n) {
+    return n <= 0 ? 0u : n >= 32 ? w : w & ((1u << n) - 1u);
+}
+
 // Dense backward item: a strip of NT pixels, one thread per pixel walking its
 // list back to front from the saved final state.
 template <int NT, int B>
@@ -1254,8 +1535,11 @@ __device__ __forceinline__ void bwd_dense_item(
             if (i0 < hm.cap) hw0 = __ldcg(hm.words + i0);
             if (i1 < hm.cap) hw1 = __ldcg(hm.words + i1);
         }
+        hw0 = bits_below(hw0, nc - kb0 * 32);
+        hw1 = bits_below(hw1, nc - kb1 * 32);
         // entries no pixel of the item hit are dropped from the batch before
-        // staging (the masks of pixels past their n_contributors are zero)
+        // staging (the bits at and past n_contributors, which the forward may
+        // have left unwritten, are cleared above)
         uint32_t o0 = hw0, o1 = hw1;
 #pragma unroll
         for (int off = WarpShape<NT>::kTopOffset; off > 0; off >>= 1) {
@@ -1303,7 +1587,7 @@ __device__ __forceinline__ void bwd_dense_item(
             const int off = lo + S.cidx[jj] - rg.x;
             // with the forward's masks, only its hits are revisited
             const uint32_t hw = (off >> 5) == kb0 ? hw0 : hw1;
-            const bool act_a = inside && off < nc && ((hw >> (off & 31)) & 1u);
+            const bool act_a = (hw >> (off & 31)) & 1u;
             const uint32_t bal_a = __ballot_sync(kMask, act_a);
             if (!bal_a) {
                 --jj;
@@ -1319,7 +1603,7 @@ __device__ __forceinline__ void bwd_dense_item(
                 if (jj >= 1) {
                     const int off_b = lo + S.cidx[jj - 1] - rg.x;
                     const uint32_t hwb = (off_b >> 5) == kb0 ? hw0 : hw1;
-                    act_b = inside && off_b < nc && ((hwb >> (off_b & 31)) & 1u);
+                    act_b = (hwb >> (off_b & 31)) & 1u;
                     bal_b = __ballot_sync(kMask, act_b);
                     if (bal_a & bal_b) {
                         act_b = false;
@@ -2207,9 +2491,10 @@ int side_stream(cudaStream_t caller, SideStream** out) {
 }
 
 int launch_order(const int32_t* ranges, int G, const BlendWs& w, int heavy_shift, cudaStream_t s,
-                 uint32_t* mask_header = nullptr, MaskHeader mh = MaskHeader{}, const uint32_t* seg_header = nullptr) {
+                 uint32_t* mask_header = nullptr, MaskHeader mh = MaskHeader{}, const uint32_t* seg_header = nullptr,
+                 int quarter_slots = 0) {
     order_kernel<<<1, 1024, 0, s>>>((const int2*)ranges, G, w.order, w.info, w.tickets, heavy_shift, mask_header, mh,
-                                    seg_header);
+                                    seg_header, quarter_slots);
     return rm_host::check_launch("rm_blend order");
 }
 
@@ -2267,8 +2552,10 @@ int launch_fwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, cons
     const bool masks = tn.hit_masks && PX == 64 && PX_PAIR == 64 && w.mask_header;
     const int subs = sh.tile_px / PX;
     const int subs_pair = sh.tile_px / PX_PAIR;
+    const int pair_cap = tn.pair_ctas_per_sm * sm_count();
     int rc = launch_order(ranges, G, w, tn.heavy_shift, s, w.mask_header,
-                          masks ? mask_header_for(w.mask_cap, G, subs) : MaskHeader{});
+                          masks ? mask_header_for(w.mask_cap, G, subs) : MaskHeader{}, nullptr,
+                          PX_PAIR == 64 ? (pair_cap > subs_pair ? pair_cap / subs_pair : 1) : 0);
     if (rc) return rc;
     const HitMasks hm = {masks ? w.mask_words : nullptr, w.mask_cap, w.mask_header, nullptr, 0, kNoSegments};
     const Queue qd = {w.order, w.info, w.tickets + 0, G, subs, false, hm, tn.status, rm_host::wait_limit(),
@@ -2280,8 +2567,8 @@ int launch_fwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, cons
                            : blend_fwd_pair_kernel<PX_PAIR, NT_PAIR, B_PAIR, 768 / NT_PAIR, V>;
     const int smem = (int)sizeof(FwdPairSmem<PX_PAIR, B_PAIR>);
     cudaFuncSetAttribute(pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    const int pair_cap = tn.pair_ctas_per_sm * sm_count();
-    const int pair_grid = G * subs_pair < pair_cap ? G * subs_pair : pair_cap;
+    const int64_t pair_items = (int64_t)G * subs_pair * (PX_PAIR == 64 ? 4 : 1);
+    const int pair_grid = pair_items < pair_cap ? (int)pair_items : pair_cap;
     if (tn.heavy_shift == 1) {
         pair_kernel<<<pair_grid, NT_PAIR, smem, s>>>(ids, (const int2*)ranges, w.recs, (const float2*)jitter, views,
                                                      (float4*)img, dist, nc, qp);

@@ -1,23 +1,32 @@
-"""Lists around the lengths at which the passes change how they walk them:
-the backward takes a list in stretches of 128 entries, each from the state
-the forward left there, so lists one entry short of, at and past whole
-stretches are compared with the oracle's adjoint, with pixels that end before,
-inside and after a stretch."""
+"""Lists around the lengths at which the passes change how they walk them.
+
+The forward takes a list in blocks of 32 entries, drops the entries that no
+ray of a strip can hit and fills a batch from as many blocks as that leaves
+room for: lists around whole blocks, dense and mostly dropped, are compared
+with the oracle bit for bit (log T, distortion, n_contributors).  The backward
+takes a list in stretches of 128 entries, each from the state the forward
+left there: lists one entry short of, at and past whole stretches are compared
+with the oracle's adjoint, with pixels that end before, inside and after a
+stretch."""
 import numpy as np
 import pytest
 
+from gpu_util import bits, run_gpu_forward
+from oracle import oracle as O
 from radiance_meshes_b200.camera import pinhole_tcam
 from test_gpu_backward import _run
 
 pytestmark = pytest.mark.gpu
 
 
-def _stack(n, density, seed):
+def _stack(n, density, seed, small=0.0):
     """n thin tets one behind the other along the view axis, wider than most
-    of the image, each shifted sideways a little."""
+    of the image, each shifted sideways a little; a fraction `small` of them a
+    few pixels wide."""
     rng = np.random.default_rng(seed)
     z = 2.0 + 0.02 * np.arange(n)[:, None]
     s = z * rng.uniform(0.3, 1.2, size=(n, 1))
+    s[rng.uniform(size=n) < small] *= 0.05
     cx, cy = (z * rng.uniform(-0.2, 0.2, size=(n, 1)) for _ in range(2))
     corners = [(-1, -1, 0.0), (1, -1, 0.0), (0, 1.2, 0.0), (0.0, 0.0, 0.015)]
     verts = np.concatenate([np.concatenate([cx + a * s, cy + b * s, z + dz], 1)[:, None] for a, b, dz in corners], 1)
@@ -34,3 +43,20 @@ def test_backward_over_stretches(cuda, n, density):
     tcam = pinhole_tcam((0.0, 0.0, 0.0), (0.0, 0.0, 1.0), 11, 13, 30.0, tile_size=8)
     jitter = np.random.default_rng(n).uniform(0, 1, (11, 13, 2)).astype(np.float32)
     _run(verts, idx, cv, tcam, jitter, "linear", seed=n, check_f64=False, hit_masks=True)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 65, 191, 193, 420])
+@pytest.mark.parametrize("small", [0.0, 0.95])
+@pytest.mark.parametrize("density,tile", [(0.3, 8), (6.0, 8), (6.0, 16), (1.0, 4)])
+def test_forward_over_blocks(cuda, n, small, density, tile):
+    verts, idx, cv = _stack(n, density, n, small)
+    cv[::7, 0] = 0.0
+    tcam = pinhole_tcam((0.1, 0.0, 0.0), (0.0, 0.0, 1.0), 21, 18, 30.0, tile_size=tile)
+    jitter = np.random.default_rng(n).uniform(0, 1, (21, 18, 2)).astype(np.float32)
+    L = O.rasterize_lists(idx, verts, tcam)
+    img, dist, nc = O.blend_fwd_f32(L, idx, verts, cv, jitter)
+    r = run_gpu_forward(verts, idx, cv, tcam, jitter, keep_debug=False, hit_masks=True)
+    assert np.array_equal(r["nc"].cpu().numpy()[..., 0], nc)
+    assert np.array_equal(bits(r["img"].cpu().numpy()[..., 3]), bits(img[..., 3]))
+    assert np.array_equal(bits(r["dist"].cpu().numpy()), bits(dist))
+    assert np.abs(r["img"].cpu().numpy() - img).max() <= 1e-4
