@@ -319,12 +319,13 @@ RM_API size_t rm_blend_status_offset(int64_t n_tets, int64_t n_tiles);
 #define RM_BLEND_STRIP_SHIFT 8
 #define RM_BLEND_STRIP(log2_pixels) ((log2_pixels) << RM_BLEND_STRIP_SHIFT)
 /* flags bits 16..19: heavy-tile threshold, in powers of two above the mean
- * list length (0 = default, 1 = every tile is heavy); bits 20..23: resident
- * CTAs per SM of the kernel that takes the heavy tiles (0 = default) */
+ * list length (0 = default: the forward decides by the lists' lengths, the
+ * backward has none; 1 = every tile is heavy); bits 20..23: resident CTAs per
+ * SM of the kernel that takes the heavy tiles (0 = default) */
 #define RM_BLEND_HEAVY_SHIFT 16
 #define RM_BLEND_PAIR_CTAS_SHIFT 20
 /* flags bits 24..27: log2 of the tets staged per shared-memory batch by the
- * pass's main kernel (forward: the pair kernel, backward: the dense kernel);
+ * pass's main kernel (forward: the pair items, backward: the dense kernel);
  * 4, 5 or 6 (0 = default 32) */
 #define RM_BLEND_BATCH_SHIFT 24
 

@@ -6,11 +6,11 @@ Knobs, all measured on the caller's own mesh and cameras:
   blend (the same, or 2^k times smaller, down to 8: the sorted lists are then
   split in order, rm_fine_lists_multi).  Smaller blend tiles waste fewer
   ray/tet tests per pixel; smaller list tiles cost more pairs to sort.
-* work split between the two blend kernels, i.e. pixels per thread: the
-  one-thread-per-pixel dense kernel versus the pair kernel that spreads a
-  strip's (entry, pixel) tests over four threads per pixel (heavy-tile
-  threshold; 1 sends every tile to the pair kernel), and the pair kernel's
-  resident CTAs per SM.
+* work split of the blend, i.e. threads per pixel: a warp of its own for
+  half a strip versus a CTA that spreads a strip's (entry, pixel) tests over
+  four threads per pixel (heavy-tile threshold; 0 lets the lists' lengths
+  decide in the forward, 1 sends every tile to the CTAs), and the resident
+  CTAs per SM.
 * pixels per work item (strip of 16 or 64 pixels).
 * tets per shared-memory batch (16, 32 or 64).
 
@@ -54,11 +54,13 @@ def flags(strip: int = 0, heavy_shift: int = 0, pair_ctas: int = 0, batch: int =
 
 def candidates_fwd(tile: int):
     out = []
+    strip = 64 if tile >= 8 else 16
     for b in (16, 32, 64):
-        for ctas in (2, 3, 4):
-            out.append(dict(strip=64 if tile >= 8 else 16, heavy_shift=1, pair_ctas=ctas, batch=b))
+        for ctas in (2, 3):
+            out.append(dict(strip=strip, heavy_shift=0, pair_ctas=ctas, batch=b))
+    out.append(dict(strip=strip, heavy_shift=1, pair_ctas=3, batch=32))
     out.append(dict(strip=16, heavy_shift=1, pair_ctas=3, batch=32))
-    out.append(dict(strip=64 if tile >= 8 else 16, heavy_shift=3, pair_ctas=2, batch=32))
+    out.append(dict(strip=strip, heavy_shift=3, pair_ctas=2, batch=32))
     return out
 
 
@@ -66,7 +68,7 @@ def candidates_bwd(tile: int):
     out = []
     for strip in ((16, 64) if tile >= 8 else (16,)):
         for b in (16, 32, 64):
-            out.append(dict(strip=strip, heavy_shift=15, pair_ctas=1, batch=b))
+            out.append(dict(strip=strip, heavy_shift=0, pair_ctas=1, batch=b))
     out.append(dict(strip=64 if tile >= 8 else 16, heavy_shift=3, pair_ctas=1, batch=32))
     return out
 

@@ -9,22 +9,25 @@
 // the reference obtains from Slang autodiff written out by hand.
 //
 // Work decomposition.  Per-tile list lengths are heavy-tailed (a few tiles
-// hold 10-30x the mean), and a pixel whose ray sees through a dense region
-// crosses thousands of tets.  Each pass therefore runs two persistent kernels
-// concurrently, fed by one heavy-first tile order computed on the device:
-//   * the dense kernel walks the ordinary tiles, one thread per pixel, in
-//     strips of 64 pixels (one CTA per strip);
-//   * the pair kernel takes the heavy tiles (list length >= ~4x the mean) and
-//     spreads each strip's (entry, pixel) pairs over 4 threads per pixel; the
-//     strictly ordered part of the walk (log T, termination, distortion
-//     moments in the forward; the undo chains in the backward) is a few adds
-//     per entry done by one owner thread per pixel, in the same arithmetic as
-//     the dense walk, so results do not depend on which kernel ran a tile.
-// In both, per-tet records (128 B, packed once per frame by pack_kernel) are
-// staged in shared memory per batch of list entries.  Backward gradients are
-// summed per list entry across the pixels of a CTA (warp reduce-scatter, then
-// shared-memory atomics) and converted to vertex gradients once per
-// (CTA, entry) before the global atomics.
+// hold 10-100x the mean), and a pixel whose ray sees through a dense region
+// crosses thousands of tets.  Each pass is one persistent kernel fed by a
+// heavy-first tile order computed on the device, whose work items differ by
+// the length of the list:
+//   * forward, warp items: half of a 64-pixel strip walked by one warp;
+//   * forward, pair items: lists longer than a warp's share of the launch are
+//     walked by a CTA that spreads the (entry, pixel) pairs over its threads,
+//     the longest by quarters of a strip; the strictly ordered part of the
+//     walk (log T, termination, distortion moments) is a few adds per entry
+//     by one owner thread per pixel, in the same arithmetic, so results do
+//     not depend on which kind of item ran a tile;
+//   * backward: strips of 64 pixels, one thread per pixel, long lists in
+//     stretches that start from states the forward left (checkpoints).
+// The backward's pair kernel (4 threads per pixel) runs on request only.
+// Per-tet records (128 B, packed once per frame by pack_kernel) are staged in
+// shared memory per block of list entries.  Backward gradients are summed per
+// list entry across the pixels of a CTA (warp sums, then shared-memory
+// atomics) and converted to vertex gradients once per (CTA, entry) before the
+// global atomics.
 #include <mutex>
 
 #include "rm_internal.cuh"
@@ -273,9 +276,6 @@ struct WarpShape {
     static constexpr int kWarps = NT >= 32 ? NT / 32 : 1;
 };
 
-// Work queue shared by the kernels of one pass.  order[] lists the tiles
-// heaviest first; info[0] is the number of heavy tiles (the first entries of
-// order[]), which go to the pair kernel, the rest to the dense kernel.
 // Hit masks written by the forward and read by the backward
 // (RM_BLEND_HIT_MASKS; 64-pixel work items only).  A tile's list is cut into
 // blocks of 32 entries counted from its start; pixel p of work item `sub`
@@ -350,6 +350,10 @@ __device__ __forceinline__ HitMasks live_masks(HitMasks hm, int subs) {
     return hm;
 }
 
+// Work queue shared by the kernels of one pass.  order[] lists the tiles
+// heaviest first; info[0] is the number of heavy tiles (the first entries of
+// order[]), which go by pair items, the rest by warp items (forward) or to the
+// dense kernel (backward).
 struct Queue {
     const int32_t* order;
     const int32_t* info;
@@ -513,82 +517,20 @@ __device__ __forceinline__ EntryResult eval_entry(const float4* __restrict__ q, 
     r.d4 = 0.f;
     r.rgb[0] = r.rgb[1] = r.rgb[2] = 0.f;
     if (is.geo && s.a > 0.f) {
-        integrate(q, o, d, is.enter, is.exit, s);
         r.a = s.a;
+        // compute_integral (interp_version.slang:30-69) with the colour linear
+        // along the ray: c(t) = base + dot(grd, o - v0) + t dot(grd, d)
+        const f3 grd = {q[4].w, q[5].w, q[6].w};
+        const float c0 = -dot3(grd, xyz(q[4]) - o), gd = dot3(grd, d);
+        const Weights w = seg_weights(s.a);
+        const float lin = fmaf(w.w0, fmaf(is.exit, gd, c0), w.w1 * fmaf(is.enter, gd, c0)), sum = w.w0 + w.w1;
+        r.rgb[0] = fmaf(sum, q[1].w, lin);
+        r.rgb[1] = fmaf(sum, q[2].w, lin);
+        r.rgb[2] = fmaf(sum, q[3].w, lin);
         r.m1 = density * (is.exit + is.enter) / 2.0f;
         r.d4 = third(density * density * s.dt);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) r.rgb[k] = s.rgb[k];
     }
     return r;
-}
-
-// Dense forward item: a strip of NT pixels (NT / tile_width rows), one thread
-// per pixel walking the tile's list in order.
-template <int B>
-struct FwdDenseSmem {
-    float4 srec[B][kRecFloat4];
-    int32_t sid[B];
-};
-
-template <int NT, int B>
-__device__ __forceinline__ void fwd_dense_item(int tile, int sub, const int32_t* __restrict__ ids,
-                                               const int2* __restrict__ ranges, const float4* __restrict__ recs,
-                                               const float2* __restrict__ jitter, const rm_camera& cam,
-                                               float4* __restrict__ out_img, float* __restrict__ out_dist,
-                                               int32_t* __restrict__ out_nc, FwdDenseSmem<B>& S,
-                                               const HitMasks& hm, int subs, int gtile, const Queue& lq) {
-    constexpr bool kMasks = NT == 64 && B % 32 == 0;
-    const int tx = tile % cam.grid_width, ty = tile / cam.grid_width;
-    int lx, ly;
-    strip_pixel<NT>(cam, sub, (int)threadIdx.x, lx, ly);
-    const int px = tx * cam.tile_width + lx, py = ty * cam.tile_height + ly;
-    const bool inside = px < cam.image_width && py < cam.image_height;
-    const int64_t pix = (int64_t)py * cam.image_width + px;
-    f3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f};
-    if (inside) {
-        const float2 j = __ldg(jitter + pix);
-        make_ray(cam, px, py, j.x, j.y, o, d);
-    }
-    const int2 rg = __ldg(ranges + tile);
-    PixelState st = {{0.f, 0.f, 0.f}, 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}};
-    int32_t nc = 0;
-    bool active = inside;
-    if (__syncthreads_or(active)) {
-        for (int base = rg.x; base < rg.y; base += B) {
-            const int n = min(B, rg.y - base);
-            if (kMasks && active) write_checkpoint(hm, st, rg.x, base, sub, subs, (int)threadIdx.x);
-            for (int k = threadIdx.x; k < n; k += NT) S.sid[k] = list_id(ids, base + k, lq);
-            __syncthreads();
-            for (int k = threadIdx.x; k < n * kRecFloat4; k += NT) {
-                const int j = k >> 3, c = k & 7;
-                S.srec[j][c] = record_part(recs, S.sid[j], c);
-            }
-            __syncthreads();
-            uint64_t hb = 0;  // bit j: entry j of the batch was a hit
-            if (__any_sync(WarpShape<NT>::kMask, active)) {
-                for (int j = 0; j < n; ++j) {
-                    if (!active) break;
-                    ++nc;
-                    const EntryResult r = eval_entry(S.srec[j], o, d);
-                    if (r.a > 0.f) {
-                        hb |= 1ull << j;
-                        fold_hit(st, r.a, S.srec[j][0].w, r.m1, r.d4, r.rgb);
-                        if (st.logT < kTermLogT) active = false;
-                    }
-                }
-            }
-            if (kMasks && hm.words) write_masks(hm, hb, gtile, rg.x, base, n, sub, subs, (int)threadIdx.x);
-            if (!__syncthreads_or(active)) break;
-        }
-    }
-    if (inside) {
-        out_img[pix] = make_float4(st.c[0], st.c[1], st.c[2], st.logT);
-        float* dd = out_dist + 5 * pix;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) dd[k] = st.D[k];
-        out_nc[pix] = nc;
-    }
 }
 
 // A bundle of rays from one point: every ray direction is a positive multiple
@@ -615,7 +557,7 @@ __device__ __forceinline__ bool entry_reaches(const float4* __restrict__ r, cons
                                               float inv_z) {
     const f3 c = {cam.cam_pos[0], cam.cam_pos[1], cam.cam_pos[2]};
     const float* M = cam.world_view;
-    const f3 a0 = xyz(__ldg(r + 4)) - c, a1 = xyz(__ldg(r + 5)) - c;
+    const f3 a0 = xyz(r[4]) - c, a1 = xyz(r[5]) - c;
     const float A = fmaxf(fabsf(a0.x) + fabsf(a0.y) + fabsf(a0.z), fabsf(a1.x) + fabsf(a1.y) + fabsf(a1.z)) +
                     (fabsf(c.x) + fabsf(c.y) + fabsf(c.z)) + cam.min_t;
     float dist[4], N[4];
@@ -623,7 +565,7 @@ __device__ __forceinline__ bool entry_reaches(const float4* __restrict__ r, cons
     uint32_t outside = 0, inside = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const f3 n = xyz(__ldg(r + i));
+        const f3 n = xyz(r[i]);
         dist[i] = -dot3(n, i == 3 ? a1 : a0);
         N[i] = fabsf(n.x) + fabsf(n.y) + fabsf(n.z);
         const float sure = fmaf(2e-6f * N[i], A, 1e-9f * (1.0f + cam.min_t));
@@ -649,6 +591,18 @@ __device__ __forceinline__ bool entry_reaches(const float4* __restrict__ r, cons
         }
     }
     return reach;
+}
+
+// 1 / (least z) of a bundle, or 0 when entry_reaches does not apply (rays
+// starting behind the camera position, axes that are no rotation, rays far
+// off the axis).
+__device__ __forceinline__ float bundle_inv_z(const rm_camera& cam, float z_min) {
+    const float* M = cam.world_view;
+    const f3 r0 = mk3(M[0], M[1], M[2]), r1 = mk3(M[4], M[5], M[6]), r2 = mk3(M[8], M[9], M[10]);
+    const float skew = fmaxf(fmaxf(fmaxf(fabsf(dot3(r0, r1)), fabsf(dot3(r0, r2))), fabsf(dot3(r1, r2))),
+                             fmaxf(fmaxf(fabsf(dot3(r0, r0) - 1.f), fabsf(dot3(r1, r1) - 1.f)),
+                                   fabsf(dot3(r2, r2) - 1.f)));
+    return cam.min_t >= 0.f && skew < 2e-6f && z_min > 0.05f ? 1.0f / z_min : 0.f;
 }
 
 // Pair forward item: a strip of PX pixels (PX / tile_width rows of one tile)
@@ -707,6 +661,12 @@ __device__ __forceinline__ void store_result(FwdPairSmem<PX, B>& S, int j, int s
     S.res[5][j][sl] = r.rgb[2];
 }
 
+// One record (a 128-byte line: four sectors, fetched one by one) into L1.
+__device__ __forceinline__ void prefetch_record(const float4* r) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) asm volatile("prefetch.global.L1 [%0];" ::"l"(r + 2 * k));
+}
+
 // Stages a batch from block `blk` of the list [x, y) on with the staging
 // warps (sw: this warp's number among them): looks at up to `tries` blocks,
 // one per warp, and keeps as many as fit in B records (at least one).
@@ -725,6 +685,7 @@ __device__ __forceinline__ void stage_pair_batch(FwdPairSmem<PX, B>& S, int buf,
         if (lane < Sh::RB && e < y) g = list_id(ids, e, lq);
         if (g >= 0) {
             r = recs + (int64_t)kRecFloat4 * g;
+            prefetch_record(r);  // the record's four sectors at once
             keep = __ldg(&r[0].w) > 0.f;  // a density of zero hits nothing
             if (keep && inv_z > 0.f) {
                 Bundle bd = {S.bnd[rd][0][0], S.bnd[rd][0][1], S.bnd[rd][0][2], S.bnd[rd][0][3]};
@@ -737,6 +698,14 @@ __device__ __forceinline__ void stage_pair_batch(FwdPairSmem<PX, B>& S, int buf,
         }
         bal = __ballot_sync(0xffffffffu, keep);
         if (lane == 0) S.bal[sw] = bal;
+    } else if (sw == tries) {
+        // the block after: its records into L1, where the next staging finds
+        // them (a batch of a long list is otherwise mostly load latency)
+        const int e = x + (blk + sw) * Sh::RB + lane;
+        if (lane < Sh::RB && e < y) {
+            const int32_t g = __ldg(ids + e);
+            if (g >= 0 && (int64_t)g < lq.n_recs) prefetch_record(recs + (int64_t)kRecFloat4 * g);
+        }
     }
     if (Sh::kStageWarps > 1)
         asm volatile("bar.sync 1, %0;" ::"r"(Sh::kStageWarps * 32) : "memory");
@@ -851,18 +820,12 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
         if (lane == 0) S.z_min[warp] = z;
     }
     int n_active = __syncthreads_count(active);
-    // 1 / (least z), 0: the bundle test is off (rays starting behind the
-    // camera position, axes that are no rotation, rays far off the axis)
     float inv_z = 0.f;
     if (!own_warp) {
         float z = S.z_min[0];
 #pragma unroll
         for (int w = 1; w < Sh::kOwnWarps; ++w) z = fminf(z, S.z_min[w]);
-        const f3 r0 = mk3(M[0], M[1], M[2]), r1 = mk3(M[4], M[5], M[6]), r2 = mk3(M[8], M[9], M[10]);
-        const float skew = fmaxf(fmaxf(fmaxf(fabsf(dot3(r0, r1)), fabsf(dot3(r0, r2))), fabsf(dot3(r1, r2))),
-                                 fmaxf(fmaxf(fabsf(dot3(r0, r0) - 1.f), fabsf(dot3(r1, r1) - 1.f)),
-                                       fabsf(dot3(r2, r2) - 1.f)));
-        if (cam.min_t >= 0.f && skew < 2e-6f && z > 0.05f) inv_z = 1.0f / z;
+        inv_z = bundle_inv_z(cam, z);
     }
     if (!own_warp && n_active > 0)
         stage_pair_batch<PX, NT, B>(S, 0, 0, 0, 1, rg.x, rg.y, ids, recs, cam, inv_z, lq, warp - Sh::kOwnWarps, lane);
@@ -931,21 +894,27 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
                 uint32_t hb = 0;  // bit k: entry k of the block was a hit for this owner's pixel
                 if (kMasks && active) write_checkpoint(hm, st, rg.x, rg.x + (blk + w) * RB, sub, subs, p);
                 for (int j = S.start[cur][w]; j < j1 && active; j += 4) {
-                    float a[4];
+                    // four entries' results read ahead, whatever they are (rows past
+                    // the block's last are there to read and not used)
+                    float r[6][4], dens[4];
+                    uint32_t bit[4];
                     float logT = st.logT;
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        a[k] = j + k < j1 ? S.res[0][min(j + k, B - 1)][slot] : 0.f;
-                        logT = logT - a[k];
+                        const int jk = min(j + k, B - 1);
+#pragma unroll
+                        for (int c = 0; c < 6; ++c) r[c][k] = S.res[c][jk][slot];
+                        dens[k] = S.dens[cur][jk];
+                        bit[k] = 1u << S.pos[cur][jk];
+                        if (j + k >= j1) r[0][k] = r[1][k] = r[2][k] = r[3][k] = r[4][k] = r[5][k] = 0.f;
+                        logT = logT - r[0][k];
                     }
-                    if (j + 4 <= j1 && !(logT < kTermLogT)) {  // log T never rises: none of the four ends the walk
+                    if (!(logT < kTermLogT)) {  // log T never rises: none of the four ends the walk
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
-                            const bool hit = a[k] > 0.f;
-                            hb |= hit ? 1u << S.pos[cur][j + k] : 0u;
-                            fold_any(st, a[k], hit ? S.dens[cur][j + k] : 0.f, S.res[1][j + k][slot],
-                                     S.res[2][j + k][slot], S.res[3][j + k][slot], S.res[4][j + k][slot],
-                                     S.res[5][j + k][slot]);
+                            const bool hit = r[0][k] > 0.f;
+                            hb |= hit ? bit[k] : 0u;
+                            fold_any(st, r[0][k], hit ? dens[k] : 0.f, r[1][k], r[2][k], r[3][k], r[4][k], r[5][k]);
                         }
                     } else {
                         for (int k = 0; k < 4 && j + k < j1; ++k) {
@@ -987,30 +956,120 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
     }
 }
 
-template <int NT, int B, class V>
-__global__ void __launch_bounds__(NT, (NT >= 64 ? 1024 / NT : 32)) blend_fwd_dense_kernel(
-    const int32_t* __restrict__ ids, const int2* __restrict__ ranges, const float4* __restrict__ recs,
-    const float2* __restrict__ jitter, const __grid_constant__ V views, float4* __restrict__ out_img,
-    float* __restrict__ out_dist, int32_t* __restrict__ out_nc, const Queue q) {
-    __shared__ FwdDenseSmem<B> S;
-    __shared__ int s_item;
-    const int n_items = queue_items(q);
-    const HitMasks hm = live_masks(q.hm, q.subs);
-    for (;;) {
-        const int item = next_item(q, &s_item);
-        if (item >= n_items) return;
-        const int t = queue_tile(q, item), v = views.find(t);
-        const int tb = views.tile_base(v);
-        const int64_t pb = views.pixel_base(v);
-        fwd_dense_item<NT, B>(t - tb, item % q.subs, ids, ranges + tb, recs, jitter + pb, views.camera(v),
-                              out_img + pb, out_dist + 5 * pb, out_nc + pb, S, hm, q.subs, t, q);
+// Warp forward item: half of a 64-pixel strip (8x4 pixels; a whole strip of
+// 16), one lane per pixel, the list walked by one warp on its own: each block
+// of 32 records is copied to the warp's shared memory (asynchronous 16-byte
+// copies, eight lanes to a record's line; one lane per record took six times
+// the L1 lookups), each lane looks at one entry, and those that the warp's
+// rays can hit (entry_reaches) are walked in order.  No exchange of results and no barrier across warps: a third fewer instructions
+// per ray/tet test than the pair items, but a list's walk takes as long as one
+// warp needs, so only lists that many other warps outlast come here
+// (order_kernel).
+struct FwdWarpSmem {
+    float4 srec[32][kRecFloat4 + 1];  // padded: 32 lanes read one record each without conflicts
+};
+
+template <int PX>
+__device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const int32_t* __restrict__ ids,
+                                              const int2* __restrict__ ranges, const float4* __restrict__ recs,
+                                              const float2* __restrict__ jitter, const rm_camera& cam,
+                                              float4* __restrict__ out_img, float* __restrict__ out_dist,
+                                              int32_t* __restrict__ out_nc, FwdWarpSmem& S, const HitMasks& hm,
+                                              int subs, int gtile, const Queue& lq) {
+    const int lane = threadIdx.x & 31;
+    const int2 rg = __ldg(ranges + tile);
+    const int p = half * 32 + lane;
+    const int tx = tile % cam.grid_width, ty = tile / cam.grid_width;
+    int lx, ly;
+    strip_pixel<PX>(cam, sub, p, lx, ly);
+    const int px = tx * cam.tile_width + lx, py = ty * cam.tile_height + ly;
+    const bool inside = p < PX && px < cam.image_width && py < cam.image_height;
+    const int64_t pix = (int64_t)py * cam.image_width + px;
+    const float* M = cam.world_view;
+    f3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f};
+    float u = 0.f, v = 0.f, z = 3e38f;
+    if (inside) {
+        const float2 j = __ldg(jitter + pix);
+        make_ray(cam, px, py, j.x, j.y, o, d);
+        z = dot3(mk3(M[8], M[9], M[10]), d);
+        u = dot3(mk3(M[0], M[1], M[2]), d) / z;
+        v = dot3(mk3(M[4], M[5], M[6]), d) / z;
+    }
+#pragma unroll
+    for (int off = 16; off; off >>= 1) z = fminf(z, __shfl_xor_sync(0xffffffffu, z, off));
+    const float inv_z = bundle_inv_z(cam, z);
+    Bundle bd;
+    auto bounds = [&](bool in) {
+        bd = {in ? u : 3e38f, in ? u : -3e38f, in ? v : 3e38f, in ? v : -3e38f};
+#pragma unroll
+        for (int off = 16; off; off >>= 1)
+            bd = {fminf(bd.u0, __shfl_xor_sync(0xffffffffu, bd.u0, off)),
+                  fmaxf(bd.u1, __shfl_xor_sync(0xffffffffu, bd.u1, off)),
+                  fminf(bd.v0, __shfl_xor_sync(0xffffffffu, bd.v0, off)),
+                  fmaxf(bd.v1, __shfl_xor_sync(0xffffffffu, bd.v1, off))};
+    };
+    PixelState st = {{0.f, 0.f, 0.f}, 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}};
+    int32_t nc = rg.y - rg.x;  // entries walked: all of them unless log T runs out
+    bool active = inside && nc > 0;
+    bounds(active);
+    int32_t g = rg.x + lane < rg.y ? list_id(ids, rg.x + lane, lq) : -1;  // this lane's entry of the next block
+    for (int base = rg.x; base < rg.y && __any_sync(0xffffffffu, active); base += 32) {
+        if (PX == 64 && active) write_checkpoint(hm, st, rg.x, base, sub, subs, p);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int k = 4 * i + (lane >> 3);
+            const int32_t gk = __shfl_sync(0xffffffffu, g, k);
+            if (gk >= 0) async_copy16(&S.srec[k][lane & 7], recs + (int64_t)kRecFloat4 * gk + (lane & 7));
+        }
+        const bool valid = g >= 0;
+        g = base + 32 + lane < rg.y ? list_id(ids, base + 32 + lane, lq) : -1;
+        async_wait();
+        __syncwarp();
+        const bool keep = valid && S.srec[lane][0].w > 0.f &&  // a density of zero hits nothing
+                          (!(inv_z > 0.f) || entry_reaches(S.srec[lane], cam, bd, inv_z));
+        const uint32_t bal = __ballot_sync(0xffffffffu, keep);
+        uint32_t hb = 0;  // bit k: entry k of the block was a hit for this lane's pixel
+        bool ended = false;
+        if (active) {
+            for (uint32_t left = bal; left; left &= left - 1u) {
+                const int j = __ffs(left) - 1;
+                const EntryResult e = eval_entry(S.srec[j], o, d);
+                if (e.a > 0.f) {
+                    hb |= 1u << j;
+                    fold_hit(st, e.a, S.srec[j][0].w, e.m1, e.d4, e.rgb);
+                    if (st.logT < kTermLogT) {
+                        nc = base - rg.x + j + 1;
+                        ended = true;
+                        break;
+                    }
+                }
+            }
+        }
+        if (PX == 64 && hm.words) {
+            const int64_t i = mask_word(gtile, rg.x, (base - rg.x) >> 5, sub, subs, p);
+            if (i < hm.cap) __stcg(hm.words + i, hb);
+        }
+        if (__any_sync(0xffffffffu, ended)) {
+            active = active && !ended;
+            bounds(active);
+        }
+        __syncwarp();  // the walk's reads of the records are done
+    }
+    if (inside) {
+        out_img[pix] = make_float4(st.c[0], st.c[1], st.c[2], st.logT);
+        float* dd = out_dist + 5 * pix;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) dd[k] = st.D[k];
+        out_nc[pix] = nc;
     }
 }
 
-// MINB resident CTAs per SM: 1024 / NT caps registers at 64 (some spill),
-// 768 / NT at 80 (none spill) for launches asking fewer CTAs per SM.
-template <int PX, int NT, int B, int MINB, class V>
-__global__ void __launch_bounds__(NT, MINB) blend_fwd_pair_kernel(
+// 768 threads per SM (80 registers): at 1024 (64 registers) the spills cost
+// more than the warps gain, with the little L1 that the shared memory leaves
+// (1.3M tets, 1297x840: 1461 -> 1293 and 1357 -> 1024 us; a batch of four
+// served views 4187 -> 3500 us).
+template <int PX, int NT, int B, class V>
+__global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
     const int32_t* __restrict__ ids, const int2* __restrict__ ranges, const float4* __restrict__ recs,
     const float2* __restrict__ jitter, const __grid_constant__ V views, float4* __restrict__ out_img,
     float* __restrict__ out_dist, int32_t* __restrict__ out_nc, const Queue q) {
@@ -1018,6 +1077,7 @@ __global__ void __launch_bounds__(NT, MINB) blend_fwd_pair_kernel(
     FwdPairSmem<PX, B>& S = *reinterpret_cast<FwdPairSmem<PX, B>*>(fwd_smem_raw);
     __shared__ int s_item;
     __shared__ HitMasks hm;  // read once per batch: kept out of the registers
+    // first the pair items (the heavy tiles), then each warp on its own
     // the first info[1] tiles of the order go by quarters of their strips
     const int nq = PX == 64 ? __ldg(q.info + 1) : 0;
     const int q_items = nq * q.subs * 4;
@@ -1025,7 +1085,7 @@ __global__ void __launch_bounds__(NT, MINB) blend_fwd_pair_kernel(
     if (threadIdx.x == 0) hm = live_masks(q.hm, q.subs);  // seen after next_item's barriers
     for (;;) {
         int item = next_item(q, &s_item);
-        if (item >= n_items) return;
+        if (item >= n_items) break;
         int quarter = -1, at = 0;
         if (item < q_items) {
             quarter = item & 3;
@@ -1040,6 +1100,22 @@ __global__ void __launch_bounds__(NT, MINB) blend_fwd_pair_kernel(
         fwd_pair_item<PX, NT, B>(t - tb, item % q.subs, quarter, ids, ranges + tb, recs, jitter + pb, views.camera(v),
                                  out_img + pb, out_dist + 5 * pb, out_nc + pb, S, hm, q.subs, t, q);
     }
+    constexpr int kParts = PX / 32 > 0 ? PX / 32 : 1;
+    FwdWarpSmem& W = reinterpret_cast<FwdWarpSmem*>(fwd_smem_raw)[threadIdx.x >> 5];
+    const int heavy = __ldg(q.info);
+    const int w_items = (q.G - heavy) * q.subs * kParts;
+    for (;;) {
+        int item = 0;
+        if ((threadIdx.x & 31) == 0) item = (int)atomicAdd(q.ticket + 1, 1u);
+        item = __shfl_sync(0xffffffffu, item, 0);
+        if (item >= w_items) return;
+        const int part = item % kParts, strip = item / kParts;
+        const int t = __ldg(q.order + heavy + strip / q.subs), v = views.find(t);
+        const int tb = views.tile_base(v);
+        const int64_t pb = views.pixel_base(v);
+        fwd_warp_item<PX>(t - tb, strip % q.subs, part, ids, ranges + tb, recs, jitter + pb, views.camera(v),
+                          out_img + pb, out_dist + 5 * pb, out_nc + pb, W, hm, q.subs, t, q);
+    }
 }
 
 // Orders the tiles heaviest first by floor(log2(list length)) (the order
@@ -1050,7 +1126,7 @@ __global__ void __launch_bounds__(1024) order_kernel(const int2* __restrict__ ra
                                                      int32_t* __restrict__ order, int32_t* info,
                                                      uint32_t* tickets, int heavy_shift, uint32_t* mask_header,
                                                      const MaskHeader mh, const uint32_t* seg_header,
-                                                     int quarter_slots) {
+                                                     int fwd_slots) {
     // Warp-aggregated counting: lanes that share a bucket elect one leader
     // (match_any) for the shared atomic, and the list-length sum and the
     // non-empty count are reduced per warp before one shared update each.
@@ -1101,7 +1177,14 @@ __global__ void __launch_bounds__(1024) order_kernel(const int2* __restrict__ ra
         }
         const uint32_t mean = ne ? (uint32_t)(sum / ne) : 0u;
         // heavy_shift 1 sends every tile to the pair kernel, 0 none
-        const int b_thr = heavy_shift == 1 ? 0 : heavy_shift == 0 ? 33 : max(11, 32 - __clz(mean) + heavy_shift);
+        int b_thr = heavy_shift == 1 ? 0 : heavy_shift == 0 ? 33 : max(11, 32 - __clz(mean) + heavy_shift);
+        if (heavy_shift == 0 && fwd_slots > 0) {
+            // forward, by itself: a strip is walked by two of the 8 warps of a
+            // resident CTA unless its list is longer than a warp's share of
+            // all entries
+            const unsigned long long share = sum / (8ull * fwd_slots);
+            while (b_thr > 1 && (1ull << (b_thr - 2)) >= share) --b_thr;
+        }
         int heavy = 0;
         for (int b = 32; b >= b_thr; --b) heavy += (int)cnt[b];
         info[0] = heavy;
@@ -1109,8 +1192,8 @@ __global__ void __launch_bounds__(1024) order_kernel(const int2* __restrict__ ra
         // entries go by quarters: walked by one CTA each, they would outlast
         // the launch.  A launch with fewer strips than CTAs splits most.
         int quarters = 0;
-        if (quarter_slots > 0) {
-            const unsigned long long share = sum / quarter_slots;
+        if (fwd_slots > 0) {
+            const unsigned long long share = sum / (4ull * fwd_slots);
             for (int b = 32; b > 0 && (1ull << (b - 1)) >= share; --b) quarters += (int)cnt[b];
         }
         info[1] = min(quarters, heavy);
@@ -2492,9 +2575,9 @@ int side_stream(cudaStream_t caller, SideStream** out) {
 
 int launch_order(const int32_t* ranges, int G, const BlendWs& w, int heavy_shift, cudaStream_t s,
                  uint32_t* mask_header = nullptr, MaskHeader mh = MaskHeader{}, const uint32_t* seg_header = nullptr,
-                 int quarter_slots = 0) {
+                 int fwd_slots = 0) {
     order_kernel<<<1, 1024, 0, s>>>((const int2*)ranges, G, w.order, w.info, w.tickets, heavy_shift, mask_header, mh,
-                                    seg_header, quarter_slots);
+                                    seg_header, fwd_slots);
     return rm_host::check_launch("rm_blend order");
 }
 
@@ -2539,53 +2622,32 @@ struct Shape {
     int tile_px;
 };
 
-// Forward pass: order kernel, then the pair kernel (heavy tiles) and the
-// dense kernel (other tiles).  When every tile is heavy the pair kernel runs
-// alone on the caller's stream; otherwise it runs on the side stream
-// concurrently with the dense kernel and is joined back after both launches.
-template <int PX, int B_DENSE, int PX_PAIR, int NT_PAIR, int B_PAIR, class V>
+// Forward pass: order kernel, then one persistent kernel for the heavy tiles
+// (pair items) and the others (warp items).
+template <int PX, int NT, int B, class V>
 int launch_fwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, const float* jitter, const V& views,
                const Shape& sh, float* img, float* dist, int32_t* nc, const Tuning& tn, cudaStream_t s) {
     const int G = sh.G;
-    // hit masks need 64-pixel items in both kernels; the header records whether
-    // this forward wrote them, so a backward never reads stale masks
-    const bool masks = tn.hit_masks && PX == 64 && PX_PAIR == 64 && w.mask_header;
+    // hit masks need 64-pixel items; the header records whether this forward
+    // wrote them, so a backward never reads stale masks
+    const bool masks = tn.hit_masks && PX == 64 && w.mask_header;
     const int subs = sh.tile_px / PX;
-    const int subs_pair = sh.tile_px / PX_PAIR;
-    const int pair_cap = tn.pair_ctas_per_sm * sm_count();
-    int rc = launch_order(ranges, G, w, tn.heavy_shift, s, w.mask_header,
-                          masks ? mask_header_for(w.mask_cap, G, subs) : MaskHeader{}, nullptr,
-                          PX_PAIR == 64 ? (pair_cap > subs_pair ? pair_cap / subs_pair : 1) : 0);
+    const int cap = tn.pair_ctas_per_sm * sm_count();
+    int rc = launch_order(ranges, G, w, PX == 64 ? tn.heavy_shift : tn.heavy_shift == 0 ? 1 : tn.heavy_shift, s,
+                          w.mask_header, masks ? mask_header_for(w.mask_cap, G, subs) : MaskHeader{}, nullptr,
+                          PX == 64 ? (cap > subs ? cap / subs : 1) : 0);
     if (rc) return rc;
     const HitMasks hm = {masks ? w.mask_words : nullptr, w.mask_cap, w.mask_header, nullptr, 0, kNoSegments};
-    const Queue qd = {w.order, w.info, w.tickets + 0, G, subs, false, hm, tn.status, rm_host::wait_limit(),
-                      tn.n_recs};
-    const Queue qp = {w.order, w.info, w.tickets + 1, G, subs_pair, true, hm, tn.status, rm_host::wait_limit(),
-                      tn.n_recs};
-    auto pair_kernel = tn.pair_ctas_per_sm * NT_PAIR >= 1024
-                           ? blend_fwd_pair_kernel<PX_PAIR, NT_PAIR, B_PAIR, 1024 / NT_PAIR, V>
-                           : blend_fwd_pair_kernel<PX_PAIR, NT_PAIR, B_PAIR, 768 / NT_PAIR, V>;
-    const int smem = (int)sizeof(FwdPairSmem<PX_PAIR, B_PAIR>);
-    cudaFuncSetAttribute(pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    const int64_t pair_items = (int64_t)G * subs_pair * (PX_PAIR == 64 ? 4 : 1);
-    const int pair_grid = pair_items < pair_cap ? (int)pair_items : pair_cap;
-    if (tn.heavy_shift == 1) {
-        pair_kernel<<<pair_grid, NT_PAIR, smem, s>>>(ids, (const int2*)ranges, w.recs, (const float2*)jitter, views,
-                                                     (float4*)img, dist, nc, qp);
-        return rm_host::check_launch("rm_blend_fwd (pair)");
-    }
-    std::lock_guard<std::mutex> lock(g_side_mu);
-    SideStream* side = nullptr;
-    if ((rc = side_stream(s, &side)) || (rc = fork_side(s, side))) return rc;
-    pair_kernel<<<pair_grid, NT_PAIR, smem, side->stream>>>(ids, (const int2*)ranges, w.recs, (const float2*)jitter,
-                                                            views, (float4*)img, dist, nc, qp);
-    if ((rc = rm_host::check_launch("rm_blend_fwd (pair)"))) return rc;
-    auto dense_kernel = blend_fwd_dense_kernel<PX, B_DENSE, V>;
-    const int grid = persistent_grid(dense_kernel, PX, 0, G * subs);
-    dense_kernel<<<grid, PX, 0, s>>>(ids, (const int2*)ranges, w.recs, (const float2*)jitter, views, (float4*)img,
-                                     dist, nc, qd);
-    if ((rc = rm_host::check_launch("rm_blend_fwd (dense)"))) return rc;
-    return join_side(s, side);
+    const Queue q = {w.order, w.info, w.tickets + 0, G, subs, true, hm, tn.status, rm_host::wait_limit(), tn.n_recs};
+    auto kernel = blend_fwd_kernel<PX, NT, B, V>;
+    constexpr int kPairSmem = (int)sizeof(FwdPairSmem<PX, B>), kWarpSmem = NT / 32 * (int)sizeof(FwdWarpSmem);
+    constexpr int smem = kPairSmem > kWarpSmem ? kPairSmem : kWarpSmem;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int64_t items = (int64_t)G * subs * (PX == 64 ? 4 : 1);
+    const int grid = items < cap ? (int)items : cap;
+    kernel<<<grid, NT, smem, s>>>(ids, (const int2*)ranges, w.recs, (const float2*)jitter, views, (float4*)img, dist,
+                                  nc, q);
+    return rm_host::check_launch("rm_blend_fwd");
 }
 
 template <int PX, int B_DENSE, int PX_PAIR, int NT_PAIR, int B_PAIR, class V>
@@ -2729,15 +2791,14 @@ int blend_fwd_any(const char* who, const int32_t* sorted_ids, const int32_t* ran
         rc = pack(indices, vertices, n_verts, cell_values, n_tets, tiles_touched, w.recs, s);
         if (rc) return rc;
     }
-    // measured on the 1.3M-tet workload: every tile through the pair kernel, 4 CTAs/SM
-    Tuning tn = tuning_from_flags(flags, 1, 4);
+    Tuning tn = tuning_from_flags(flags, 0, 3);
     tn.n_recs = n_tets;
     if ((rc = pass_status(who, w, status_dev, s, &tn.status))) return rc;
-    // tets per shared-memory batch of the pair kernel: 16, 32 (default) or 64
+    // tets per shared-memory batch of the pair items: 16, 32 (default) or 64
     const int key = strip_pixels(cam0, flags) * 1000 + batch_size(flags, 32);
 #define RM_FWD_CASE(PX, NT, BP)                                                                                  \
     case PX * 1000 + BP:                                                                                         \
-        return launch_fwd<PX, 64, PX, NT, BP>(sorted_ids, ranges, w, ray_jitter, views, sh, out_img, out_distortion, \
+        return launch_fwd<PX, NT, BP>(sorted_ids, ranges, w, ray_jitter, views, sh, out_img, out_distortion, \
                                               n_contrib, tn, s);
     switch (key) {
         RM_FWD_CASE(16, 64, 16)
