@@ -205,8 +205,8 @@ __device__ __forceinline__ Weights seg_weights(float x) {
 // d phi / dx = -(d w1 / dx): series below 0.25, (alpha - phi) / x = -w0 / x above.
 __device__ __forceinline__ float dphi_f(float x, const Weights& w) {
     if (x < 0.25f)
-        return -(0.5f + x * (-1.0f / 3.0f + x * (0.125f + x * (-1.0f / 30.0f + x * (1.0f / 144.0f +
-                 x * (-1.0f / 840.0f))))));
+        return -fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, -1.0f / 840.0f, 1.0f / 144.0f), -1.0f / 30.0f), 0.125f),
+                             -1.0f / 3.0f), 0.5f);
     return -__fdividef(w.w0, x);
 }
 
@@ -273,7 +273,6 @@ template <int NT>
 struct WarpShape {
     static constexpr unsigned kMask = NT >= 32 ? 0xffffffffu : ((1u << NT) - 1u);
     static constexpr int kTopOffset = NT >= 32 ? 16 : NT / 2;
-    static constexpr int kWarps = NT >= 32 ? NT / 32 : 1;
 };
 
 // Hit masks written by the forward and read by the backward
@@ -384,7 +383,6 @@ __device__ __forceinline__ int queue_tile(const Queue& q, int item) {
 // order_kernel: entry 32 - b = first segment item of bucket b (without the
 // strips), down to bucket seg_shift, where the one-segment tiles begin.
 constexpr int kSegInfoOff = 33;  // of the workspace's info words (after the status word)
-constexpr int kSegInfoLen = 31;
 
 struct SegItem {
     int tile, seg, sub;
@@ -440,17 +438,6 @@ __device__ __forceinline__ int32_t list_id(const int32_t* __restrict__ ids, int6
 
 __device__ __forceinline__ float4 record_part(const float4* __restrict__ recs, int32_t g, int c) {
     return g >= 0 ? __ldg(recs + (int64_t)kRecFloat4 * g + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-}
-
-// Stores the hit bits of one batch (B a multiple of 32, starting 32-aligned
-// relative to the list start) for pixel p: one word per 32 entries.
-__device__ __forceinline__ void write_masks(const HitMasks& hm, uint64_t hb, int gtile, int x, int base, int n,
-                                            int sub, int subs, int p) {
-    const int k0 = (base - x) >> 5;
-    for (int w = 0; w * 32 < n; ++w) {
-        const int64_t i = mask_word(gtile, x, k0 + w, sub, subs, p);
-        if (i < hm.cap) __stcg(hm.words + i, (uint32_t)(hb >> (32 * w)));
-    }
 }
 
 // Stores the checkpoint of pixel p (p of the strip's 64) at list position
@@ -1525,35 +1512,132 @@ __device__ __forceinline__ uint32_t bits_below(uint32_t w, int n) {
     return n <= 0 ? 0u : n >= 32 ? w : w & ((1u << n) - 1u);
 }
 
-// Dense backward item: a strip of NT pixels, one thread per pixel walking its
-// list back to front from the saved final state.
-template <int NT, int B>
-struct BwdDenseSmem {
-    float4 srec[B][kRecFloat4];
-    float4 red[NT >= 32 ? NT / 32 : 1][NT >= 32 ? 32 * kRedStride / 4 : 1];  // warp_sum_rows_planes rows, per warp
-    int32_t sid[B];
-    float sacc[B][kNGrad];
-    int32_t smax[WarpShape<NT>::kWarps];
-    uint32_t sor[WarpShape<NT>::kWarps][2];  // per warp: OR of its pixels' hit bits (two 32-entry blocks)
-    uint8_t cidx[B];                          // batch positions of the entries some pixel hit
-    int32_t n_keep;
+// Warp backward item: half of a 64-pixel strip (8x4 pixels; a whole strip of
+// 16) over one stretch of a tile's list, walked back to front by one warp, one
+// pixel per lane.  Per block of 32 entries (one mask word per pixel) the
+// records of the entries some pixel hit are copied to the warp's shared
+// memory and walked; each entry is met once, so its sums over the lanes are
+// final when formed (no accumulators to clear, no atomics in shared memory)
+// and are turned into vertex and cell-value gradients for all 32 entries at
+// once, one entry per lane, at the end of the block.
+//
+// Per hit the lane forms 23 partials: for each face p the sums G_p of
+// dL/dt / dot(n_p, d) over the hits that enter or leave through it and H_p of
+// the same times the hit point relative to v0, density, rgb and the colour
+// gradient.  The gradient of the face normals, of v0 and v1 follow from them
+// once per entry (flush_sums): with t_p = dot(n_p, v_ref - o) / dot(n_p, d),
+// dt/dn = -(hit point - v_ref) / dot(n, d) and dt/dv_ref = n / dot(n, d).
+//
+// Bound: instruction issue, about 300 instructions for an entry and up to 32
+// pixels (540 before: 25 partials formed with separate multiplies and adds,
+// normals and reference points selected per lane, CTA barriers per batch).
+struct BwdWarpSmem {
+    float4 srec[32][kRecFloat4 + 1];
+    float4 red[32 * kRedStride / 4];  // one row of partials per lane
+    float4 sums[32][6];               // per entry: (G, H) of the four faces, density rgb, grd 0
 };
 
-template <int NT, int B>
-__device__ __forceinline__ void bwd_dense_item(
-    int tile, int sub, const int32_t* __restrict__ ids, const int2* __restrict__ ranges,
+// Adds up the 24 columns of the lanes' rows: the lane's group (lane / 8) takes
+// eight rows, its place in it (< 6) four columns; the groups meet by shuffles.
+// Rows of the lanes in bal_a go to a, the others to b (SPLIT) or to a too.
+template <bool SPLIT>
+__device__ __forceinline__ void warp_sum_rows(const float4* __restrict__ red, int lane, uint32_t bal_a, float4& a,
+                                              float4& b) {
+    const int quad = lane & 7, row0 = lane & 24;
+    a = make_float4(0.f, 0.f, 0.f, 0.f);
+    b = a;
+    __syncwarp();
+    if (quad < 6) {
+        const uint32_t in = bal_a >> row0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const float4 v = red[(row0 + r) * (kRedStride / 4) + quad];
+            if (!SPLIT || ((in >> r) & 1u)) {
+                a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+            } else {
+                b.x += v.x; b.y += v.y; b.z += v.z; b.w += v.w;
+            }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int off = 8; off <= 16; off <<= 1) {
+        a.x += __shfl_xor_sync(0xffffffffu, a.x, off);
+        a.y += __shfl_xor_sync(0xffffffffu, a.y, off);
+        a.z += __shfl_xor_sync(0xffffffffu, a.z, off);
+        a.w += __shfl_xor_sync(0xffffffffu, a.w, off);
+        if (SPLIT) {
+            b.x += __shfl_xor_sync(0xffffffffu, b.x, off);
+            b.y += __shfl_xor_sync(0xffffffffu, b.y, off);
+            b.z += __shfl_xor_sync(0xffffffffu, b.z, off);
+            b.w += __shfl_xor_sync(0xffffffffu, b.w, off);
+        }
+    }
+}
+
+// One entry's sums -> gradients of its four vertices and seven cell values,
+// added to global memory by one thread.
+__device__ __forceinline__ void flush_sums(const float4* __restrict__ q, const float4* __restrict__ s, int32_t g,
+                                           const int4* __restrict__ indices, float* __restrict__ gverts,
+                                           float* __restrict__ gcv) {
+    const f3 P[4] = {xyz(q[4]), xyz(q[5]), xyz(q[6]), xyz(q[7])};
+    const uint32_t flips = __float_as_uint(q[7].w);
+    const float4 c = s[4];  // density, r, g, b
+    const float4 k = s[5];  // grd
+    const float dsum = -(c.y + c.z + c.w);
+    f3 gv[4] = {{q[4].w * dsum, q[5].w * dsum, q[6].w * dsum}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+    const int pp[4] = {1, 1, 2, 2}, pq[4] = {0, 0, 0, 1}, pr[4] = {2, 3, 3, 3};
+    bool any = c.x != 0.f || c.y != 0.f || c.z != 0.f || c.w != 0.f || k.x != 0.f || k.y != 0.f || k.z != 0.f;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const float4 h = s[p];  // (G, H)
+        any |= h.x != 0.f || h.y != 0.f || h.z != 0.f || h.w != 0.f;
+        const f3 n = xyz(q[p]);
+        f3& ref = gv[pq[p]];
+        ref = {fmaf(n.x, h.x, ref.x), fmaf(n.y, h.x, ref.y), fmaf(n.z, h.x, ref.z)};
+        f3 gc = {-h.y, -h.z, -h.w};  // gradient of the normal
+        if (p == 3) {
+            const f3 e = P[1] - P[0];
+            gc = {fmaf(e.x, h.x, gc.x), fmaf(e.y, h.x, gc.y), fmaf(e.z, h.x, gc.z)};
+        }
+        if (flips & (1u << p)) gc = neg3(gc);
+        const f3 ea = P[pp[p]] - P[pq[p]], eb = P[pr[p]] - P[pq[p]];
+        const f3 ga = cross3(eb, gc), gb = cross3(gc, ea);
+        gv[pp[p]] = gv[pp[p]] + ga;
+        gv[pr[p]] = gv[pr[p]] + gb;
+        ref = ref - (ga + gb);
+    }
+    if (!any) return;
+    const int4 id = __ldg(indices + g);
+    const int vid[4] = {id.x, id.y, id.z, id.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float* dst = gverts + 3 * (int64_t)vid[i];
+        if (gv[i].x != 0.f) atomicAdd(dst, gv[i].x);
+        if (gv[i].y != 0.f) atomicAdd(dst + 1, gv[i].y);
+        if (gv[i].z != 0.f) atomicAdd(dst + 2, gv[i].z);
+    }
+    const float out[7] = {c.x, c.y, c.z, c.w, k.x, k.y, k.z};
+    float* dc = gcv + 7 * (int64_t)g;
+#pragma unroll
+    for (int i = 0; i < 7; ++i)
+        if (out[i] != 0.f) atomicAdd(dc + i, out[i]);
+}
+
+template <int PX>
+__device__ __forceinline__ void bwd_warp_item(
+    int tile, int sub, int half, int seg, const int32_t* __restrict__ ids, const int2* __restrict__ ranges,
     const float4* __restrict__ recs, const int4* __restrict__ indices, const float2* __restrict__ jitter,
     const rm_camera& cam, const float4* __restrict__ img, const float* __restrict__ dist,
     const int32_t* __restrict__ ncs, const float4* __restrict__ gimg, const float* __restrict__ gdist,
-    float* __restrict__ gverts, float* __restrict__ gcv, BwdDenseSmem<NT, B>& S, const HitMasks& hm, int subs, int gtile,
-    const Queue& lq, int seg) {
-    constexpr unsigned kMask = WarpShape<NT>::kMask;
-    constexpr bool kMasks = NT == 64;
+    float* __restrict__ gverts, float* __restrict__ gcv, BwdWarpSmem& S, const HitMasks& hm, int subs, int gtile,
+    const Queue& lq) {
+    constexpr unsigned kAll = 0xffffffffu;
     const int2 rg = __ldg(ranges + tile);
     const int len = rg.y - rg.x;
     // this item's stretch [s0, s1) of the list, as offsets from its start
     int s0 = 0, s1 = len;
-    if (kMasks && hm.ck && len > (1 << hm.seg_shift)) {
+    if (hm.ck && len > (1 << hm.seg_shift)) {
         const int shift = hm.seg_shift;
         if (ck_id(rg.x, (len - 1) >> shift, shift) < hm.ck_cap) {
             s0 = seg << shift;
@@ -1565,185 +1649,177 @@ __device__ __forceinline__ void bwd_dense_item(
         return;
     }
     if (s0 >= s1) return;
+    const int lane = threadIdx.x & 31;
+    const int p = half * 32 + lane;
     const int tx = tile % cam.grid_width, ty = tile / cam.grid_width;
     int lx, ly;
-    strip_pixel<NT>(cam, sub, (int)threadIdx.x, lx, ly);
+    strip_pixel<PX>(cam, sub, p, lx, ly);
     const int px = tx * cam.tile_width + lx, py = ty * cam.tile_height + ly;
-    const bool inside = px < cam.image_width && py < cam.image_height;
+    const bool inside = p < PX && px < cam.image_width && py < cam.image_height;
     const int64_t pix = (int64_t)py * cam.image_width + px;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int32_t nc = inside ? __ldg(ncs + pix) : 0;
+    if (nc <= s0) nc = 0;
+    if (!__any_sync(kAll, nc > 0)) return;  // every pixel's walk ends before this stretch
     f3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f};
     float logT = 0.f, D2 = 0.f, D3 = 0.f;  // state along the reverse walk
     float dS_c[3] = {0.f, 0.f, 0.f}, dS_logT = 0.f, dS_D[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    int32_t nc = inside ? __ldg(ncs + pix) : 0;
-    if (s0 > 0 && !__syncthreads_or(nc > s0)) return;  // every pixel's walk ends before this stretch
-    if (nc <= s0) nc = 0;
     if (nc > 0) {
         const float2 j = __ldg(jitter + pix);
         make_ray(cam, px, py, j.x, j.y, o, d);
-        logT = __ldg(img + pix).w;
+        const float4 c = __ldg(img + pix);
+        logT = c.w;
         D2 = __ldg(dist + 5 * pix + 2);
         D3 = __ldg(dist + 5 * pix + 3);
         const float4 g = __ldg(gimg + pix);
         dS_c[0] = g.x; dS_c[1] = g.y; dS_c[2] = g.z; dS_logT = g.w;
 #pragma unroll
         for (int k = 0; k < 5; ++k) dS_D[k] = gdist ? __ldg(gdist + 5 * pix + k) : 0.f;
-        if (kMasks && nc > s1) {
-            seed_segment(hm, rg.x, s1, sub, subs, (int)threadIdx.x, __ldg(img + pix), logT, D2, D3, dS_c, dS_logT,
-                         dS_D);
+        if (PX == 64 && nc > s1) {
+            seed_segment(hm, rg.x, s1, sub, subs, p, c, logT, D2, D3, dS_c, dS_logT, dS_D);
             nc = s1;
         }
     }
-    int32_t m = nc;
+    // constants of the walk
+    const float dS0 = 2.0f * dS_D[0], dS1 = 2.0f * dS_D[1], dS4 = dS_D[4] * (1.0f / 3.0f);
+    const float dS_sum = dS_c[0] + dS_c[1] + dS_c[2];
+    float dS2 = dS_D[2], dS3 = dS_D[3];
+    float* const row = reinterpret_cast<float*>(S.red) + lane * kRedStride;
+    float4* const row4 = reinterpret_cast<float4*>(row);
+
+    // A pixel's hit bits of block k: the forward's word, all entries without
+    // one; none at or past n_contributors.
+    auto hit_word = [&](int k) {
+        uint32_t w = 0xffffffffu;
+        if (PX == 64 && hm.words) {
+            const int64_t i = mask_word(gtile, rg.x, k, sub, subs, p);
+            if (i < hm.cap) w = __ldcg(hm.words + i);
+        }
+        return bits_below(w, nc - 32 * k);
+    };
+    const int last = (int)__reduce_max_sync(kAll, (unsigned)nc);
+    int k = (last - 1) >> 5;
+    uint32_t w = hit_word(k);
+    for (; k >= s0 >> 5; --k) {
+        const uint32_t cur = w;
+        if (k > s0 >> 5) w = hit_word(k - 1);  // the next block's, ahead of its use
+        const uint32_t any = __reduce_or_sync(kAll, cur);
+        if (!any) continue;
+        int32_t g = -1;
+        if ((any >> lane) & 1u) g = list_id(ids, rg.x + 32 * k + lane, lq);
 #pragma unroll
-    for (int off = WarpShape<NT>::kTopOffset; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(kMask, m, off));
-    if (lane == 0) S.smax[warp] = m;
-    __syncthreads();
-    int32_t tile_max = 0;
-#pragma unroll
-    for (int w = 0; w < WarpShape<NT>::kWarps; ++w) tile_max = max(tile_max, S.smax[w]);
-    const int end = min(rg.x + s1, rg.x + tile_max);
-    // batches aligned to multiples of B from the list start, so that one spans
-    // at most two 32-entry mask blocks (B <= 64)
-    for (int top = end, lo; top > rg.x + s0; top = lo) {
-        lo = rg.x + ((top - 1 - rg.x) / B) * B;
-        const int n = top - lo;
-        __syncthreads();
-        // this pixel's hit bits of the (at most two) 32-entry blocks the batch spans
-        const int kb0 = (lo - rg.x) >> 5, kb1 = (top - 1 - rg.x) >> 5;
-        uint32_t hw0 = 0xffffffffu, hw1 = 0xffffffffu;
-        if (kMasks && hm.words) {
-            const int64_t i0 = mask_word(gtile, rg.x, kb0, sub, subs, (int)threadIdx.x);
-            const int64_t i1 = mask_word(gtile, rg.x, kb1, sub, subs, (int)threadIdx.x);
-            if (i0 < hm.cap) hw0 = __ldcg(hm.words + i0);
-            if (i1 < hm.cap) hw1 = __ldcg(hm.words + i1);
+        for (int i = 0; i < 8; ++i) {
+            const int e = 4 * i + (lane >> 3);
+            const int32_t ge = __shfl_sync(kAll, g, e);
+            if (ge >= 0)
+                async_copy16(&S.srec[e][lane & 7], recs + (int64_t)kRecFloat4 * ge + (lane & 7));
+            else if ((any >> e) & 1u)
+                S.srec[e][lane & 7] = make_float4(0.f, 0.f, 0.f, 0.f);  // names no tet: nothing hits it
         }
-        hw0 = bits_below(hw0, nc - kb0 * 32);
-        hw1 = bits_below(hw1, nc - kb1 * 32);
-        // entries no pixel of the item hit are dropped from the batch before
-        // staging (the bits at and past n_contributors, which the forward may
-        // have left unwritten, are cleared above)
-        uint32_t o0 = hw0, o1 = hw1;
-#pragma unroll
-        for (int off = WarpShape<NT>::kTopOffset; off > 0; off >>= 1) {
-            o0 |= __shfl_xor_sync(kMask, o0, off);
-            o1 |= __shfl_xor_sync(kMask, o1, off);
-        }
-        if (lane == 0) {
-            S.sor[warp][0] = o0;
-            S.sor[warp][1] = o1;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            uint32_t c0 = 0, c1 = 0;
-#pragma unroll
-            for (int w = 0; w < WarpShape<NT>::kWarps; ++w) {
-                c0 |= S.sor[w][0];
-                c1 |= S.sor[w][1];
-            }
-            int base_c = 0;
-            constexpr int kLanes = NT >= 32 ? 32 : NT;
-            for (int k0 = 0; k0 < n; k0 += kLanes) {
-                const int k = k0 + lane;
-                bool keep = false;
-                if (k < n) {
-                    const int off = lo + k - rg.x;
-                    keep = ((((off >> 5) == kb0 ? c0 : c1) >> (off & 31)) & 1u) != 0u;
-                }
-                const unsigned bal = __ballot_sync(kMask, keep);
-                if (keep) S.cidx[base_c + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)k;
-                base_c += __popc(bal);
-            }
-            if (lane == 0) S.n_keep = base_c;
-        }
-        __syncthreads();
-        const int nk = S.n_keep;
-        for (int k = threadIdx.x; k < nk; k += NT) S.sid[k] = list_id(ids, lo + S.cidx[k], lq);
-        for (int k = threadIdx.x; k < nk * kNGrad; k += NT) (&S.sacc[0][0])[k] = 0.f;
-        __syncthreads();
-        for (int k = threadIdx.x; k < nk * kRecFloat4; k += NT) {
-            const int j = k >> 3, c = k & 7;
-            S.srec[j][c] = record_part(recs, S.sid[j], c);
-        }
-        __syncthreads();
-        for (int jj = nk - 1; jj >= 0;) {
-            const int off = lo + S.cidx[jj] - rg.x;
-            // with the forward's masks, only its hits are revisited
-            const uint32_t hw = (off >> 5) == kb0 ? hw0 : hw1;
-            const bool act_a = (hw >> (off & 31)) & 1u;
-            const uint32_t bal_a = __ballot_sync(kMask, act_a);
-            if (!bal_a) {
-                --jj;
-                continue;
-            }
-            // When no pixel of the warp walks both this entry and the one
-            // before it, the warp takes both at once: each lane walks the one
-            // it hits (its own order is unchanged), and the partials go to
-            // the two entries' accumulators by lane.
-            bool act_b = false;
-            uint32_t bal_b = 0u;
-            if constexpr (NT >= 32) {
-                if (jj >= 1) {
-                    const int off_b = lo + S.cidx[jj - 1] - rg.x;
-                    const uint32_t hwb = (off_b >> 5) == kb0 ? hw0 : hw1;
-                    act_b = (hwb >> (off_b & 31)) & 1u;
-                    bal_b = __ballot_sync(kMask, act_b);
-                    if (bal_a & bal_b) {
-                        act_b = false;
-                        bal_b = 0u;
-                    }
+        async_wait();
+        __syncwarp();
+        uint32_t left = any, done = 0u;  // entries to walk; entries with sums
+        while (left) {
+            const int ja = 31 - __clz(left);
+            left &= ~(1u << ja);
+            bool act = (cur >> ja) & 1u;
+            uint32_t bal_a = kAll;
+            // When no pixel of the warp hits both this entry and the next one,
+            // the warp takes both at once: each lane walks the one it hits
+            // (its own order is unchanged), and the rows go to the two
+            // entries' sums by lane.
+            int je = ja, jb = -1;
+            if (left) {
+                jb = 31 - __clz(left);
+                const uint32_t both = (1u << ja) | (1u << jb);
+                if (__any_sync(kAll, (cur & both) == both)) {
+                    jb = -1;
+                } else {
+                    left &= ~(1u << jb);
+                    bal_a = __ballot_sync(kAll, act);
+                    const bool act_b = (cur >> jb) & 1u;
+                    je = act_b ? jb : ja;
+                    act |= act_b;
                 }
             }
-            const bool act = act_a || act_b;
-            const int je = act_b ? jj - 1 : jj;
             const float4* q = S.srec[je];
-            float gl[kNGrad];
-#pragma unroll
-            for (int k = 0; k < kNGrad; ++k) gl[k] = 0.f;
             const Isect is = intersect<true>(q, o, d);
             const float density = q[0].w;
-            Segment s;
-            s.dt = fmaxf(is.exit - is.enter, 0.f);
-            s.a = density * s.dt;
-            const bool hit = act && is.geo && s.a > 0.f;
-            f3 dne = {0.f, 0.f, 0.f}, dnx = {0.f, 0.f, 0.f};
+            const float dt = fmaxf(is.exit - is.enter, 0.f);
+            const float a = density * dt;
+            const bool hit = act && is.geo && a > 0.f;
+            const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) row4[c] = z4;
+            float4 g_val = z4, g_grd = z4;
             if (hit) {
-                integrate(q, o, d, is.enter, is.exit, s);
-                // undo_alpha_out (alphablend_shader_interp.slang:128-192): only log T, D2
-                // and D3 of the earlier state enter the adjoint
-                const float m1 = density * (is.exit + is.enter) / 2.0f;
-                const float logT_old = logT + s.a;
-                const float T = __expf(logT_old);
+                // the segment (integrate_tetra_segment), the colour linear along the ray
+                const f3 a0 = xyz(q[4]) - o;
+                const f3 ve = {fmaf(is.enter, d.x, -a0.x), fmaf(is.enter, d.y, -a0.y), fmaf(is.enter, d.z, -a0.z)};
+                const f3 vx = {fmaf(is.exit, d.x, -a0.x), fmaf(is.exit, d.y, -a0.y), fmaf(is.exit, d.z, -a0.z)};
+                const f3 grd = {q[4].w, q[5].w, q[6].w};
+                const f3 base = {q[1].w, q[2].w, q[3].w};
+                const float gd = dot3(grd, d);
+                const float ce = dot3(grd, ve), cx = dot3(grd, vx);
+                const Weights wt = seg_weights(a);
+                const float wsum = wt.w0 + wt.w1;
+                const float lin = fmaf(wt.w0, cx, wt.w1 * ce);
+                // undo_alpha_out (alphablend_shader_interp.slang:128-192): only
+                // log T, D2 and D3 of the earlier state enter the adjoint
+                const float sum_t = is.exit + is.enter;
+                const float m1 = density * sum_t / 2.0f;
+                logT = logT + a;
+                const float T = __expf(logT);
                 D2 = D2 - density;
                 D3 = D3 - m1;
-                logT = logT_old;
-                float nD2, nD3;
-                if constexpr (NT >= 32)
-                    dS_logT = hit_grads_planes(q, xyz(q[4]) - o, xyz(q[5]) - o, d, is, s, T, D2, D3, dS_c, dS_logT,
-                                               dS_D, gl, dne, dnx, nD2, nD3);
-                else
-                    dS_logT = hit_grads(q, o, d, is, s, T, D2, D3, dS_c, dS_logT, dS_D, gl, nD2, nD3);
-                dS_D[2] = nD2;
-                dS_D[3] = nD3;
+                // update_distortion_state
+                const float dm1 = fmaf(dS0, D2, dS3), dm0 = fmaf(dS1, D3, dS2);
+                dS2 = fmaf(dS0, m1, dS2);
+                dS3 = fmaf(dS1, density, dS3);
+                float d_dens = fmaf(dm1, 0.5f * sum_t, dm0);
+                const float half_m = 0.5f * dm1 * density;
+                const float d4 = dS4 * density;
+                float d_dt = d4 * density;
+                d_dens = fmaf(2.0f * d4, dt, d_dens);
+                // update_pixel_state, compute_integral
+                const f3 d_rgb = {dS_c[0] * T, dS_c[1] * T, dS_c[2] * T};
+                const float sum_d = dS_sum * T;
+                const float d_base = dot3(d_rgb, base);
+                const float dT = fmaf(wsum, d_base, lin * sum_d);  // T times dot(dL/dc, rgb)
+                const float d_w0 = fmaf(sum_d, cx, d_base);
+                const float d_sx = sum_d * wt.w0, d_se = sum_d * wt.w1;
+                const float d_x = fmaf(sum_d * (cx - ce), dphi_f(a, wt), d_w0 * wt.alpha) - dS_logT;
+                dS_logT = dS_logT + dT;
+                d_dt = fmaf(d_x, density, d_dt);
+                d_dens = fmaf(d_x, dt, d_dens);
+                // a hit has exit = tx > enter, so both ends move the segment
+                const float d_tx = fmaf(d_sx, gd, half_m) + d_dt;
+                const float d_te = is.te > 0.f ? fmaf(d_se, gd, half_m) - d_dt : 0.f;
+                // gradient factors only (the hit and its t values are exact
+                // above): the approximate quotient (2 ulp) is far inside the
+                // gradients' tolerance
+                const float ge = __fdividef(d_te, is.dene), gx = __fdividef(d_tx, is.denx);
+                if (is.ie >= 0) row4[is.ie] = make_float4(ge, ge * ve.x, ge * ve.y, ge * ve.z);
+                if (is.ix >= 0) row4[is.ix] = make_float4(gx, gx * vx.x, gx * vx.y, gx * vx.z);
+                g_val = make_float4(d_dens, d_rgb.x * wsum, d_rgb.y * wsum, d_rgb.z * wsum);
+                g_grd = make_float4(fmaf(d_se, ve.x, d_sx * vx.x), fmaf(d_se, ve.y, d_sx * vx.y),
+                                    fmaf(d_se, ve.z, d_sx * vx.z), 0.f);
             }
-            if (__any_sync(kMask, hit)) {
-                if constexpr (NT >= 32) {
-                    warp_sum_rows_planes(reinterpret_cast<float*>(S.red[warp]), gl, dne, dnx, hit ? is.ie : -1,
-                                         hit ? is.ix : -1, lane, S.sacc[jj], bal_a,
-                                         bal_b ? S.sacc[jj - 1] : nullptr);
-                } else {
-                    using RS = ReduceScatter<kNGrad, WarpShape<NT>::kTopOffset>;
-                    int slot = 0;
-                    RS::template run<kMask>(gl, lane, slot);
-#pragma unroll
-                    for (int r = 0; r < RS::R; ++r)
-                        if (slot + r < kNGrad && gl[r] != 0.f) atomicAdd(&S.sacc[jj][slot + r], gl[r]);
-                }
+            row4[4] = g_val;
+            row4[5] = g_grd;
+            float4 sa, sb;
+            if (jb < 0) {
+                warp_sum_rows<false>(S.red, lane, bal_a, sa, sb);
+            } else {
+                warp_sum_rows<true>(S.red, lane, bal_a, sa, sb);
+                if (lane < 6) S.sums[jb][lane] = sb;
+                done |= 1u << jb;
             }
-            jj -= bal_b ? 2 : 1;
+            if (lane < 6) S.sums[ja][lane] = sa;
+            done |= 1u << ja;
         }
-        __syncthreads();
-        flush_entries<NT, B>(nk, S.srec, S.sid, S.sacc, indices, gverts, gcv);
+        __syncwarp();
+        if (((done >> lane) & 1u) && g >= 0) flush_sums(S.srec[lane], S.sums[lane], g, indices, gverts, gcv);
+        __syncwarp();  // the next block overwrites the records
     }
 }
 
@@ -2165,47 +2241,52 @@ __device__ __forceinline__ void bwd_pair_item(
     }
 }
 
-// Resident CTAs per SM (of 64 threads) the dense backward is compiled for.
-#ifndef RM_BWD_DENSE_MINB
-#define RM_BWD_DENSE_MINB 8
-#endif
+// Warps per CTA and resident CTAs per SM of the backward's warp items.
+constexpr int kBwdWarps = 4;
+constexpr int kBwdCtas = 4;
 
-template <int NT, int B, class V>
-__global__ void __launch_bounds__(NT, (NT >= 64 ? RM_BWD_DENSE_MINB * 64 / NT : 16)) blend_bwd_dense_kernel(
+template <int PX, class V>
+__global__ void __launch_bounds__(kBwdWarps * 32, kBwdCtas) blend_bwd_warp_kernel(
     const int32_t* __restrict__ ids, const int2* __restrict__ ranges, const float4* __restrict__ recs,
     const int4* __restrict__ indices, const float2* __restrict__ jitter, const __grid_constant__ V views,
     const float4* __restrict__ img, const float* __restrict__ dist, const int32_t* __restrict__ ncs,
     const float4* __restrict__ gimg, const float* __restrict__ gdist, float* __restrict__ gverts,
     float* __restrict__ gcv, const Queue q) {
-    __shared__ BwdDenseSmem<NT, B> S;
-    __shared__ int4 s_item;
-    HitMasks hm = live_masks(q.hm, q.subs);
+    __shared__ BwdWarpSmem S[kBwdWarps];
+    constexpr int kParts = PX / 32 > 0 ? PX / 32 : 1;
+    __shared__ HitMasks hm;  // read once per block: kept out of the registers
+    if (threadIdx.x == 0) {
+        hm = live_masks(q.hm, q.subs);
+        if (__ldg(q.info) != 0) hm.ck = nullptr;  // tiles split off to the pair kernel: the others whole
+    }
+    __syncthreads();
     // every tile by its segments when the forward left checkpoints, else the
     // queue's tiles whole
-    const bool segs = hm.ck != nullptr && __ldg(q.info) == 0;
-    if (!segs) hm.ck = nullptr;
-    const int64_t n_items = segs ? segment_items(q.info, q.G, hm.seg_shift) * q.subs : (int64_t)queue_items(q);
+    const bool segs = hm.ck != nullptr;
+    const int64_t n_items =
+        (segs ? segment_items(q.info, q.G, hm.seg_shift) * q.subs : (int64_t)queue_items(q)) * kParts;
     for (;;) {
-        if (threadIdx.x == 0) {
+        SegItem it = {-1, 0, 0};
+        int part = 0;
+        if ((threadIdx.x & 31) == 0) {
             const int item = (int)atomicAdd(q.ticket, 1u);
-            SegItem it = {-1, 0, 0};
             if (item < n_items) {
-                if (segs) it = segment_item(q, item, hm.seg_shift);
-                else it = {queue_tile(q, item), 0, item % q.subs};
+                part = item % kParts;
+                const int strip = item / kParts;
+                if (segs) it = segment_item(q, strip, hm.seg_shift);
+                else it = {queue_tile(q, strip), 0, strip % q.subs};
             }
-            s_item = make_int4(it.tile, it.seg, it.sub, 0);
         }
-        __syncthreads();
-        const int4 it = s_item;
-        __syncthreads();
-        const int t = it.x;
+        const int t = __shfl_sync(0xffffffffu, it.tile, 0);
         if (t < 0) return;
+        const int seg = __shfl_sync(0xffffffffu, it.seg, 0), sub = __shfl_sync(0xffffffffu, it.sub, 0);
+        part = __shfl_sync(0xffffffffu, part, 0);
         const int v = views.find(t);
         const int tb = views.tile_base(v);
         const int64_t pb = views.pixel_base(v);
-        bwd_dense_item<NT, B>(t - tb, it.z, ids, ranges + tb, recs, indices, jitter + pb, views.camera(v),
-                              img + pb, dist + 5 * pb, ncs + pb, gimg + pb, gdist ? gdist + 5 * pb : nullptr,
-                              gverts, gcv, S, hm, q.subs, t, q, it.y);
+        bwd_warp_item<PX>(t - tb, sub, part, seg, ids, ranges + tb, recs, indices, jitter + pb, views.camera(v),
+                          img + pb, dist + 5 * pb, ncs + pb, gimg + pb, gdist ? gdist + 5 * pb : nullptr, gverts,
+                          gcv, S[threadIdx.x >> 5], hm, q.subs, t, q);
     }
 }
 
@@ -2681,13 +2762,13 @@ int launch_bwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, cons
                                            (const float4*)gimg, gdist, gverts, gcv, qd);
             return rm_host::check_launch("rm_blend_bwd (dense, bulk-copy staging)");
         }
-        auto dense_kernel = blend_bwd_dense_kernel<PX, B_DENSE, V>;
+        auto warp_kernel = blend_bwd_warp_kernel<PX, V>;
         // segments make more items than tiles: always the resident grid
-        const int grid = persistent_grid(dense_kernel, PX, 0, masks ? 1 << 30 : G * subs);
-        dense_kernel<<<grid, PX, 0, s>>>(ids, (const int2*)ranges, w.recs, (const int4*)indices,
-                                         (const float2*)jitter, views, (const float4*)img, dist, nc,
-                                         (const float4*)gimg, gdist, gverts, gcv, qd);
-        return rm_host::check_launch("rm_blend_bwd (dense)");
+        const int grid = persistent_grid(warp_kernel, kBwdWarps * 32, 0, masks ? 1 << 30 : G * subs);
+        warp_kernel<<<grid, kBwdWarps * 32, 0, s>>>(ids, (const int2*)ranges, w.recs, (const int4*)indices,
+                                                    (const float2*)jitter, views, (const float4*)img, dist, nc,
+                                                    (const float4*)gimg, gdist, gverts, gcv, qd);
+        return rm_host::check_launch("rm_blend_bwd (warp items)");
     };
     if (tn.heavy_shift == 0) return launch_dense();
     if (tn.heavy_shift == 1) {
