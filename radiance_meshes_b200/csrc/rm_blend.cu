@@ -1537,6 +1537,18 @@ struct BwdWarpSmem {
     float4 sums[32][6];               // per entry: (G, H) of the four faces, density rgb, grd 0
 };
 
+// a += v by two packed additions.
+__device__ __forceinline__ void add4(float4& a, float4 v) {
+    unsigned long long* p = reinterpret_cast<unsigned long long*>(&a);
+    const unsigned long long* q = reinterpret_cast<const unsigned long long*>(&v);
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(p[0]) : "l"(q[0]));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(p[1]) : "l"(q[1]));
+}
+__device__ __forceinline__ float4 shfl_xor4(float4 a, int off) {
+    return make_float4(__shfl_xor_sync(0xffffffffu, a.x, off), __shfl_xor_sync(0xffffffffu, a.y, off),
+                       __shfl_xor_sync(0xffffffffu, a.z, off), __shfl_xor_sync(0xffffffffu, a.w, off));
+}
+
 // Adds up the 24 columns of the lanes' rows: the lane's group (lane / 8) takes
 // eight rows, its place in it (< 6) four columns; the groups meet by shuffles.
 // Rows of the lanes in bal_a go to a, the others to b (SPLIT) or to a too.
@@ -1552,26 +1564,15 @@ __device__ __forceinline__ void warp_sum_rows(const float4* __restrict__ red, in
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
             const float4 v = red[(row0 + r) * (kRedStride / 4) + quad];
-            if (!SPLIT || ((in >> r) & 1u)) {
-                a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
-            } else {
-                b.x += v.x; b.y += v.y; b.z += v.z; b.w += v.w;
-            }
+            if (!SPLIT || ((in >> r) & 1u)) add4(a, v);
+            else add4(b, v);
         }
     }
     __syncwarp();
 #pragma unroll
     for (int off = 8; off <= 16; off <<= 1) {
-        a.x += __shfl_xor_sync(0xffffffffu, a.x, off);
-        a.y += __shfl_xor_sync(0xffffffffu, a.y, off);
-        a.z += __shfl_xor_sync(0xffffffffu, a.z, off);
-        a.w += __shfl_xor_sync(0xffffffffu, a.w, off);
-        if (SPLIT) {
-            b.x += __shfl_xor_sync(0xffffffffu, b.x, off);
-            b.y += __shfl_xor_sync(0xffffffffu, b.y, off);
-            b.z += __shfl_xor_sync(0xffffffffu, b.z, off);
-            b.w += __shfl_xor_sync(0xffffffffu, b.w, off);
-        }
+        add4(a, shfl_xor4(a, off));
+        if (SPLIT) add4(b, shfl_xor4(b, off));
     }
 }
 
@@ -2243,7 +2244,7 @@ __device__ __forceinline__ void bwd_pair_item(
 
 // Warps per CTA and resident CTAs per SM of the backward's warp items.
 constexpr int kBwdWarps = 4;
-constexpr int kBwdCtas = 4;
+constexpr int kBwdCtas = 5;
 
 template <int PX, class V>
 __global__ void __launch_bounds__(kBwdWarps * 32, kBwdCtas) blend_bwd_warp_kernel(
