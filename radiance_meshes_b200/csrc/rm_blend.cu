@@ -215,16 +215,16 @@ __device__ __forceinline__ float rcp_approx(float x) {
 
 __device__ __forceinline__ Weights seg_weights(float x) {
     Weights w;
-    w.alpha = exp_approx(-x);
+    w.alpha = __expf(-x);
     if (x < 0.25f) {
         // w1 = x/2 - x^2/6 + x^3/24 - x^4/120 + x^5/720 - x^6/5040 + x^7/40320
-        w.w1 = x * fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, 1.0f / 40320.0f, -1.0f / 5040.0f), 1.0f / 720.0f),
-                                            -1.0f / 120.0f), 1.0f / 24.0f), -1.0f / 6.0f), 0.5f);
+        w.w1 = x * (0.5f + x * (-1.0f / 6.0f + x * (1.0f / 24.0f + x * (-1.0f / 120.0f + x * (1.0f / 720.0f +
+                 x * (-1.0f / 5040.0f + x * (1.0f / 40320.0f)))))));
         // w0 = x/2 - x^2/3 + x^3/8 - x^4/30 + x^5/144 - x^6/840 + x^7/5760
-        w.w0 = x * fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, fmaf(x, 1.0f / 5760.0f, -1.0f / 840.0f), 1.0f / 144.0f),
-                                            -1.0f / 30.0f), 0.125f), -1.0f / 3.0f), 0.5f);
+        w.w0 = x * (0.5f + x * (-1.0f / 3.0f + x * (0.125f + x * (-1.0f / 30.0f + x * (1.0f / 144.0f +
+                 x * (-1.0f / 840.0f + x * (1.0f / 5760.0f)))))));
     } else {
-        const float phi = (1.0f - w.alpha) * rcp_approx(x);
+        const float phi = __fdividef(1.0f - w.alpha, x);
         w.w0 = phi - w.alpha;
         w.w1 = 1.0f - phi;
     }
@@ -491,7 +491,7 @@ __device__ __forceinline__ void write_checkpoint(const HitMasks& hm, const Pixel
 // alphablend_shader_interp.slang:84-183): colour += rgb * T, log T -= a, and
 // the five distortion moments with m0 = density, m1 = density * (a + b) / 2.
 __device__ __forceinline__ void fold_hit(PixelState& st, float a, float m0, float m1, float d4, const float* rgb) {
-    const float T = exp_approx(st.logT);
+    const float T = __expf(st.logT);
 #pragma unroll
     for (int k = 0; k < 3; ++k) st.c[k] = fmaf(rgb[k], T, st.c[k]);
     st.logT = st.logT - a;
@@ -534,15 +534,9 @@ __device__ __forceinline__ EntryResult eval_entry(const float4* __restrict__ q, 
     r.rgb[0] = r.rgb[1] = r.rgb[2] = 0.f;
     if (is.geo && s.a > 0.f) {
         r.a = s.a;
-        // compute_integral (interp_version.slang:30-69) with the colour linear
-        // along the ray: c(t) = base + dot(grd, o - v0) + t dot(grd, d)
-        const f3 grd = {q[4].w, q[5].w, q[6].w};
-        const float c0 = -dot3(grd, xyz(q[4]) - o), gd = dot3(grd, d);
-        const Weights w = seg_weights(s.a);
-        const float lin = fmaf(w.w0, fmaf(is.exit, gd, c0), w.w1 * fmaf(is.enter, gd, c0)), sum = w.w0 + w.w1;
-        r.rgb[0] = fmaf(sum, q[1].w, lin);
-        r.rgb[1] = fmaf(sum, q[2].w, lin);
-        r.rgb[2] = fmaf(sum, q[3].w, lin);
+        integrate(q, o, d, is.enter, is.exit, s);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) r.rgb[k] = s.rgb[k];
         r.m1 = density * (is.exit + is.enter) / 2.0f;
         r.d4 = third(density * density * s.dt);
     }
@@ -752,7 +746,7 @@ __device__ __forceinline__ void stage_pair_batch(FwdPairSmem<PX, B>& S, int buf,
 // One entry of the fold, hit or miss (a = 0, every increment zero).
 __device__ __forceinline__ void fold_any(PixelState& st, float a, float m0, float m1, float d4, float r, float g,
                                          float b) {
-    const float T = exp_approx(st.logT);
+    const float T = __expf(st.logT);
     st.c[0] = fmaf(r, T, st.c[0]);
     st.c[1] = fmaf(g, T, st.c[1]);
     st.c[2] = fmaf(b, T, st.c[2]);
@@ -1541,14 +1535,18 @@ __device__ __forceinline__ uint32_t bits_below(uint32_t w, int n) {
     return n <= 0 ? 0u : n >= 32 ? w : w & ((1u << n) - 1u);
 }
 
-// Warp backward item: half of a 64-pixel strip (8x4 pixels; a whole strip of
-// 16) over one stretch of a tile's list, walked back to front by one warp, one
+// Backward item: a 64-pixel strip (16 for 16-pixel strips) over one stretch of
+// a tile's list, walked back to front by one warp per 32 pixels (8x4), one
 // pixel per lane.  Per block of 32 entries (one mask word per pixel) the
-// records of the entries some pixel hit are copied to the warp's shared
-// memory and walked; each entry is met once, so its sums over the lanes are
-// final when formed (no accumulators to clear, no atomics in shared memory)
-// and are turned into vertex and cell-value gradients for all 32 entries at
-// once, one entry per lane, at the end of the block.
+// records of the entries some pixel hit are copied to shared memory; each warp
+// walks those that its pixels hit, meets each once, and so has its sums over
+// the lanes final when formed (no accumulators to clear, no atomics in shared
+// memory).  One of the two warps, in turn, then adds up both warps' sums and
+// turns them into vertex and cell-value gradients, one entry per lane.  (Each
+// warp adding its own half to global memory saves the barriers, but doubles
+// the float additions into the tets and vertices that fill much of the image,
+// and with them the rounding of those sums: 1.46e-6 against 0.67e-6 relative
+// to 64 bits for the cell values of a 1.3M-tet frame.)
 //
 // Per hit the lane forms 23 partials: for each face p the sums G_p of
 // dL/dt / dot(n_p, d) over the hits that enter or leave through it and H_p of
@@ -1557,13 +1555,15 @@ __device__ __forceinline__ uint32_t bits_below(uint32_t w, int n) {
 // once per entry (flush_sums): with t_p = dot(n_p, v_ref - o) / dot(n_p, d),
 // dt/dn = -(hit point - v_ref) / dot(n, d) and dt/dv_ref = n / dot(n, d).
 //
-// Bound: instruction issue, about 300 instructions for an entry and up to 32
-// pixels (540 before: 25 partials formed with separate multiplies and adds,
-// normals and reference points selected per lane, CTA barriers per batch).
-struct BwdWarpSmem {
+// Bound: instruction issue, about 440 instructions for an entry and up to 32
+// pixels, and the shared-memory traffic of the row sums.
+template <int NW>
+struct BwdSmem {
     float4 srec[32][kRecFloat4 + 1];
-    float4 red[32 * kRedStride / 4];  // one row of partials per lane
-    float4 sums[32][6];               // per entry: (G, H) of the four faces, density rgb, grd 0
+    float4 red[NW][32 * kRedStride / 4];  // one row of partials per lane
+    float4 sums[NW][32][6];  // per entry: (G, H) of the four faces, density rgb, grd 0
+    uint32_t any[2][NW];     // entries that the warp's pixels hit, of this block and the next
+    int4 item;
 };
 
 // a += v by two packed additions.
@@ -1607,7 +1607,7 @@ __device__ __forceinline__ void warp_sum_rows(const float4* __restrict__ red, in
 
 // One entry's sums -> gradients of its four vertices and seven cell values,
 // added to global memory by one thread.
-__device__ __forceinline__ void flush_sums(const float4* __restrict__ q, const float4* __restrict__ s, int32_t g,
+__device__ __forceinline__ void flush_sums(const float4* __restrict__ q, const float4* s, int32_t g,
                                            const int4* __restrict__ indices, float* __restrict__ gverts,
                                            float* __restrict__ gcv) {
     const f3 P[4] = {xyz(q[4]), xyz(q[5]), xyz(q[6]), xyz(q[7])};
@@ -1655,13 +1655,14 @@ __device__ __forceinline__ void flush_sums(const float4* __restrict__ q, const f
 }
 
 template <int PX>
-__device__ __forceinline__ void bwd_warp_item(
-    int tile, int sub, int half, int seg, const int32_t* __restrict__ ids, const int2* __restrict__ ranges,
+__device__ __forceinline__ void bwd_item(
+    int tile, int sub, int seg, const int32_t* __restrict__ ids, const int2* __restrict__ ranges,
     const float4* __restrict__ recs, const int4* __restrict__ indices, const float2* __restrict__ jitter,
     const rm_camera& cam, const float4* __restrict__ img, const float* __restrict__ dist,
     const int32_t* __restrict__ ncs, const float4* __restrict__ gimg, const float* __restrict__ gdist,
-    float* __restrict__ gverts, float* __restrict__ gcv, BwdWarpSmem& S, const HitMasks& hm, int subs, int gtile,
-    const Queue& lq) {
+    float* __restrict__ gverts, float* __restrict__ gcv, BwdSmem<PX / 32 + (PX < 32)>& S, const HitMasks& hm, int subs,
+    int gtile, const Queue& lq) {
+    constexpr int kWarps = PX / 32 + (PX < 32);
     constexpr unsigned kAll = 0xffffffffu;
     const int2 rg = __ldg(ranges + tile);
     const int len = rg.y - rg.x;
@@ -1679,8 +1680,7 @@ __device__ __forceinline__ void bwd_warp_item(
         return;
     }
     if (s0 >= s1) return;
-    const int lane = threadIdx.x & 31;
-    const int p = half * 32 + lane;
+    const int p = threadIdx.x, lane = p & 31, warp = p >> 5;
     const int tx = tile % cam.grid_width, ty = tile / cam.grid_width;
     int lx, ly;
     strip_pixel<PX>(cam, sub, p, lx, ly);
@@ -1689,7 +1689,17 @@ __device__ __forceinline__ void bwd_warp_item(
     const int64_t pix = (int64_t)py * cam.image_width + px;
     int32_t nc = inside ? __ldg(ncs + pix) : 0;
     if (nc <= s0) nc = 0;
-    if (!__any_sync(kAll, nc > 0)) return;  // every pixel's walk ends before this stretch
+    // the last block that some pixel's walk reaches (none: they all end before
+    // this stretch)
+    int last = min((int)__reduce_max_sync(kAll, (unsigned)nc), s1);
+    if (kWarps > 1) {
+        if (lane == 0) S.any[0][warp] = (uint32_t)last;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) last = max(last, (int)S.any[0][i]);
+        __syncthreads();
+    }
+    if (last == 0) return;
     f3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f};
     float logT = 0.f, D2 = 0.f, D3 = 0.f;  // state along the reverse walk
     float dS_c[3] = {0.f, 0.f, 0.f}, dS_logT = 0.f, dS_D[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
@@ -1713,8 +1723,7 @@ __device__ __forceinline__ void bwd_warp_item(
     const float dS0 = 2.0f * dS_D[0], dS1 = 2.0f * dS_D[1], dS4 = dS_D[4] * (1.0f / 3.0f);
     const float dS_sum = dS_c[0] + dS_c[1] + dS_c[2];
     float dS2 = dS_D[2], dS3 = dS_D[3];
-    float* const row = reinterpret_cast<float*>(S.red) + lane * kRedStride;
-    float4* const row4 = reinterpret_cast<float4*>(row);
+    float4* const row4 = S.red[warp] + lane * (kRedStride / 4);
 
     // A pixel's hit bits of block k: the forward's word, all entries without
     // one; none at or past n_contributors.
@@ -1726,19 +1735,30 @@ __device__ __forceinline__ void bwd_warp_item(
         }
         return bits_below(w, nc - 32 * k);
     };
-    const int last = (int)__reduce_max_sync(kAll, (unsigned)nc);
     int k = (last - 1) >> 5;
-    uint32_t w = hit_word(k);
+    uint32_t w = hit_word(k), mine = __reduce_or_sync(kAll, w);
+    if (lane == 0) S.any[k & 1][warp] = mine;
+    __syncthreads();
     for (; k >= s0 >> 5; --k) {
-        const uint32_t cur = w;
-        if (k > s0 >> 5) w = hit_word(k - 1);  // the next block's, ahead of its use
-        const uint32_t any = __reduce_or_sync(kAll, cur);
-        if (!any) continue;
+        const uint32_t cur = w, own = mine;
+        uint32_t any = 0u;
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) any |= S.any[k & 1][i];
+        const uint32_t any_other = S.any[k & 1][kWarps - 1 - warp];  // the other warp's (its own for one)
+        if (k > s0 >> 5) {  // the next block's, ahead of its use
+            w = hit_word(k - 1);
+            mine = __reduce_or_sync(kAll, w);
+            if (lane == 0) S.any[(k - 1) & 1][warp] = mine;
+        }
+        if (!any) {
+            __syncthreads();  // S.any of the next block
+            continue;
+        }
         int32_t g = -1;
         if ((any >> lane) & 1u) g = list_id(ids, rg.x + 32 * k + lane, lq);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int e = 4 * i + (lane >> 3);
+        for (int i = 0; i < 8 / kWarps; ++i) {
+            const int e = 4 * (warp + kWarps * i) + (lane >> 3);
             const int32_t ge = __shfl_sync(kAll, g, e);
             if (ge >= 0)
                 async_copy16(&S.srec[e][lane & 7], recs + (int64_t)kRecFloat4 * ge + (lane & 7));
@@ -1746,8 +1766,8 @@ __device__ __forceinline__ void bwd_warp_item(
                 S.srec[e][lane & 7] = make_float4(0.f, 0.f, 0.f, 0.f);  // names no tet: nothing hits it
         }
         async_wait();
-        __syncwarp();
-        uint32_t left = any, done = 0u;  // entries to walk; entries with sums
+        __syncthreads();
+        uint32_t left = own;  // entries to walk
         while (left) {
             const int ja = 31 - __clz(left);
             left &= ~(1u << ja);
@@ -1838,18 +1858,29 @@ __device__ __forceinline__ void bwd_warp_item(
             row4[5] = g_grd;
             float4 sa, sb;
             if (jb < 0) {
-                warp_sum_rows<false>(S.red, lane, bal_a, sa, sb);
+                warp_sum_rows<false>(S.red[warp], lane, bal_a, sa, sb);
             } else {
-                warp_sum_rows<true>(S.red, lane, bal_a, sa, sb);
-                if (lane < 6) S.sums[jb][lane] = sb;
-                done |= 1u << jb;
+                warp_sum_rows<true>(S.red[warp], lane, bal_a, sa, sb);
+                if (lane < 6) S.sums[warp][jb][lane] = sb;
             }
-            if (lane < 6) S.sums[ja][lane] = sa;
-            done |= 1u << ja;
+            if (lane < 6) S.sums[warp][ja][lane] = sa;
         }
-        __syncwarp();
-        if (((done >> lane) & 1u) && g >= 0) flush_sums(S.srec[lane], S.sums[lane], g, indices, gverts, gcv);
-        __syncwarp();  // the next block overwrites the records
+        __syncthreads();
+        if (warp == k % kWarps && g >= 0) {
+            float4 sum[6];
+#pragma unroll
+            for (int c = 0; c < 6; ++c) sum[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < kWarps; ++i) {
+                const uint32_t had = i == warp ? own : any_other;
+                if ((had >> lane) & 1u) {
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) add4(sum[c], S.sums[i][lane][c]);
+                }
+            }
+            flush_sums(S.srec[lane], sum, g, indices, gverts, gcv);
+        }
+        __syncthreads();  // the next block overwrites the records and the sums
     }
 }
 
@@ -2271,19 +2302,17 @@ __device__ __forceinline__ void bwd_pair_item(
     }
 }
 
-// Warps per CTA and resident CTAs per SM of the backward's warp items.
-constexpr int kBwdWarps = 4;
-constexpr int kBwdCtas = 5;
+// Resident warps per SM of the backward.
+constexpr int kBwdWarpsPerSm = 20;
 
 template <int PX, class V>
-__global__ void __launch_bounds__(kBwdWarps * 32, kBwdCtas) blend_bwd_warp_kernel(
+__global__ void __launch_bounds__(PX < 32 ? 32 : PX, PX < 32 ? kBwdWarpsPerSm : kBwdWarpsPerSm * 32 / PX) blend_bwd_kernel(
     const int32_t* __restrict__ ids, const int2* __restrict__ ranges, const float4* __restrict__ recs,
     const int4* __restrict__ indices, const float2* __restrict__ jitter, const __grid_constant__ V views,
     const float4* __restrict__ img, const float* __restrict__ dist, const int32_t* __restrict__ ncs,
     const float4* __restrict__ gimg, const float* __restrict__ gdist, float* __restrict__ gverts,
     float* __restrict__ gcv, const Queue q) {
-    __shared__ BwdWarpSmem S[kBwdWarps];
-    constexpr int kParts = PX / 32 > 0 ? PX / 32 : 1;
+    __shared__ BwdSmem<PX / 32 + (PX < 32)> S;
     __shared__ HitMasks hm;  // read once per block: kept out of the registers
     if (threadIdx.x == 0) {
         hm = live_masks(q.hm, q.subs);
@@ -2293,30 +2322,27 @@ __global__ void __launch_bounds__(kBwdWarps * 32, kBwdCtas) blend_bwd_warp_kerne
     // every tile by its segments when the forward left checkpoints, else the
     // queue's tiles whole
     const bool segs = hm.ck != nullptr;
-    const int64_t n_items =
-        (segs ? segment_items(q.info, q.G, hm.seg_shift) * q.subs : (int64_t)queue_items(q)) * kParts;
+    const int64_t n_items = segs ? segment_items(q.info, q.G, hm.seg_shift) * q.subs : (int64_t)queue_items(q);
     for (;;) {
-        SegItem it = {-1, 0, 0};
-        int part = 0;
-        if ((threadIdx.x & 31) == 0) {
+        if (threadIdx.x == 0) {
             const int item = (int)atomicAdd(q.ticket, 1u);
+            SegItem it = {-1, 0, 0};
             if (item < n_items) {
-                part = item % kParts;
-                const int strip = item / kParts;
-                if (segs) it = segment_item(q, strip, hm.seg_shift);
-                else it = {queue_tile(q, strip), 0, strip % q.subs};
+                if (segs) it = segment_item(q, item, hm.seg_shift);
+                else it = {queue_tile(q, item), 0, item % q.subs};
             }
+            S.item = make_int4(it.tile, it.seg, it.sub, 0);
         }
-        const int t = __shfl_sync(0xffffffffu, it.tile, 0);
-        if (t < 0) return;
-        const int seg = __shfl_sync(0xffffffffu, it.seg, 0), sub = __shfl_sync(0xffffffffu, it.sub, 0);
-        part = __shfl_sync(0xffffffffu, part, 0);
-        const int v = views.find(t);
+        __syncthreads();
+        const int4 it = S.item;
+        __syncthreads();
+        if (it.x < 0) return;
+        const int v = views.find(it.x);
         const int tb = views.tile_base(v);
         const int64_t pb = views.pixel_base(v);
-        bwd_warp_item<PX>(t - tb, sub, part, seg, ids, ranges + tb, recs, indices, jitter + pb, views.camera(v),
-                          img + pb, dist + 5 * pb, ncs + pb, gimg + pb, gdist ? gdist + 5 * pb : nullptr, gverts,
-                          gcv, S[threadIdx.x >> 5], hm, q.subs, t, q);
+        bwd_item<PX>(it.x - tb, it.z, it.y, ids, ranges + tb, recs, indices, jitter + pb, views.camera(v), img + pb,
+                     dist + 5 * pb, ncs + pb, gimg + pb, gdist ? gdist + 5 * pb : nullptr, gverts, gcv, S, hm, q.subs,
+                     it.x, q);
     }
 }
 
@@ -2792,13 +2818,14 @@ int launch_bwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, cons
                                            (const float4*)gimg, gdist, gverts, gcv, qd);
             return rm_host::check_launch("rm_blend_bwd (dense, bulk-copy staging)");
         }
-        auto warp_kernel = blend_bwd_warp_kernel<PX, V>;
+        auto kernel = blend_bwd_kernel<PX, V>;
+        constexpr int threads = PX < 32 ? 32 : PX;
         // segments make more items than tiles: always the resident grid
-        const int grid = persistent_grid(warp_kernel, kBwdWarps * 32, 0, masks ? 1 << 30 : G * subs);
-        warp_kernel<<<grid, kBwdWarps * 32, 0, s>>>(ids, (const int2*)ranges, w.recs, (const int4*)indices,
-                                                    (const float2*)jitter, views, (const float4*)img, dist, nc,
-                                                    (const float4*)gimg, gdist, gverts, gcv, qd);
-        return rm_host::check_launch("rm_blend_bwd (warp items)");
+        const int grid = persistent_grid(kernel, threads, 0, masks ? 1 << 30 : G * subs);
+        kernel<<<grid, threads, 0, s>>>(ids, (const int2*)ranges, w.recs, (const int4*)indices, (const float2*)jitter,
+                                        views, (const float4*)img, dist, nc, (const float4*)gimg, gdist, gverts, gcv,
+                                        qd);
+        return rm_host::check_launch("rm_blend_bwd");
     };
     if (tn.heavy_shift == 0) return launch_dense();
     if (tn.heavy_shift == 1) {
