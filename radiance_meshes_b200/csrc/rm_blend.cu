@@ -199,9 +199,31 @@ struct Weights {
     float alpha, w0, w1;
 };
 
+// Two floats in one register pair: packed operations round each half as the
+// scalar ones do and take one issue slot for both.
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pair(float lo, float hi) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpair(Pair p, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair add2(Pair a, Pair b) {
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // exp(x) for x <= 0 and 1 / x by the approximate instructions alone: __expf and
 // __fdividef add range handling (six instructions each time) for results
-// below 2^-126 and divisors above 2^126.
+// below 2^-126 and divisors above 2^126, and are equal to these elsewhere.
 __device__ __forceinline__ float exp_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.44269504f));
@@ -215,16 +237,22 @@ __device__ __forceinline__ float rcp_approx(float x) {
 
 __device__ __forceinline__ Weights seg_weights(float x) {
     Weights w;
-    w.alpha = __expf(-x);
+    w.alpha = exp_approx(-x);
     if (x < 0.25f) {
         // w1 = x/2 - x^2/6 + x^3/24 - x^4/120 + x^5/720 - x^6/5040 + x^7/40320
-        w.w1 = x * (0.5f + x * (-1.0f / 6.0f + x * (1.0f / 24.0f + x * (-1.0f / 120.0f + x * (1.0f / 720.0f +
-                 x * (-1.0f / 5040.0f + x * (1.0f / 40320.0f)))))));
         // w0 = x/2 - x^2/3 + x^3/8 - x^4/30 + x^5/144 - x^6/840 + x^7/5760
-        w.w0 = x * (0.5f + x * (-1.0f / 3.0f + x * (0.125f + x * (-1.0f / 30.0f + x * (1.0f / 144.0f +
-                 x * (-1.0f / 840.0f + x * (1.0f / 5760.0f)))))));
+        // both at once, a product and a sum rounded separately at each step
+        const Pair xx = pair(x, x);
+        Pair p = pair(1.0f / 40320.0f, 1.0f / 5760.0f);
+        p = add2(mul2(p, xx), pair(-1.0f / 5040.0f, -1.0f / 840.0f));
+        p = add2(mul2(p, xx), pair(1.0f / 720.0f, 1.0f / 144.0f));
+        p = add2(mul2(p, xx), pair(-1.0f / 120.0f, -1.0f / 30.0f));
+        p = add2(mul2(p, xx), pair(1.0f / 24.0f, 0.125f));
+        p = add2(mul2(p, xx), pair(-1.0f / 6.0f, -1.0f / 3.0f));
+        p = add2(mul2(p, xx), pair(0.5f, 0.5f));
+        unpair(mul2(p, xx), w.w1, w.w0);
     } else {
-        const float phi = __fdividef(1.0f - w.alpha, x);
+        const float phi = (1.0f - w.alpha) * rcp_approx(x);
         w.w0 = phi - w.alpha;
         w.w1 = 1.0f - phi;
     }
@@ -491,7 +519,7 @@ __device__ __forceinline__ void write_checkpoint(const HitMasks& hm, const Pixel
 // alphablend_shader_interp.slang:84-183): colour += rgb * T, log T -= a, and
 // the five distortion moments with m0 = density, m1 = density * (a + b) / 2.
 __device__ __forceinline__ void fold_hit(PixelState& st, float a, float m0, float m1, float d4, const float* rgb) {
-    const float T = __expf(st.logT);
+    const float T = exp_approx(st.logT);
 #pragma unroll
     for (int k = 0; k < 3; ++k) st.c[k] = fmaf(rgb[k], T, st.c[k]);
     st.logT = st.logT - a;
@@ -746,7 +774,7 @@ __device__ __forceinline__ void stage_pair_batch(FwdPairSmem<PX, B>& S, int buf,
 // One entry of the fold, hit or miss (a = 0, every increment zero).
 __device__ __forceinline__ void fold_any(PixelState& st, float a, float m0, float m1, float d4, float r, float g,
                                          float b) {
-    const float T = __expf(st.logT);
+    const float T = exp_approx(st.logT);
     st.c[0] = fmaf(r, T, st.c[0]);
     st.c[1] = fmaf(g, T, st.c[1]);
     st.c[2] = fmaf(b, T, st.c[2]);
