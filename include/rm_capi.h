@@ -584,7 +584,10 @@ RM_API int rm_blend_bwd_multi(const int32_t* sorted_ids, const int32_t* ranges,
  * and the maximum of int(65535 * T).  Columns 3 and 4 are left untouched, as
  * in the reference, whose walk also starts from log T = 1 and stops once
  * log T < -5.5.  Workspace and flags as rm_blend_fwd (records are packed
- * unless RM_BLEND_REUSE_RECORDS).
+ * unless RM_BLEND_REUSE_RECORDS).  A workspace with rm_blend_hit_mask_bytes and
+ * 4 bytes per pixel (and 512) beyond rm_blend_workspace_size lets long lists be
+ * taken in stretches (64-pixel strips): the same counts and maxima, several
+ * times faster where a few lists are long.
  */
 RM_API int rm_calc_tet_err(const int32_t* sorted_ids, const int32_t* ranges,
                            const int32_t* indices, const float* vertices,

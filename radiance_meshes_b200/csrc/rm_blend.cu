@@ -549,6 +549,8 @@ __device__ __forceinline__ float third(float x) {
     return x <= 3.402823466e38f ? y : x;
 }
 
+// LOGT: a only (the statistics' walk).
+template <bool LOGT>
 __device__ __forceinline__ EntryResult eval_entry(const float4* __restrict__ q, f3 o, f3 d) {
     EntryResult r;
     const Isect is = intersect<false>(q, o, d);
@@ -560,7 +562,9 @@ __device__ __forceinline__ EntryResult eval_entry(const float4* __restrict__ q, 
     r.m1 = 0.f;
     r.d4 = 0.f;
     r.rgb[0] = r.rgb[1] = r.rgb[2] = 0.f;
-    if (is.geo && s.a > 0.f) {
+    if (LOGT) {
+        if (is.geo && s.a > 0.f) r.a = s.a;
+    } else if (is.geo && s.a > 0.f) {
         r.a = s.a;
         integrate(q, o, d, is.enter, is.exit, s);
 #pragma unroll
@@ -689,9 +693,10 @@ struct FwdPairSmem {
     int32_t warp_base[(PX + 31) / 32];
 };
 
-template <int PX, int B>
+template <bool LOGT, int PX, int B>
 __device__ __forceinline__ void store_result(FwdPairSmem<PX, B>& S, int j, int sl, const EntryResult& r) {
     S.res[0][j][sl] = r.a;
+    if (LOGT) return;
     S.res[1][j][sl] = r.m1;
     S.res[2][j][sl] = r.d4;
     S.res[3][j][sl] = r.rgb[0];
@@ -787,7 +792,7 @@ __device__ __forceinline__ void fold_any(PixelState& st, float a, float m0, floa
     st.D[4] = st.D[4] + d4;
 }
 
-template <int PX, int NT, int B>
+template <int PX, int NT, int B, bool LOGT>
 __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, const int32_t* __restrict__ ids,
                                          const int2* __restrict__ ranges, const float4* __restrict__ recs,
                                          const float2* __restrict__ jitter, const rm_camera& cam,
@@ -811,7 +816,7 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
     const int px = tx * cam.tile_width + lx, py = ty * cam.tile_height + ly;
     const bool inside = owner && px < cam.image_width && py < cam.image_height;
     const int64_t pix = (int64_t)py * cam.image_width + px;
-    PixelState st = {{0.f, 0.f, 0.f}, 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}};
+    PixelState st = {{0.f, 0.f, 0.f}, LOGT ? 1.0f : 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}};
     int32_t nc = rg.y - rg.x;  // entries walked: all of them unless log T runs out
     bool active = inside && nc > 0;
     int rank = 0, slot = tid;  // rank among the warp's active pixels; where the pixel's ray and results lie
@@ -844,7 +849,7 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
         float z = 3e38f;
         rank = rank_active();
         if (active) {
-            const float2 j = __ldg(jitter + pix);
+            const float2 j = LOGT ? make_float2(0.5f, 0.5f) : __ldg(jitter + pix);
             make_ray(cam, px, py, j.x, j.y, o, d);
             z = dot3(mk3(M[8], M[9], M[10]), d);
             S.uv[0][tid] = dot3(mk3(M[0], M[1], M[2]), d) / z;
@@ -914,7 +919,7 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
                 const f3 o = {S.ray[0][sl], S.ray[1][sl], S.ray[2][sl]};
                 const f3 d = {S.ray[3][sl], S.ray[4][sl], S.ray[5][sl]};
                 for (int j = member * groups + lane / span; j < n; j += team * groups)
-                    store_result(S, j, sl, eval_entry(S.srec[j], o, d));
+                    store_result<LOGT>(S, j, sl, eval_entry<LOGT>(S.srec[j], o, d));
             }
             __syncthreads();
         }
@@ -931,7 +936,17 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
                 const int j1 = S.start[cur][w + 1];
                 uint32_t hb = 0;  // bit k: entry k of the block was a hit for this owner's pixel
                 if (kMasks && active) write_checkpoint(hm, st, rg.x, rg.x + (blk + w) * RB, sub, subs, p);
-                for (int j = S.start[cur][w]; j < j1 && active; j += 4) {
+                for (int j = S.start[cur][w]; LOGT && j < j1 && active; ++j) {
+                    const float a = S.res[0][j][slot];
+                    st.logT = st.logT - a;
+                    const int at = S.pos[cur][j];
+                    hb |= a > 0.f ? 1u << at : 0u;
+                    if (st.logT < kTermLogT) {
+                        active = false;
+                        nc = (blk + w) * RB + at + 1;
+                    }
+                }
+                for (int j = S.start[cur][w]; !LOGT && j < j1 && active; j += 4) {
                     // four entries' results read ahead, whatever they are (rows past
                     // the block's last are there to read and not used)
                     float r[6][4], dens[4];
@@ -986,11 +1001,12 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
         n_active = __syncthreads_count(active);
     }
     if (inside) {
+        out_nc[pix] = nc;
+        if (LOGT) return;
         out_img[pix] = make_float4(st.c[0], st.c[1], st.c[2], st.logT);
         float* dd = out_dist + 5 * pix;
 #pragma unroll
         for (int k = 0; k < 5; ++k) dd[k] = st.D[k];
-        out_nc[pix] = nc;
     }
 }
 
@@ -1007,7 +1023,7 @@ struct FwdWarpSmem {
     float4 srec[32][kRecFloat4 + 1];  // padded: 32 lanes read one record each without conflicts
 };
 
-template <int PX>
+template <int PX, bool LOGT>
 __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const int32_t* __restrict__ ids,
                                               const int2* __restrict__ ranges, const float4* __restrict__ recs,
                                               const float2* __restrict__ jitter, const rm_camera& cam,
@@ -1027,7 +1043,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
     f3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f};
     float u = 0.f, v = 0.f, z = 3e38f;
     if (inside) {
-        const float2 j = __ldg(jitter + pix);
+        const float2 j = LOGT ? make_float2(0.5f, 0.5f) : __ldg(jitter + pix);
         make_ray(cam, px, py, j.x, j.y, o, d);
         z = dot3(mk3(M[8], M[9], M[10]), d);
         u = dot3(mk3(M[0], M[1], M[2]), d) / z;
@@ -1046,7 +1062,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
                   fminf(bd.v0, __shfl_xor_sync(0xffffffffu, bd.v0, off)),
                   fmaxf(bd.v1, __shfl_xor_sync(0xffffffffu, bd.v1, off))};
     };
-    PixelState st = {{0.f, 0.f, 0.f}, 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}};
+    PixelState st = {{0.f, 0.f, 0.f}, LOGT ? 1.0f : 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}};
     int32_t nc = rg.y - rg.x;  // entries walked: all of them unless log T runs out
     bool active = inside && nc > 0;
     bounds(active);
@@ -1071,10 +1087,11 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
         if (active) {
             for (uint32_t left = bal; left; left &= left - 1u) {
                 const int j = __ffs(left) - 1;
-                const EntryResult e = eval_entry(S.srec[j], o, d);
+                const EntryResult e = eval_entry<LOGT>(S.srec[j], o, d);
                 if (e.a > 0.f) {
                     hb |= 1u << j;
-                    fold_hit(st, e.a, S.srec[j][0].w, e.m1, e.d4, e.rgb);
+                    if (LOGT) st.logT = st.logT - e.a;
+                    else fold_hit(st, e.a, S.srec[j][0].w, e.m1, e.d4, e.rgb);
                     if (st.logT < kTermLogT) {
                         nc = base - rg.x + j + 1;
                         ended = true;
@@ -1094,11 +1111,12 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
         __syncwarp();  // the walk's reads of the records are done
     }
     if (inside) {
+        out_nc[pix] = nc;
+        if (LOGT) return;
         out_img[pix] = make_float4(st.c[0], st.c[1], st.c[2], st.logT);
         float* dd = out_dist + 5 * pix;
 #pragma unroll
         for (int k = 0; k < 5; ++k) dd[k] = st.D[k];
-        out_nc[pix] = nc;
     }
 }
 
@@ -1106,7 +1124,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
 // more than the warps gain, with the little L1 that the shared memory leaves
 // (1.3M tets, 1297x840: 1461 -> 1293 and 1357 -> 1024 us; a batch of four
 // served views 4187 -> 3500 us).
-template <int PX, int NT, int B, class V>
+template <int PX, int NT, int B, class V, bool LOGT>
 __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
     const int32_t* __restrict__ ids, const int2* __restrict__ ranges, const float4* __restrict__ recs,
     const float2* __restrict__ jitter, const __grid_constant__ V views, float4* __restrict__ out_img,
@@ -1135,7 +1153,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
         const int t = __ldg(q.order + at + item / q.subs), v = views.find(t);
         const int tb = views.tile_base(v);
         const int64_t pb = views.pixel_base(v);
-        fwd_pair_item<PX, NT, B>(t - tb, item % q.subs, quarter, ids, ranges + tb, recs, jitter + pb, views.camera(v),
+        fwd_pair_item<PX, NT, B, LOGT>(t - tb, item % q.subs, quarter, ids, ranges + tb, recs, jitter + pb, views.camera(v),
                                  out_img + pb, out_dist + 5 * pb, out_nc + pb, S, hm, q.subs, t, q);
     }
     constexpr int kParts = PX / 32 > 0 ? PX / 32 : 1;
@@ -1151,7 +1169,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
         const int t = __ldg(q.order + heavy + strip / q.subs), v = views.find(t);
         const int tb = views.tile_base(v);
         const int64_t pb = views.pixel_base(v);
-        fwd_warp_item<PX>(t - tb, strip % q.subs, part, ids, ranges + tb, recs, jitter + pb, views.camera(v),
+        fwd_warp_item<PX, LOGT>(t - tb, strip % q.subs, part, ids, ranges + tb, recs, jitter + pb, views.camera(v),
                           out_img + pb, out_dist + 5 * pb, out_nc + pb, W, hm, q.subs, t, q);
     }
 }
@@ -1205,6 +1223,7 @@ __global__ void __launch_bounds__(1024) order_kernel(const int2* __restrict__ ra
         // segments per bucket of the masks' segment length (segment_item)
         int shift = kNoSegments;
         if (seg_header && __ldcg(seg_header) == kMaskValid) shift = (int)__ldcg(seg_header + 1);
+        if (mask_header && mh.state == kMaskValid) shift = (int)mh.seg_shift;
         if (shift >= kMinSegShift && shift < kNoSegments) {
             uint32_t at = 0;
             for (int b = 32; b > shift; --b) {
@@ -2568,6 +2587,198 @@ __global__ void __launch_bounds__(NT, (NT >= 64 ? 1024 / NT : 32)) err_kernel(
     }
 }
 
+// The statistics from a forward walk's leavings.  The walk itself (which
+// pixel hits which entry, until its log T runs out) is the forward kernel with
+// log T started at 1 and nothing but a formed (LOGT); it leaves the hit masks,
+// n_contributors and log T at every checkpoint.  Each stretch of a list is
+// then an item of its own, as in the backward: one warp per 32 pixels goes
+// through the entries that its pixels hit, front to back, and the sums of both
+// warps of a strip are added to global memory once per entry.  (One kernel
+// walking whole lists, as err_kernel does, is bound by its longest list: 4.3
+// ms for 653k tets at 1297x840, now 1.66 ms in both kernels.)
+constexpr int kErrStride = 20;  // floats per row of 13 values: conflict-free 16-byte stores
+
+struct ErrSegSmem {
+    float4 srec[32][kRecFloat4 + 1];
+    float4 red[2][32 * kErrStride / 4];
+    float4 sums[2][32][4];
+    int32_t most[2][32];
+    uint8_t count[2][32];
+    uint32_t any[2][2];
+    int4 item;
+};
+
+__device__ __forceinline__ void err_seg_item(int tile, int sub, int seg, const int32_t* __restrict__ ids,
+                                             const int2* __restrict__ ranges, const float4* __restrict__ recs,
+                                             const rm_camera& cam, const int32_t* __restrict__ ncs,
+                                             const float* __restrict__ pixel_err, const float* __restrict__ ssim_err,
+                                             float* __restrict__ tet_err, int32_t* __restrict__ tet_count,
+                                             ErrSegSmem& S, const HitMasks& hm, int subs, const Queue& lq) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int2 rg = __ldg(ranges + tile);
+    const int len = rg.y - rg.x;
+    int s0 = 0, s1 = len;
+    if (len > (1 << hm.seg_shift)) {
+        const int shift = hm.seg_shift;
+        if (ck_id(rg.x, (len - 1) >> shift, shift) < hm.ck_cap) {
+            s0 = seg << shift;
+            s1 = min(len, s0 + (1 << shift));
+        } else if (seg) {
+            return;
+        }
+    } else if (seg) {
+        return;
+    }
+    if (s0 >= s1) return;
+    const int p = threadIdx.x, lane = p & 31, warp = p >> 5;
+    const int tx = tile % cam.grid_width, ty = tile / cam.grid_width;
+    int lx, ly;
+    strip_pixel<64>(cam, sub, p, lx, ly);
+    const int px = tx * cam.tile_width + lx, py = ty * cam.tile_height + ly;
+    const bool inside = px < cam.image_width && py < cam.image_height;
+    const int64_t pix = (int64_t)py * cam.image_width + px;
+    int32_t nc = inside ? min(__ldcg(ncs + pix), s1) : 0;
+    if (nc <= s0) nc = 0;
+    const int mine_last = (int)__reduce_max_sync(kAll, (unsigned)nc);
+    if (lane == 0) S.any[0][warp] = (uint32_t)mine_last;
+    __syncthreads();
+    const int last = max((int)S.any[0][0], (int)S.any[0][1]);
+    __syncthreads();
+    if (last == 0) return;
+    f3 o = {0.f, 0.f, 0.f}, d = {0.f, 0.f, 1.f};
+    float err = 0.f, serr = 0.f, logT = 1.0f;
+    if (nc > 0) {
+        make_ray(cam, px, py, 0.5f, 0.5f, o, d);  // pixel centre
+        err = __ldg(pixel_err + pix);
+        serr = __ldg(ssim_err + pix);
+        if (s0 > 0) logT = __ldcg(ck_at(hm, ck_id(rg.x, seg, hm.seg_shift), sub, subs, p));
+    }
+    float4* const row4 = S.red[warp] + lane * (kErrStride / 4);
+    auto hit_word = [&](int k) {
+        const int64_t i = mask_word(tile, rg.x, k, sub, subs, p);
+        return bits_below(i < hm.cap ? __ldcg(hm.words + i) : 0xffffffffu, nc - 32 * k);
+    };
+    int k = s0 >> 5;
+    uint32_t w = hit_word(k), mine = __reduce_or_sync(kAll, w);
+    if (lane == 0) S.any[k & 1][warp] = mine;
+    __syncthreads();
+    for (; 32 * k < last; ++k) {
+        const uint32_t cur = w, own = mine;
+        const uint32_t other = S.any[k & 1][1 - warp], any = own | other;
+        w = 32 * (k + 1) < last ? hit_word(k + 1) : 0u;
+        mine = __reduce_or_sync(kAll, w);
+        if (lane == 0) S.any[(k + 1) & 1][warp] = mine;
+        if (!any) {
+            __syncthreads();  // S.any of the next block
+            continue;
+        }
+        int32_t g = -1;
+        if ((any >> lane) & 1u) g = list_id(ids, rg.x + 32 * k + lane, lq);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int e = 4 * (warp + 2 * i) + (lane >> 3);
+            const int32_t ge = __shfl_sync(kAll, g, e);
+            if (ge >= 0)
+                async_copy16(&S.srec[e][lane & 7], recs + (int64_t)kRecFloat4 * ge + (lane & 7));
+            else if ((any >> e) & 1u)
+                S.srec[e][lane & 7] = make_float4(0.f, 0.f, 0.f, 0.f);  // names no tet: nothing hits it
+        }
+        async_wait();
+        __syncthreads();
+        for (uint32_t left = own; left; left &= left - 1u) {
+            const int j = __ffs(left) - 1;
+            const float4* q = S.srec[j];
+            const Isect is = intersect<false>(q, o, d);
+            const float a = q[0].w * fmaxf(is.exit - is.enter, 0.f);
+            const bool hit = ((cur >> j) & 1u) && is.geo && a > 0.f;
+            const float T = hit ? expf(logT) * a : 0.f;
+            logT = hit ? logT - a : logT;
+            // a lane without a hit adds zeros (its distances may be infinite)
+            const float enter = hit ? is.enter : 0.f, exit = hit ? is.exit : 0.f, mid = 0.5f * (enter + exit);
+            const float Te = T * err;
+            row4[0] = make_float4(T, Te, Te * err, T * serr);
+            row4[1] = make_float4(T * fmaf(enter, d.x, o.x), T * fmaf(enter, d.y, o.y), T * fmaf(enter, d.z, o.z),
+                                  T * fmaf(exit, d.x, o.x));
+            row4[2] = make_float4(T * fmaf(exit, d.y, o.y), T * fmaf(exit, d.z, o.z), T * fmaf(mid, d.x, o.x),
+                                  T * fmaf(mid, d.y, o.y));
+            row4[3] = make_float4(T * fmaf(mid, d.z, o.z), 0.f, 0.f, 0.f);
+            const unsigned bal = __ballot_sync(kAll, hit);
+            const int most = __reduce_max_sync(kAll, __float2int_rz(65535.0f * T));
+            __syncwarp();
+            // four columns of four rows per lane, then over the eight groups
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            const int quad = lane & 3, row0 = lane & 28;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) add4(s, S.red[warp][(row0 + r) * (kErrStride / 4) + quad]);
+            __syncwarp();
+#pragma unroll
+            for (int off = 4; off <= 16; off <<= 1) add4(s, shfl_xor4(s, off));
+            if (lane < 4) S.sums[warp][j][lane] = s;
+            if (lane == 0) {
+                S.most[warp][j] = most;
+                S.count[warp][j] = (uint8_t)__popc(bal);
+            }
+        }
+        __syncthreads();
+        if (warp == (k & 1) && g >= 0) {
+            float v[16];
+            float4* v4 = reinterpret_cast<float4*>(v);
+            int count = 0, most = 0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) v4[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if (((i == warp ? own : other) >> lane) & 1u) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) add4(v4[c], S.sums[i][lane][c]);
+                    count += S.count[i][lane];
+                    most = max(most, S.most[i][lane]);
+                }
+            }
+            if (count > 0) {
+                float* te = tet_err + 16 * (int64_t)g;
+                const int col[13] = {0, 1, 2, 5, 6, 7, 8, 9, 10, 11, 13, 14, 15};
+#pragma unroll
+                for (int c = 0; c < 13; ++c)
+                    if (v[c] != 0.f) atomicAdd(te + col[c], v[c]);
+                if (v[0] != 0.f) atomicAdd(te + 12, v[0]);
+                atomicAdd(tet_count + 2 * (int64_t)g, count);
+                atomicMax(tet_count + 2 * (int64_t)g + 1, most);
+            }
+        }
+        __syncthreads();  // the next block overwrites the records and the sums
+    }
+}
+
+__global__ void __launch_bounds__(64, 12) err_seg_kernel(const int32_t* __restrict__ ids,
+                                                         const int2* __restrict__ ranges,
+                                                         const float4* __restrict__ recs, const rm_camera cam,
+                                                         const int32_t* __restrict__ ncs,
+                                                         const float* __restrict__ pixel_err,
+                                                         const float* __restrict__ ssim_err,
+                                                         float* __restrict__ tet_err, int32_t* __restrict__ tet_count,
+                                                         const Queue q) {
+    __shared__ ErrSegSmem S;
+    __shared__ HitMasks hm;
+    if (threadIdx.x == 0) hm = live_masks(q.hm, q.subs);
+    __syncthreads();
+    const int64_t n_items = segment_items(q.info, q.G, hm.seg_shift) * q.subs;
+    for (;;) {
+        if (threadIdx.x == 0) {
+            const int item = (int)atomicAdd(q.ticket, 1u);
+            SegItem it = {-1, 0, 0};
+            if (item < n_items) it = segment_item(q, item, hm.seg_shift);
+            S.item = make_int4(it.tile, it.seg, it.sub, 0);
+        }
+        __syncthreads();
+        const int4 it = S.item;
+        __syncthreads();
+        if (it.x < 0) return;
+        err_seg_item(it.x, it.z, it.y, ids, ranges, recs, cam, ncs, pixel_err, ssim_err, tet_err, tet_count, S, hm,
+                     q.subs, q);
+    }
+}
+
 struct BlendWs {
     float4* recs;
     int32_t* order;
@@ -2789,7 +3000,7 @@ struct Shape {
 
 // Forward pass: order kernel, then one persistent kernel for the heavy tiles
 // (pair items) and the others (warp items).
-template <int PX, int NT, int B, class V>
+template <int PX, int NT, int B, class V, bool LOGT = false>
 int launch_fwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, const float* jitter, const V& views,
                const Shape& sh, float* img, float* dist, int32_t* nc, const Tuning& tn, cudaStream_t s) {
     const int G = sh.G;
@@ -2804,7 +3015,7 @@ int launch_fwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, cons
     if (rc) return rc;
     const HitMasks hm = {masks ? w.mask_words : nullptr, w.mask_cap, w.mask_header, nullptr, 0, kNoSegments};
     const Queue q = {w.order, w.info, w.tickets + 0, G, subs, true, hm, tn.status, rm_host::wait_limit(), tn.n_recs};
-    auto kernel = blend_fwd_kernel<PX, NT, B, V>;
+    auto kernel = blend_fwd_kernel<PX, NT, B, V, LOGT>;
     constexpr int kPairSmem = (int)sizeof(FwdPairSmem<PX, B>), kWarpSmem = NT / 32 * (int)sizeof(FwdWarpSmem);
     constexpr int smem = kPairSmem > kWarpSmem ? kPairSmem : kWarpSmem;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -3065,10 +3276,35 @@ int rm_calc_tet_err(const int32_t* sorted_ids, const int32_t* ranges, const int3
         rc = pack(indices, vertices, n_verts, cell_values, n_tets, tiles_touched, w.recs, s);
         if (rc) return rc;
     }
-    // every tile in one heavy-first queue (heavy_shift 1 marks all tiles heavy)
-    if ((rc = launch_order(ranges, (int)G, w, 1, s))) return rc;
     const int strip = strip_pixels(cam, flags);
     const int subs = cam->tile_width * cam->tile_height / strip;
+    // with room for hit masks and n_contributors: the forward's walk, then the
+    // statistics by stretches
+    const size_t nc_bytes = (size_t)cam->image_height * cam->image_width * sizeof(int32_t);
+    if (strip == 64 && workspace_bytes > blend_ws_bytes(n_tets, G) + nc_bytes + 512) {
+        const size_t nc_off = (workspace_bytes - nc_bytes) / 256 * 256;
+        const BlendWs wm = blend_ws(workspace, n_tets, G, nc_off);
+        if (wm.mask_header && mask_header_for(wm.mask_cap, G, subs).seg_shift < (uint32_t)kNoSegments) {
+            int32_t* nc = (int32_t*)((char*)workspace + nc_off);
+            const OneView one = {*cam};
+            const Shape sh = {(int)G, cam->tile_width * cam->tile_height};
+            Tuning tn = tuning_from_flags(flags, 0, 3);
+            tn.hit_masks = true;
+            tn.n_recs = n_tets;
+            rc = launch_fwd<64, 256, 32, OneView, true>(sorted_ids, ranges, wm, nullptr, one, sh, nullptr, nullptr, nc,
+                                                        tn, s);
+            if (rc) return rc;
+            const HitMasks hm = {wm.mask_words, wm.mask_cap, wm.mask_header, nullptr, 0, kNoSegments};
+            const Queue q = {wm.order, wm.info, wm.tickets + 2, (int)G, subs, true, hm, nullptr,
+                             rm_host::wait_limit(), n_tets};
+            const int grid = persistent_grid(err_seg_kernel, 64, 0, 1 << 30);
+            err_seg_kernel<<<grid, 64, 0, s>>>(sorted_ids, (const int2*)ranges, wm.recs, *cam, nc, pixel_err, ssim_err,
+                                               tet_err, tet_count, q);
+            return rm_host::check_launch("rm_calc_tet_err");
+        }
+    }
+    // every tile in one heavy-first queue (heavy_shift 1 marks all tiles heavy)
+    if ((rc = launch_order(ranges, (int)G, w, 1, s))) return rc;
     const Queue qd = {w.order, w.info, w.tickets + 0, (int)G, subs, true, HitMasks{}, nullptr,
                       rm_host::wait_limit(), n_tets};
     if (strip == 16) {

@@ -712,12 +712,15 @@ def calc_tet_err(sorted_ids, ranges, indices, vertices, cell_values, cam: RMCame
     if tet_count is None:
         tet_count = torch.zeros((T, 2), dtype=torch.int32, device=dev)
     L = C.lib()
-    ws_n = L.rm_blend_workspace_size(T, cam.grid_width * cam.grid_height)
+    G = cam.grid_width * cam.grid_height
+    # with room for hit masks and a count per pixel the walk and the sums run as two kernels
+    ws_n = (L.rm_blend_workspace_size(T, G) + 512 + 4 * cam.image_height * cam.image_width +
+            L.rm_blend_hit_mask_bytes(sorted_ids.shape[0], G, cam.tile_width * cam.tile_height))
     ws = _POOL.get("err", ws_n, dev)
     _call("rm_calc_tet_err", lambda: L.rm_calc_tet_err(
         C.ptr(sorted_ids), C.ptr(ranges), C.ptr(indices), C.ptr(vertices), C.ptr(cell_values), T, vertices.shape[0],
         C.ptr(tiles_touched), ctypes.byref(cam), C.ptr(pixel_err), C.ptr(ssim_err), C.ptr(tet_err),
-        C.ptr(tet_count), C.ptr(ws), ws_n, 0, _stream()))
+        C.ptr(tet_count), C.ptr(ws), ws.numel(), 0, _stream()))
     return tet_err, tet_count
 
 

@@ -8,11 +8,16 @@ takes a list in stretches of 128 entries, each from the state the forward
 left there: lists one entry short of, at and past whole stretches are compared
 with the oracle's adjoint, with pixels that end before, inside and after a
 stretch."""
+import ctypes
+
 import numpy as np
 import pytest
+import torch
 
-from gpu_util import bits, run_gpu_forward
+from gpu_util import bits, run_gpu_forward, to_dev
 from oracle import oracle as O
+from radiance_meshes_b200 import _capi as C
+from radiance_meshes_b200 import rasterizer as R
 from radiance_meshes_b200.camera import pinhole_tcam
 from test_gpu_backward import _run
 
@@ -60,3 +65,27 @@ def test_forward_over_blocks(cuda, n, small, density, tile):
     assert np.array_equal(bits(r["img"].cpu().numpy()[..., 3]), bits(img[..., 3]))
     assert np.array_equal(bits(r["dist"].cpu().numpy()), bits(dist))
     assert np.abs(r["img"].cpu().numpy() - img).max() <= 1e-4
+
+
+@pytest.mark.parametrize("n", [1, 32, 33, 127, 128, 129, 400])
+@pytest.mark.parametrize("density", [0.3, 6.0])
+def test_statistics_over_stretches(cuda, n, density):
+    """The statistics by stretches (a workspace with room for the masks) and by
+    whole lists (without): equal counts and maxima, sums within 1e-5."""
+    verts, idx, cv = _stack(n, density, n, 0.3)
+    tcam = pinhole_tcam((0.1, 0.0, 0.0), (0.0, 0.0, 1.0), 21, 18, 30.0, tile_size=8)
+    jitter = np.full((21, 18, 2), 0.5, np.float32)
+    r = run_gpu_forward(verts, idx, cv, tcam, jitter, keep_debug=False)
+    rng = np.random.default_rng(n)
+    pe, se = (to_dev(rng.uniform(0, 1, (21, 18)).astype(np.float32)) for _ in range(2))
+    L, cam = r["lists"], r["cam"]
+    err, cnt = R.calc_tet_err(L.sorted_ids, L.ranges, r["i"], r["v"], r["c"], cam, pe, se)
+    err0, cnt0 = torch.zeros_like(err), torch.zeros_like(cnt)
+    size = C.lib().rm_blend_workspace_size(n, cam.grid_width * cam.grid_height)
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    C.check(C.lib().rm_calc_tet_err(C.ptr(L.sorted_ids), C.ptr(L.ranges), C.ptr(r["i"]), C.ptr(r["v"]), C.ptr(r["c"]),
+                                    n, len(verts), None, ctypes.byref(cam), C.ptr(pe), C.ptr(se), C.ptr(err0),
+                                    C.ptr(cnt0), C.ptr(ws), size, 0, C.stream_handle()), "rm_calc_tet_err")
+    assert cnt0[:, 0].sum() > 0 and torch.equal(cnt, cnt0)
+    scale = err0.abs().amax(dim=0).clamp(min=1e-30)
+    assert ((err - err0).abs() / scale).max() <= 1e-5
