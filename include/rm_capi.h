@@ -597,6 +597,12 @@ RM_API int rm_calc_tet_err(const int32_t* sorted_ids, const int32_t* ranges,
                            float* tet_err, int32_t* tet_count, void* workspace,
                            size_t workspace_bytes, int flags, void* stream);
 
+/* Structural similarity map of n_planes pairs of height x width images, as the
+ * statistics above read it (render_err.py:121): Gaussian window of 11 taps
+ * (host pointer, separable), zero padding, C1 = 0.01^2, C2 = 0.03^2. */
+RM_API int rm_ssim_map(const float* img1, const float* img2, int n_planes, int height, int width,
+                       const float* window, float* out, void* stream);
+
 /* ------------------------------------------------- per-tet feature producer -- */
 /*
  * The cell values the blend consumes, from the model's raw per-tet outputs:

@@ -20,6 +20,14 @@ from .render_grid import RenderGrid
 from .tile_shader_slang import vertex_and_tile_shader
 
 
+def _ssim(img, gt):
+    # one kernel for the plain case (float32 images of one shape on one GPU); anything else as ssim_map takes it
+    if (type(gt) is torch.Tensor and gt.dtype == torch.float32 and gt.device == img.device and gt.shape == img.shape
+            and gt.dim() == 3):
+        return R.ssim_map(img, gt)
+    return ssim_map(img, gt)
+
+
 def render_err(gt_image, camera, model, tile_size=16, min_t=0.1, **kwargs):
     device = model.device
     indices = model.indices
@@ -41,7 +49,7 @@ def render_err(gt_image, camera, model, tile_size=16, min_t=0.1, **kwargs):
                                    tiles_touched=mask.to(torch.int32))
         render_img = img.permute(2, 0, 1)[:3].clip(min=0, max=1)
         pixel_err = (render_img - gt_image).mean(dim=0)
-        ssim_err = (1 - ssim_map(render_img, gt_image).mean(dim=0)).clip(min=0, max=1)
+        ssim_err = (1 - _ssim(render_img, gt_image).mean(dim=0)).clip(min=0, max=1)
         amask = camera.gt_alpha_mask.to(device)
         pixel_err = (pixel_err * amask[0]).contiguous()
         ssim_err = (ssim_err * amask[0]).contiguous()

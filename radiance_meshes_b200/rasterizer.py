@@ -12,6 +12,7 @@ Stage map (reference file:line in delaunay_rasterization/internal/):
 from __future__ import annotations
 
 import ctypes
+import math
 import threading
 from dataclasses import dataclass
 
@@ -722,6 +723,23 @@ def calc_tet_err(sorted_ids, ranges, indices, vertices, cell_values, cam: RMCame
         C.ptr(tiles_touched), ctypes.byref(cam), C.ptr(pixel_err), C.ptr(ssim_err), C.ptr(tet_err),
         C.ptr(tet_count), C.ptr(ws), ws.numel(), 0, _stream()))
     return tet_err, tet_count
+
+
+_SSIM_TAPS = [math.exp(-(k * k) / (2.0 * 1.5 * 1.5)) for k in range(-5, 6)]
+_SSIM_WINDOW = (ctypes.c_float * 11)(*[w / sum(_SSIM_TAPS) for w in _SSIM_TAPS])
+
+
+def ssim_map(img1: torch.Tensor, img2: torch.Tensor) -> torch.Tensor:
+    """The map of ``ssim.ssim_map`` (11 taps, sigma 1.5) of two float32 CUDA
+    images [C,H,W] by one kernel (rm_ssim_map), without gradients."""
+    _require_cuda(img1=img1, img2=img2)
+    a, b = _f32(img1.detach()), _f32(img2.detach())
+    if a.dim() != 3 or a.shape != b.shape or a.device != b.device:
+        raise ValueError("two [C,H,W] images of one shape on one device")
+    out = torch.empty_like(a)
+    _call("rm_ssim_map", lambda: C.lib().rm_ssim_map(C.ptr(a), C.ptr(b), a.shape[0], a.shape[1], a.shape[2],
+                                                     _SSIM_WINDOW, C.ptr(out), _stream()))
+    return out
 
 
 def read_status(workspace: torch.Tensor) -> int:

@@ -100,3 +100,17 @@ def test_render_err_dropin(cuda):
     ref_err, ref_cnt, ref_max = O.calc_tet_err(lists, mesh.indices, mesh.vertices, mesh.cell_values,
                                                extras["pixel_err"].cpu().numpy(), extras["ssim_err"].cpu().numpy())
     _check(tet_err, extras["tet_count"], ref_err, ref_cnt, ref_max)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 5, 7), (3, 32, 32), (1, 33, 31), (3, 75, 130), (2, 11, 200)])
+def test_ssim_map_matches_convolutions(cuda, shape):
+    """The fused map against the convolutions in 64 bits: an error of a few
+    float32 roundings of the moments (3e-7) over the least denominator (the
+    images' variance is near 1/12)."""
+    from radiance_meshes_b200.ssim import ssim_map
+
+    g = torch.Generator("cuda").manual_seed(sum(shape))
+    a, b = (torch.rand(shape, device="cuda", generator=g) for _ in range(2))
+    got, ref = R.ssim_map(a, b).double(), ssim_map(a.double(), b.double())
+    assert got.shape == ref.shape and (got - ref).abs().max() <= 2e-5
+    assert (R.ssim_map(a.transpose(1, 2).contiguous().transpose(1, 2), b).double() - ref).abs().max() <= 2e-5
