@@ -5,6 +5,12 @@
 // adjoint.  One thread per tet: 4 vertex gathers, the circumcenter, the raw
 // attributes and the SH coefficients in, the 7 cell values out.
 //
+// Bound: HBM.  Where a tet's SH rows are packed, they and their gradient pass
+// through shared memory in 16-byte pieces, so that a warp moves whole lines:
+// read by one thread per tet, 180 bytes apart, the backward at degree 3 over
+// 1.3M tets took 432 us, now 199, and the forward 105, now 90.  (4-byte
+// pieces: 545 and 230.)
+//
 // Per tet (rgb, grd, density, sh_rest, circumcenter cc, vertices v0..v3):
 //   m      = min(rgb)                          g  = grd * m
 //   r      = |v0 - cc|                         ng = safe_div(g, r)
@@ -81,16 +87,19 @@ __device__ __forceinline__ f3 vload(const float* p, int i) {
     return {__ldg(q), __ldg(q + 1), __ldg(q + 2)};
 }
 
-template <int DEG, bool BWD>
-__global__ void __launch_bounds__(128) features_kernel(
-    const int4* __restrict__ indices, const float* __restrict__ verts, int64_t n_verts, const float* __restrict__ ccs,
-    const float* __restrict__ density, const float* __restrict__ rgb, const float* __restrict__ grd,
-    const float* __restrict__ sh, int n_rest, f3 cam, int64_t n_tets, float* __restrict__ feat,
-    const float* __restrict__ gfeat, float* __restrict__ g_density, float* __restrict__ g_rgb,
-    float* __restrict__ g_grd, float* __restrict__ g_sh, float* __restrict__ g_verts, float* __restrict__ g_cc) {
+constexpr int kThreads = 128;
+
+// One tet, with its n_rest SH rows at shp and their gradient to gsh (which may
+// be the same place).
+template <int DEG, bool BWD, bool STAGED>
+__device__ __forceinline__ void tet_features(
+    int64_t t, const float* shp, float* gsh, int n_rest, const int4* __restrict__ indices, const float* __restrict__ verts, int64_t n_verts,
+    const float* __restrict__ ccs, const float* __restrict__ density, const float* __restrict__ rgb,
+    const float* __restrict__ grd, f3 cam, float* __restrict__ feat, const float* __restrict__ gfeat,
+    float* __restrict__ g_density, float* __restrict__ g_rgb, float* __restrict__ g_grd, float* __restrict__ g_verts,
+    float* __restrict__ g_cc) {
     constexpr int kRest = (DEG + 1) * (DEG + 1) - 1;
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_tets) return;
+    auto sh_at = [&](int k) { return STAGED ? shp[k] : __ldg(shp + k); };
     const int4 id = __ldg(indices + t);
     if (!tet_indices_ok(id, n_verts)) {  // zero features, no gradients; the vertices are never read
         if (!BWD) {
@@ -100,7 +109,7 @@ __global__ void __launch_bounds__(128) features_kernel(
             g_density[t] = 0.f;
 #pragma unroll
             for (int k = 0; k < 3; ++k) g_rgb[3 * t + k] = g_grd[3 * t + k] = g_cc[3 * t + k] = 0.f;
-            for (int k = 0; k < 3 * n_rest; ++k) g_sh[(int64_t)3 * n_rest * t + k] = 0.f;
+            for (int k = 0; k < 3 * n_rest; ++k) gsh[k] = 0.f;
         }
         return;
     }
@@ -113,7 +122,7 @@ __global__ void __launch_bounds__(128) features_kernel(
             g_density[t] = 0.f;
 #pragma unroll
             for (int k = 0; k < 3; ++k) g_rgb[3 * t + k] = g_grd[3 * t + k] = g_cc[3 * t + k] = 0.f;
-            for (int k = 0; k < 3 * n_rest; ++k) g_sh[(int64_t)3 * n_rest * t + k] = 0.f;
+            for (int k = 0; k < 3 * n_rest; ++k) gsh[k] = 0.f;
             return;
         }
     }
@@ -154,13 +163,12 @@ __global__ void __launch_bounds__(128) features_kernel(
     D3 Y[kRest > 0 ? kRest : 1];
     if (DEG > 0)
         sh_basis<DEG>({dir.x, 1.f, 0.f, 0.f}, {dir.y, 0.f, 1.f, 0.f}, {dir.z, 0.f, 0.f, 1.f}, Y);
-    const float* shp = sh + (int64_t)n_rest * 3 * t;
     float col[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const float sh0 = (c0[k] - 0.5f) / (float)kC0;
         float acc = (float)kC0 * sh0 + 0.5f;
-        for (int j = 0; j < kRest; ++j) acc = acc + Y[j].v * __ldg(shp + 3 * j + k);
+        for (int j = 0; j < kRest; ++j) acc = acc + Y[j].v * sh_at(3 * j + k);
         col[k] = acc;
     }
     if (!BWD) {
@@ -188,19 +196,16 @@ __global__ void __launch_bounds__(128) features_kernel(
     }
     // sh_rest and the direction
     f3 ddir = {0.f, 0.f, 0.f};
-    float* gsh = g_sh + (int64_t)n_rest * 3 * t;
     for (int j = 0; j < kRest; ++j) {
         float s = 0.f;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
+            s = fmaf(dcol[k], sh_at(3 * j + k), s);
             gsh[3 * j + k] = dcol[k] * Y[j].v;
-            s = fmaf(dcol[k], __ldg(shp + 3 * j + k), s);
         }
         ddir = {fmaf(s, Y[j].dx, ddir.x), fmaf(s, Y[j].dy, ddir.y), fmaf(s, Y[j].dz, ddir.z)};
     }
-    for (int j = kRest; j < n_rest; ++j)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) gsh[3 * j + k] = 0.f;
+    for (int j = 3 * kRest; j < 3 * n_rest; ++j) gsh[j] = 0.f;
     // normalize(u, eps): (I - dir dir^T) / |u| above eps, I / eps below
     f3 du;
     if (un > 1e-8f) {
@@ -256,26 +261,89 @@ __global__ void __launch_bounds__(128) features_kernel(
     }
 }
 
+// STAGED: n_rest is the degree's own number of rows and sh, g_sh are 16-byte
+// aligned.
+template <int DEG, bool BWD, bool STAGED>
+__global__ void __launch_bounds__(kThreads) features_kernel(
+    const int4* __restrict__ indices, const float* __restrict__ verts, int64_t n_verts, const float* __restrict__ ccs,
+    const float* __restrict__ density, const float* __restrict__ rgb, const float* __restrict__ grd,
+    const float* __restrict__ sh, int n_rest, f3 cam, int64_t n_tets, float* __restrict__ feat,
+    const float* __restrict__ gfeat, float* __restrict__ g_density, float* __restrict__ g_rgb,
+    float* __restrict__ g_grd, float* __restrict__ g_sh, float* __restrict__ g_verts, float* __restrict__ g_cc) {
+    const int64_t t0 = (int64_t)blockIdx.x * kThreads, t = t0 + threadIdx.x;
+    if constexpr (!STAGED) {
+        if (t < n_tets)
+            tet_features<DEG, BWD, false>(t, sh + (int64_t)n_rest * 3 * t,
+                                          BWD ? g_sh + (int64_t)n_rest * 3 * t : nullptr, n_rest, indices, verts,
+                                   n_verts, ccs, density, rgb, grd, cam, feat, gfeat, g_density, g_rgb, g_grd,
+                                   g_verts, g_cc);
+        return;
+    } else {
+        constexpr int kRow = 3 * ((DEG + 1) * (DEG + 1) - 1);
+        __shared__ __align__(16) float rows[kThreads * kRow];
+        const int64_t left = n_tets - t0;
+        const int n = left < kThreads ? (int)left : kThreads, words = n * kRow;
+        bool use = t < n_tets;
+        if (BWD && use) {  // rows are read by tets with a gradient only
+            bool zero = true;
+#pragma unroll
+            for (int k = 0; k < 7; ++k) zero &= __ldg(gfeat + 7 * t + k) == 0.f;
+            use = !zero;
+        }
+        if (__syncthreads_or(use)) {
+            const float* src = sh + t0 * kRow;
+            for (int i = threadIdx.x; i < words / 4; i += kThreads) async_copy16(rows + 4 * i, src + 4 * i);
+            for (int i = words / 4 * 4 + threadIdx.x; i < words; i += kThreads) rows[i] = __ldg(src + i);
+            async_wait();
+        }
+        __syncthreads();
+        if (t < n_tets)
+            tet_features<DEG, BWD, true>(t, rows + threadIdx.x * kRow, rows + threadIdx.x * kRow, n_rest, indices, verts,
+                                   n_verts, ccs, density, rgb, grd, cam, feat, gfeat, g_density, g_rgb, g_grd, g_verts,
+                                   g_cc);
+        if (!BWD) return;
+        __syncthreads();
+        float* dst = g_sh + t0 * kRow;
+        const float4* rows4 = reinterpret_cast<const float4*>(rows);
+        for (int i = threadIdx.x; i < words / 4; i += kThreads) reinterpret_cast<float4*>(dst)[i] = rows4[i];
+        for (int i = words / 4 * 4 + threadIdx.x; i < words; i += kThreads) dst[i] = rows[i];
+    }
+}
+
 template <bool BWD>
 int launch_features(int deg, const int32_t* indices, const float* vertices, int64_t n_verts, const float* ccs,
                     const float* density,
                     const float* rgb, const float* grd, const float* sh, int n_rest, const float* cam, int64_t T,
                     float* feat, const float* gfeat, float* gd, float* grgb, float* ggrd, float* gsh, float* gv,
                     float* gcc, cudaStream_t s) {
-    const int threads = 128;
+    const int threads = kThreads;
     const int64_t blocks = (T + threads - 1) / threads;
     const f3 c = {cam[0], cam[1], cam[2]};
-#define RM_FEAT(D)                                                                                              \
-    features_kernel<D, BWD><<<(unsigned)blocks, threads, 0, s>>>((const int4*)indices, vertices, n_verts, ccs,    \
+    const bool aligned = ((uintptr_t)sh & 15) == 0 && (!BWD || ((uintptr_t)gsh & 15) == 0);
+    // when the degree's rows are all there is (1.3M tets, in place and staged:
+    // degree 1 forward 49 and 59 us, backward 156 and 135; degree 2 forward 72
+    // and 80, backward 269 and 182; degree 3 105 and 90, 432 and 199)
+    const bool staged = aligned && n_rest == (deg + 1) * (deg + 1) - 1 && (deg == 3 || BWD);
+#define RM_FEAT(D, ST)                                                                                           \
+    features_kernel<D, BWD, ST><<<(unsigned)blocks, threads, 0, s>>>((const int4*)indices, vertices, n_verts, ccs,    \
                                                                  density,                                         \
                                                                  rgb, grd, sh, n_rest, c, T, feat, gfeat, gd,      \
                                                                  grgb, ggrd, gsh, gv, gcc)
     switch (deg) {
-        case 0: RM_FEAT(0); break;
-        case 1: RM_FEAT(1); break;
-        case 2: RM_FEAT(2); break;
-        case 3: RM_FEAT(3); break;
-        default: RM_FEAT(4); break;
+        case 0: RM_FEAT(0, false); break;
+        case 1:
+            if (staged) RM_FEAT(1, true);
+            else RM_FEAT(1, false);
+            break;
+        case 2:
+            if (staged) RM_FEAT(2, true);
+            else RM_FEAT(2, false);
+            break;
+        case 3:
+            if (staged) RM_FEAT(3, true);
+            else RM_FEAT(3, false);
+            break;
+        default: RM_FEAT(4, false); break;
     }
 #undef RM_FEAT
     return rm_host::check_launch(BWD ? "rm_activate_features_bwd" : "rm_activate_features");

@@ -86,3 +86,26 @@ def test_activate_output_matches_torch(cuda, deg):
             continue
         rel = float((a - b).norm() / (b.norm() + 1e-30))
         assert rel < 1e-4, (name, rel)
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 300])
+@pytest.mark.parametrize("deg,rows,shift", [(1, 3, 0), (3, 15, 0), (3, 15, 1), (1, 15, 0), (2, 8, 0)])
+def test_activate_output_row_layouts(cuda, n, deg, rows, shift):
+    """SH rows in whole and partial blocks of tets, more rows than the degree
+    uses, rows that start off a 16-byte boundary, and tets without a gradient."""
+    g = torch.Generator("cuda").manual_seed(n + deg)
+    v = torch.randn(60, 3, device="cuda", generator=g, requires_grad=True)
+    idx = torch.stack([torch.randperm(60, generator=g, device="cuda")[:4] for _ in range(n)]).int()
+    cc = torch.randn(n, 3, device="cuda", generator=g, requires_grad=True)
+    dens, rgb, grd = (torch.rand(n, k, device="cuda", generator=g, requires_grad=True) for k in (1, 3, 3))
+    flat = 0.3 * torch.randn(n * rows * 3 + shift, device="cuda", generator=g)
+    sh = flat[shift:].view(n, rows, 3).detach().requires_grad_(True)
+    cam = torch.tensor([3.0, 1.0, -2.0], device="cuda")
+    w = torch.randn(n, 7, device="cuda", generator=g)
+    w[torch.rand(n, device="cuda", generator=g) < 0.5] = 0.0
+    params = [dens, rgb, grd, sh, cc, v]
+    out = FT.activate_output(cam, dens, rgb, grd, sh, idx, cc, v, deg, 3)
+    ref = _reference(cam, dens, rgb, grd, sh, idx, cc, v, deg)
+    assert (out - ref).abs().max() <= 1e-5 * ref.abs().max()
+    for a, b in zip(torch.autograd.grad(out, params, w), torch.autograd.grad(ref, params, w)):
+        assert (a - b).norm() <= 1e-4 * b.norm() + 1e-6
