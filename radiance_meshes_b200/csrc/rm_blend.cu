@@ -1245,12 +1245,15 @@ __global__ void __launch_bounds__(1024) order_kernel(const int2* __restrict__ ra
         int heavy = 0;
         for (int b = 32; b >= b_thr; --b) heavy += (int)cnt[b];
         info[0] = heavy;
-        // Tiles whose list is longer than one resident CTA's share of all
-        // entries go by quarters: walked by one CTA each, they would outlast
-        // the launch.  A launch with fewer strips than CTAs splits most.
+        // Tiles whose list is longer than a fourth of one resident CTA's share
+        // of all entries go by quarters: walked by one CTA each, they would
+        // outlast the launch.  With few strips to a CTA there is little else to
+        // fill the launch with and a quarter's overhead counts: a whole share.
+        // (1.3M tets, 39 strips to a CTA: 1048 us at a fourth, 1268 at a whole;
+        // 27k tets at 256x256, 2.3 strips: 165 and 140.)
         int quarters = 0;
         if (fwd_slots > 0) {
-            const unsigned long long share = sum / (4ull * fwd_slots);
+            const unsigned long long share = sum / ((ne >= 8u * fwd_slots ? 4ull : 1ull) * fwd_slots);
             for (int b = 32; b > 0 && (1ull << (b - 1)) >= share; --b) quarters += (int)cnt[b];
         }
         info[1] = min(quarters, heavy);
