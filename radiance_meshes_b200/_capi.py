@@ -160,8 +160,10 @@ def ptr(t) -> int | None:
 def stream_handle(stream=None) -> int:
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    # torch.cuda.current_stream().cuda_stream without the Stream object (5 us a call)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def status_text(bits: int) -> str:

@@ -63,7 +63,7 @@ def _key_of(x):
     if isinstance(x, torch.Tensor):
         # identity, storage and version: an in-place change bumps the version,
         # and the cache holds the tensor, so neither id nor storage is reused
-        return ("t", id(x), x.data_ptr(), x._version, str(x.device), tuple(x.shape), str(x.dtype))
+        return ("t", id(x), x.data_ptr(), x._version, x.device, x.shape, x.dtype)
     if x is None or isinstance(x, (int, float, str)):
         return ("v", x)
     return ("a", tuple(np.asarray(x, dtype=np.float64).reshape(-1).tolist()))

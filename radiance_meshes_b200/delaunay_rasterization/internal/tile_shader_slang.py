@@ -42,7 +42,7 @@ def vertex_and_tile_shader(indices, vertices, cam, render_grid):
     if fs:
         with torch.no_grad():
             tiles, rect, vs, cc, footprint = R.project_fwd_fine(indices, vertices, camst)
-        pre = (tiles, rect, vs, cc)
+        pre = (tiles, rect, vs, cc, camst)
     tiles_touched, rect_tile_space, vs_tetra, circumcenter = VertexShader.apply(
         indices, vertices, cam, render_grid, "cuda", pre)
     with torch.no_grad():
@@ -58,12 +58,12 @@ def vertex_and_tile_shader(indices, vertices, cam, render_grid):
 class VertexShader(torch.autograd.Function):
     @staticmethod
     def forward(ctx, indices, vertices, tcam, render_grid, device="cuda", precomputed=None):
-        camst = tcam_to_struct(tcam)
         indices = indices.contiguous()
         vertices = vertices.contiguous()
-        if precomputed is not None:  # outputs of project_fwd_fine for these inputs
-            tiles_touched, rect_tile_space, vs_tetra, circumcenter = precomputed
+        if precomputed is not None:  # outputs of project_fwd_fine for these inputs, and the camera
+            tiles_touched, rect_tile_space, vs_tetra, circumcenter, camst = precomputed
         else:
+            camst = tcam_to_struct(tcam)
             tiles_touched, rect_tile_space, vs_tetra, circumcenter = R.project_fwd(indices, vertices, camst)
         ctx.save_for_backward(indices, vertices, tiles_touched)
         ctx.camst = camst

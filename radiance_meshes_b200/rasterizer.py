@@ -291,28 +291,26 @@ def project_bwd(indices, vertices, cam: RMCamera, tiles, grad_vs, grad_cc, grad_
 
 
 _PAIR_GUESS: dict = {}  # device -> pair count of the last frame built there
-_SIDE: dict = {}  # (device, thread) -> (side stream, pinned int64 [2], its numpy view) for the pair-count read
+_COUNT_READ: dict = {}  # (device, thread) -> (pinned int64 [2], its numpy view) for the pair-count read
 
 
 def _count_read_start(count: torch.Tensor):
     """Copy ``count`` (int64 [2] on the device: pair count, status word) to
-    pinned host memory on a side stream that waits for the work queued so
-    far only, so the frame's stream goes on with what is queued after this
-    call while the host waits in _count_read_finish."""
+    pinned host memory; the host waits in _count_read_finish for the copy
+    only, while the GPU goes on with what is queued after this call.  (On a
+    side stream the 16-byte copy left the frame's stream alone, and cost the
+    host two events and a stream switch: 20 us of a small frame's 445.)"""
     dev = count.device
     key = (dev, threading.get_ident())  # threads building frames at once each read their own buffer
-    st = _SIDE.get(key)
+    st = _COUNT_READ.get(key)
     if st is None:
         hb = torch.zeros(2, dtype=torch.int64, pin_memory=True)
-        st = (torch.cuda.Stream(device=dev), hb, hb.numpy())
-        _SIDE[key] = st
-    side, hb, hn = st
-    side.wait_stream(torch.cuda.current_stream(dev))
-    count.record_stream(side)
-    with torch.cuda.stream(side):
-        hb.copy_(count, non_blocking=True)
+        st = (hb, hb.numpy())
+        _COUNT_READ[key] = st
+    hb, hn = st
+    hb.copy_(count, non_blocking=True)
     done = torch.cuda.Event()
-    done.record(side)
+    done.record()
     return done, hn
 
 
@@ -345,7 +343,7 @@ def build_tile_lists(tiles: torch.Tensor, rect: torch.Tensor, vs: torch.Tensor, 
 
     By default the lists are built depth first (use_depth_first_lists): P is
     counted right after the projection (rm_count_pairs) and copied to the
-    host on a side stream.  After the first frame on a device, the pair
+    host.  After the first frame on a device, the pair
     buffers are sized from the previous frame's count (plus a quarter) and
     the whole build is queued before P is read, so the host goes on while
     the GPU builds the lists; a frame with more pairs than that is built
@@ -367,20 +365,19 @@ def build_tile_lists(tiles: torch.Tensor, rect: torch.Tensor, vs: torch.Tensor, 
     L = C.lib()
     s = _stream()
     end_bit = end_bit_for(cam.grid_width, cam.grid_height)
-    total = torch.zeros(1, dtype=torch.int64, device=dev)
+    total, n_vis = torch.zeros(2, dtype=torch.int64, device=dev).split(1)
     status = frame_status(T, dev, pool)  # the stages or their RM_STATUS_* bits into it
     depth_first = _LISTS["depth_first"] and not keep_debug and T > 0
 
     if depth_first:
         # the pair count and the status word as the projection left them,
-        # copied to the host on a side stream (read once the build is queued)
+        # copied to the host (read once the build is queued)
         count = torch.empty(2, dtype=torch.int64, device=dev)
         _call("rm_count_pairs", lambda: L.rm_count_pairs(C.ptr(tiles), T, C.ptr(status), C.ptr(count), s))
         pending = _count_read_start(count)
         # visible tets by depth, once; the pairs then need the tile bits only
         dkeys = torch.empty(T, dtype=torch.int64, device=dev)
         dvals = torch.empty(T, dtype=torch.int32, device=dev)
-        n_vis = torch.zeros(1, dtype=torch.int64, device=dev)
         dws_n = L.rm_depth_order_workspace_size(T)
         dws = pool.get("depth", dws_n, dev)
         _call("rm_depth_order", lambda: L.rm_depth_order(C.ptr(tiles), C.ptr(vs), T, C.ptr(dkeys), C.ptr(dvals),

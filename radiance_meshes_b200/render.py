@@ -68,7 +68,7 @@ def render(camera, model, cell_values=None, tile_size=16, min_t=0.1, scene_scali
     sh_reg = 0
     if cell_values is None:
         cell_values = torch.zeros((mask.shape[0], model.feature_dim), device=circumcenter.device)
-        if mask.sum() > 0 and model.mask_values:
+        if model.mask_values and mask.sum() > 0:  # the sum waits for the GPU: only where it decides
             shs, values = model.get_cell_values(camera, mask, circumcenter[mask])
             cell_values[mask] = values
         else:
