@@ -199,28 +199,6 @@ struct Weights {
     float alpha, w0, w1;
 };
 
-// Two floats in one register pair: packed operations round each half as the
-// scalar ones do and take one issue slot for both.
-using Pair = unsigned long long;
-__device__ __forceinline__ Pair pair(float lo, float hi) {
-    Pair r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpair(Pair p, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
-}
-__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
-    Pair r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ Pair add2(Pair a, Pair b) {
-    Pair r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 // exp(x) for x <= 0 and 1 / x by the approximate instructions alone: __expf and
 // __fdividef add range handling (six instructions each time) for results
 // below 2^-126 and divisors above 2^126, and are equal to these elsewhere.
@@ -235,22 +213,28 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return y;
 }
 
+// FUSED: the series with fused operations, for gradients.  The forward rounds
+// each product and sum, as it always has: a last bit of the image decides the
+// sign of an L1 loss where the two nearly meet.
+template <bool FUSED = false>
 __device__ __forceinline__ Weights seg_weights(float x) {
     Weights w;
     w.alpha = exp_approx(-x);
     if (x < 0.25f) {
         // w1 = x/2 - x^2/6 + x^3/24 - x^4/120 + x^5/720 - x^6/5040 + x^7/40320
         // w0 = x/2 - x^2/3 + x^3/8 - x^4/30 + x^5/144 - x^6/840 + x^7/5760
-        // both at once, a product and a sum rounded separately at each step
-        const Pair xx = pair(x, x);
-        Pair p = pair(1.0f / 40320.0f, 1.0f / 5760.0f);
-        p = add2(mul2(p, xx), pair(-1.0f / 5040.0f, -1.0f / 840.0f));
-        p = add2(mul2(p, xx), pair(1.0f / 720.0f, 1.0f / 144.0f));
-        p = add2(mul2(p, xx), pair(-1.0f / 120.0f, -1.0f / 30.0f));
-        p = add2(mul2(p, xx), pair(1.0f / 24.0f, 0.125f));
-        p = add2(mul2(p, xx), pair(-1.0f / 6.0f, -1.0f / 3.0f));
-        p = add2(mul2(p, xx), pair(0.5f, 0.5f));
-        unpair(mul2(p, xx), w.w1, w.w0);
+        const float c1[7] = {1.0f / 40320.0f, -1.0f / 5040.0f, 1.0f / 720.0f, -1.0f / 120.0f, 1.0f / 24.0f,
+                             -1.0f / 6.0f, 0.5f};
+        const float c0[7] = {1.0f / 5760.0f, -1.0f / 840.0f, 1.0f / 144.0f, -1.0f / 30.0f, 0.125f, -1.0f / 3.0f, 0.5f};
+        w.w1 = c1[0];
+        w.w0 = c0[0];
+#pragma unroll
+        for (int k = 1; k < 7; ++k) {
+            w.w1 = FUSED ? fmaf(w.w1, x, c1[k]) : w.w1 * x + c1[k];
+            w.w0 = FUSED ? fmaf(w.w0, x, c0[k]) : w.w0 * x + c0[k];
+        }
+        w.w1 = w.w1 * x;
+        w.w0 = w.w0 * x;
     } else {
         const float phi = (1.0f - w.alpha) * rcp_approx(x);
         w.w0 = phi - w.alpha;
@@ -1860,7 +1844,7 @@ __device__ __forceinline__ void bwd_item(
                 const f3 base = {q[1].w, q[2].w, q[3].w};
                 const float gd = dot3(grd, d);
                 const float ce = dot3(grd, ve), cx = dot3(grd, vx);
-                const Weights wt = seg_weights(a);
+                const Weights wt = seg_weights<true>(a);
                 const float wsum = wt.w0 + wt.w1;
                 const float lin = fmaf(wt.w0, cx, wt.w1 * ce);
                 // undo_alpha_out (alphablend_shader_interp.slang:128-192): only
