@@ -999,20 +999,28 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
 // of 32 records is copied to the warp's shared memory (asynchronous 16-byte
 // copies, eight lanes to a record's line; one lane per record took six times
 // the L1 lookups), each lane looks at one entry, and those that the warp's
-// rays can hit (entry_reaches) are walked in order.  No exchange of results and no barrier across warps: a third fewer instructions
-// per ray/tet test than the pair items, but a list's walk takes as long as one
-// warp needs, so only lists that many other warps outlast come here
-// (order_kernel).
+// rays can hit (entry_reaches) are walked in order.  No exchange of results
+// and no barrier across warps: a third fewer instructions per ray/tet test
+// than the pair items, but a list's walk takes as long as one warp needs, so
+// only lists that many other warps outlast come here (order_kernel).
+//
+// AHEAD: the next block's records are copied while this one is walked, into a
+// second buffer.  Launches of several views take it: 16 views of a million
+// tets 34.8 -> 33.6 ms, 4 views of 250k 3840 -> 3713 us.  One view's launch,
+// whose walks are fewer and shorter, loses more by what the second buffers
+// (110 KB an SM) take from the L1: 1297x840 1041 -> 1065 us, 1920x1080 1496 ->
+// 1530, 640x481 738 -> 752.
+template <bool AHEAD>
 struct FwdWarpSmem {
-    float4 srec[32][kRecFloat4 + 1];  // padded: 32 lanes read one record each without conflicts
+    float4 srec[AHEAD ? 2 : 1][32][kRecFloat4 + 1];  // padded: 32 lanes read one record each without conflicts
 };
 
-template <int PX, bool LOGT>
+template <int PX, bool LOGT, bool AHEAD>
 __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const int32_t* __restrict__ ids,
                                               const int2* __restrict__ ranges, const float4* __restrict__ recs,
                                               const float2* __restrict__ jitter, const rm_camera& cam,
                                               float4* __restrict__ out_img, float* __restrict__ out_dist,
-                                              int32_t* __restrict__ out_nc, FwdWarpSmem& S, const HitMasks& hm,
+                                              int32_t* __restrict__ out_nc, FwdWarpSmem<AHEAD>& S, const HitMasks& hm,
                                               int subs, int gtile, const Queue& lq) {
     const int lane = threadIdx.x & 31;
     const int2 rg = __ldg(ranges + tile);
@@ -1050,32 +1058,48 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
     int32_t nc = rg.y - rg.x;  // entries walked: all of them unless log T runs out
     bool active = inside && nc > 0;
     bounds(active);
-    int32_t g = rg.x + lane < rg.y ? list_id(ids, rg.x + lane, lq) : -1;  // this lane's entry of the next block
-    for (int base = rg.x; base < rg.y && __any_sync(0xffffffffu, active); base += 32) {
-        if (PX == 64 && active) write_checkpoint(hm, st, rg.x, base, sub, subs, p);
+    // This lane's entry of a block, and the copies of a block's records.
+    auto entry = [&](int base) { return base + lane < rg.y ? list_id(ids, base + lane, lq) : -1; };
+    auto fetch = [&](int b, int32_t g) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int k = 4 * i + (lane >> 3);
             const int32_t gk = __shfl_sync(0xffffffffu, g, k);
-            if (gk >= 0) async_copy16(&S.srec[k][lane & 7], recs + (int64_t)kRecFloat4 * gk + (lane & 7));
+            if (gk >= 0) async_copy16(&S.srec[b][k][lane & 7], recs + (int64_t)kRecFloat4 * gk + (lane & 7));
         }
+        async_commit();
+    };
+    int32_t g = entry(rg.x), g_ahead = AHEAD ? entry(rg.x + 32) : -1;
+    if (AHEAD && __any_sync(0xffffffffu, active)) fetch(0, g);
+    int buf = 0;
+    for (int base = rg.x; base < rg.y && __any_sync(0xffffffffu, active); base += 32) {
+        if (PX == 64 && active) write_checkpoint(hm, st, rg.x, base, sub, subs, p);
         const bool valid = g >= 0;
-        g = base + 32 + lane < rg.y ? list_id(ids, base + 32 + lane, lq) : -1;
-        async_wait();
+        if (AHEAD) {
+            g = g_ahead;
+            fetch(buf ^ 1, g);
+            g_ahead = entry(base + 64);
+            async_wait_but_last();
+        } else {
+            fetch(0, g);
+            g = entry(base + 32);
+            async_wait();
+        }
         __syncwarp();
-        const bool keep = valid && S.srec[lane][0].w > 0.f &&  // a density of zero hits nothing
-                          (!(inv_z > 0.f) || entry_reaches(S.srec[lane], cam, bd, inv_z));
+        const float4(*rec)[kRecFloat4 + 1] = S.srec[buf];
+        const bool keep = valid && rec[lane][0].w > 0.f &&  // a density of zero hits nothing
+                          (!(inv_z > 0.f) || entry_reaches(rec[lane], cam, bd, inv_z));
         const uint32_t bal = __ballot_sync(0xffffffffu, keep);
         uint32_t hb = 0;  // bit k: entry k of the block was a hit for this lane's pixel
         bool ended = false;
         if (active) {
             for (uint32_t left = bal; left; left &= left - 1u) {
                 const int j = __ffs(left) - 1;
-                const EntryResult e = eval_entry<LOGT>(S.srec[j], o, d);
+                const EntryResult e = eval_entry<LOGT>(rec[j], o, d);
                 if (e.a > 0.f) {
                     hb |= 1u << j;
                     if (LOGT) st.logT = st.logT - e.a;
-                    else fold_hit(st, e.a, S.srec[j][0].w, e.m1, e.d4, e.rgb);
+                    else fold_hit(st, e.a, rec[j][0].w, e.m1, e.d4, e.rgb);
                     if (st.logT < kTermLogT) {
                         nc = base - rg.x + j + 1;
                         ended = true;
@@ -1093,6 +1117,11 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
             bounds(active);
         }
         __syncwarp();  // the walk's reads of the records are done
+        if (AHEAD) buf ^= 1;
+    }
+    if (AHEAD) {  // the copies ahead, before the next item's
+        async_wait();
+        __syncwarp();
     }
     if (inside) {
         out_nc[pix] = nc;
@@ -1141,7 +1170,8 @@ __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
                                  out_img + pb, out_dist + 5 * pb, out_nc + pb, S, hm, q.subs, t, q);
     }
     constexpr int kParts = PX / 32 > 0 ? PX / 32 : 1;
-    FwdWarpSmem& W = reinterpret_cast<FwdWarpSmem*>(fwd_smem_raw)[threadIdx.x >> 5];
+    constexpr bool kAhead = V::kViews > 1;
+    FwdWarpSmem<kAhead>& W = reinterpret_cast<FwdWarpSmem<kAhead>*>(fwd_smem_raw)[threadIdx.x >> 5];
     const int heavy = __ldg(q.info);
     const int w_items = (q.G - heavy) * q.subs * kParts;
     for (;;) {
@@ -1153,7 +1183,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
         const int t = __ldg(q.order + heavy + strip / q.subs), v = views.find(t);
         const int tb = views.tile_base(v);
         const int64_t pb = views.pixel_base(v);
-        fwd_warp_item<PX, LOGT>(t - tb, strip % q.subs, part, ids, ranges + tb, recs, jitter + pb, views.camera(v),
+        fwd_warp_item<PX, LOGT, kAhead>(t - tb, strip % q.subs, part, ids, ranges + tb, recs, jitter + pb, views.camera(v),
                           out_img + pb, out_dist + 5 * pb, out_nc + pb, W, hm, q.subs, t, q);
     }
 }
@@ -1178,18 +1208,31 @@ __global__ void __launch_bounds__(1024) order_kernel(const int2* __restrict__ ra
     __syncthreads();
     unsigned long long total = 0ull;
     uint32_t nonempty = 0u;
+    // Each pass is a chain of load, match and shared atomic a tile; kBatch
+    // tiles' loads are in flight at a time.
+    constexpr int kBatch = 8;
     const int G_pad = (G + 31) & ~31;  // whole warps iterate together
-    for (int t = threadIdx.x; t < G_pad; t += blockDim.x) {
-        uint32_t len = 0u;
-        if (t < G) {
-            const int2 r = __ldg(ranges + t);
-            len = (uint32_t)max(r.y - r.x, 0);
+    auto lengths = [&](int t0, uint32_t* len) {
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const int t = t0 + k * (int)blockDim.x;
+            const int2 r = t < G ? __ldg(ranges + t) : make_int2(0, 0);
+            len[k] = (uint32_t)max(r.y - r.x, 0);
         }
-        total += len;
-        nonempty += __popc(__ballot_sync(0xffffffffu, len != 0u));
-        const int b = t < G ? 32 - __clz(len) : 33;
-        const unsigned peers = __match_any_sync(0xffffffffu, b);
-        if (b < 33 && lane == __ffs(peers) - 1) atomicAdd(&cnt[b], (uint32_t)__popc(peers));
+    };
+    for (int t0 = threadIdx.x; t0 < G_pad; t0 += kBatch * blockDim.x) {
+        uint32_t len[kBatch];
+        lengths(t0, len);
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const int t = t0 + k * (int)blockDim.x;
+            if (t >= G_pad) break;
+            total += len[k];
+            nonempty += __popc(__ballot_sync(0xffffffffu, len[k] != 0u));
+            const int b = t < G ? 32 - __clz(len[k]) : 33;
+            const unsigned peers = __match_any_sync(0xffffffffu, b);
+            if (b < 33 && lane == __ffs(peers) - 1) atomicAdd(&cnt[b], (uint32_t)__popc(peers));
+        }
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
@@ -1251,18 +1294,21 @@ __global__ void __launch_bounds__(1024) order_kernel(const int2* __restrict__ ra
     }
     __syncthreads();
     const unsigned lt = (1u << lane) - 1u;
-    for (int t = threadIdx.x; t < G_pad; t += blockDim.x) {
-        int b = 33;
-        if (t < G) {
-            const int2 r = __ldg(ranges + t);
-            b = 32 - __clz((uint32_t)max(r.y - r.x, 0));
+    for (int t0 = threadIdx.x; t0 < G_pad; t0 += kBatch * blockDim.x) {
+        uint32_t len[kBatch];
+        lengths(t0, len);
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const int t = t0 + k * (int)blockDim.x;
+            if (t >= G_pad) break;
+            const int b = t < G ? 32 - __clz(len[k]) : 33;
+            const unsigned peers = __match_any_sync(0xffffffffu, b);
+            const int leader = __ffs(peers) - 1;
+            uint32_t at = 0u;
+            if (b < 33 && lane == leader) at = atomicAdd(&cur[b], (uint32_t)__popc(peers));
+            at = __shfl_sync(0xffffffffu, at, leader);
+            if (b < 33) order[base[b] + at + __popc(peers & lt)] = t;
         }
-        const unsigned peers = __match_any_sync(0xffffffffu, b);
-        const int leader = __ffs(peers) - 1;
-        uint32_t at = 0u;
-        if (b < 33 && lane == leader) at = atomicAdd(&cur[b], (uint32_t)__popc(peers));
-        at = __shfl_sync(0xffffffffu, at, leader);
-        if (b < 33) order[base[b] + at + __popc(peers & lt)] = t;
     }
 }
 
@@ -3003,7 +3049,8 @@ int launch_fwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, cons
     const HitMasks hm = {masks ? w.mask_words : nullptr, w.mask_cap, w.mask_header, nullptr, 0, kNoSegments};
     const Queue q = {w.order, w.info, w.tickets + 0, G, subs, true, hm, tn.status, rm_host::wait_limit(), tn.n_recs};
     auto kernel = blend_fwd_kernel<PX, NT, B, V, LOGT>;
-    constexpr int kPairSmem = (int)sizeof(FwdPairSmem<PX, B>), kWarpSmem = NT / 32 * (int)sizeof(FwdWarpSmem);
+    constexpr int kPairSmem = (int)sizeof(FwdPairSmem<PX, B>),
+                  kWarpSmem = NT / 32 * (int)sizeof(FwdWarpSmem<(V::kViews > 1)>);
     constexpr int smem = kPairSmem > kWarpSmem ? kPairSmem : kWarpSmem;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     const int64_t items = (int64_t)G * subs * (PX == 64 ? 4 : 1);

@@ -156,6 +156,7 @@ __device__ __forceinline__ int tile_w_of(const rm_camera& c) { return c.tile_wid
 // cameras by value in the kernel parameters, so a captured CUDA graph holds
 // its own copy.
 struct OneView {
+    static constexpr int kViews = 1;
     rm_camera cam;
     __device__ __forceinline__ int find(int) const { return 0; }
     __device__ __forceinline__ const rm_camera& camera(int) const { return cam; }
@@ -164,6 +165,7 @@ struct OneView {
 };
 
 struct ViewSet {
+    static constexpr int kViews = RM_MAX_VIEWS;
     int n;
     int tiles[RM_MAX_VIEWS + 1];        // tile_base, with tiles[n] = total tiles
     int64_t pixels[RM_MAX_VIEWS + 1];   // pixel_base, with pixels[n] = total pixels
@@ -305,6 +307,9 @@ __device__ __forceinline__ void async_copy16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// All of this thread's committed groups but the last.
+__device__ __forceinline__ void async_wait_but_last() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
