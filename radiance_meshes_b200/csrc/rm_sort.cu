@@ -7,32 +7,39 @@
 //
 // Design: one histogram kernel computes the digit histograms of every pass in
 // a single read of the keys; then one kernel per 8-bit digit pass.  Each CTA of
-// a pass takes the next 4096-pair tile (dynamic tile id, so predecessors are
-// always running or done), ranks its keys per warp with match.any (warp-striped
-// element order keeps the sort stable), publishes per-digit tile counts and
-// obtains each digit's global offset by decoupled look-back over earlier tiles
-// (bounded spin; a timeout sets RM_STATUS_SORT_TIMEOUT and the CTA proceeds),
-// then scatters through shared memory so each digit run is written coalesced.
+// a pass takes the next tile of 4096 or 6144 pairs (dynamic tile id, so
+// predecessors are always running or done), ranks its keys per warp by the
+// lanes of equal digit (warp-striped element order keeps the sort stable),
+// publishes per-digit tile counts and obtains each digit's global offset by
+// decoupled look-back over earlier tiles (bounded spin; a timeout sets
+// RM_STATUS_SORT_TIMEOUT and the CTA proceeds), then scatters through shared
+// memory so each digit run is written coalesced.
+//
+// The equal digits come from 8 ballots: match.any, whose cost grows with the
+// distinct values in the warp, made a pass over random digits a seventh longer
+// (100M pairs 6830 -> 5930 us).  The look-back has 8 words in flight: one at a
+// time, the walk over the tiles that started together was a serial chain
+// (30k pairs 72 -> 66 us, 100M 5930 -> 5520).
 #include "rm_internal.cuh"
 
 namespace rm {
 namespace {
 
-// Tile shape of a pass (threads x pairs per thread); a build may override it
-// (threads >= 256: one thread per digit).
-#ifndef RM_SORT_THREADS
-#define RM_SORT_THREADS 512
-#endif
-#ifndef RM_SORT_ITEMS
-#define RM_SORT_ITEMS 8
-#endif
-constexpr int kSortThreads = RM_SORT_THREADS;
+// Tile shape of a pass: kSortThreads threads with kSmallItems pairs each, from
+// kLargeFrom pairs on kLargeItems (a digit's run in the output is then half as
+// long again, which is what bounds a pass that fills the GPU; 100M pairs of 48
+// key bits 5540 -> 4880 us, 4M 279 -> 263; but a tile's own chain is longer:
+// 1M 116 -> 126, 30k 70 -> 82).
+constexpr int kSortThreads = 512;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = RM_SORT_ITEMS;
+constexpr int kSmallItems = 8;
+constexpr int kLargeItems = 12;
+constexpr int64_t kLargeFrom = 3 << 20;
 static_assert(kSortThreads >= 256, "one thread per 8-bit digit");
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 pairs per CTA
 constexpr int kRadix = 256;
 constexpr int kMaxPasses = 8;
+// Earlier tiles' words that a look-back has in flight at a time.
+constexpr int kLookBack = 8;
 constexpr uint32_t kLbAgg = 1u << 30;
 constexpr uint32_t kLbInc = 2u << 30;
 constexpr uint32_t kLbMask = (1u << 30) - 1;
@@ -44,7 +51,10 @@ struct SortHeader {
     uint32_t hist[kMaxPasses][kRadix];
 };
 
-__host__ __device__ __forceinline__ int64_t sort_tiles(int64_t n) { return (n + kSortTile - 1) / kSortTile; }
+__host__ __forceinline__ int64_t sort_tiles(int64_t n) {
+    const int64_t tile = (int64_t)kSortThreads * (n < kLargeFrom ? kSmallItems : kLargeItems);
+    return (n + tile - 1) / tile;
+}
 
 __host__ __forceinline__ size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -160,22 +170,25 @@ __global__ void __launch_bounds__(kRadix) hist_scan_kernel(SortHeader* hdr) {
     hdr->hist[p][threadIdx.x] = wpre + inc - v;
 }
 
+template <int ITEMS>
 struct PassSmem {
     uint32_t warp_hist[kSortWarps][kRadix];
     uint32_t tile_off[kRadix];
     uint32_t global_start[kRadix];
     uint32_t scan_tmp[kRadix / 32];
     uint32_t tile;
-    uint64_t keys[kSortTile];
-    uint32_t vals[kSortTile];
+    uint64_t keys[kSortThreads * ITEMS];
+    uint32_t vals[kSortThreads * ITEMS];
 };
 
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads, 1024 / kSortThreads) onesweep_kernel(
     const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
     uint32_t* __restrict__ vout, int64_t cap, const int64_t* __restrict__ n_dev, int pass, int shift,
     uint32_t dmask, SortHeader* hdr, uint32_t* __restrict__ lookback, uint32_t* status, uint32_t spin_limit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PassSmem& S = *reinterpret_cast<PassSmem*>(smem_raw);
+    constexpr int kSortTile = kSortThreads * ITEMS;
+    PassSmem<ITEMS>& S = *reinterpret_cast<PassSmem<ITEMS>*>(smem_raw);
     const int64_t n = n_dev ? min(*n_dev, cap) : cap;
     if (threadIdx.x == 0) S.tile = atomicAdd(&hdr->counters[pass], 1u);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -187,13 +200,13 @@ __global__ void __launch_bounds__(kSortThreads, 1024 / kSortThreads) onesweep_ke
     const int64_t valid_in_tile = min((int64_t)kSortTile, n - tile_base);
     const uint32_t invalid = (uint32_t)(kSortTile - valid_in_tile);
 
-    uint64_t key[kSortItems];
-    uint32_t val[kSortItems];
-    uint32_t dig[kSortItems];
-    uint32_t rank[kSortItems];
-    const int64_t wbase = tile_base + (int64_t)warp * (kSortItems * 32);
+    uint64_t key[ITEMS];
+    uint32_t val[ITEMS];
+    uint32_t dig[ITEMS];
+    uint32_t rank[ITEMS];
+    const int64_t wbase = tile_base + (int64_t)warp * (ITEMS * 32);
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const int64_t idx = wbase + i * 32 + lane;
         const bool valid = idx < n;
         key[i] = valid ? __ldg(kin + idx) : ~0ull;
@@ -202,8 +215,8 @@ __global__ void __launch_bounds__(kSortThreads, 1024 / kSortThreads) onesweep_ke
     }
     const uint32_t lt = lanemask_lt();
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        const uint32_t peers = __match_any_sync(0xffffffffu, dig[i]);
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t peers = warp_peers<8>(dig[i]);
         const uint32_t before = S.warp_hist[warp][dig[i]];
         __syncwarp();
         if ((peers & lt) == 0) S.warp_hist[warp][dig[i]] = before + __popc(peers);
@@ -254,7 +267,7 @@ __global__ void __launch_bounds__(kSortThreads, 1024 / kSortThreads) onesweep_ke
     // the local scatter needs no global offsets: it runs before the look-back,
     // so the other warps' scatter overlaps the digit threads' polling
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const uint32_t lpos = S.tile_off[dig[i]] + S.warp_hist[warp][dig[i]] + rank[i];
         S.keys[lpos] = key[i];
         S.vals[lpos] = val[i];
@@ -264,26 +277,31 @@ __global__ void __launch_bounds__(kSortThreads, 1024 / kSortThreads) onesweep_ke
         uint32_t excl = 0;
         int64_t t = (int64_t)tile - 1;
         uint32_t budget = spin_limit;
-        while (t >= 0) {
-            const uint32_t st = ld_relaxed32(lookback + (size_t)t * kRadix + d);
-            const uint32_t flag = st & ~kLbMask;
-            if (flag == 0) {
-                if (!spin_budget(budget)) {
-                    atomicOr(status, RM_STATUS_SORT_TIMEOUT);
-                    break;
-                }
-                continue;
+        for (bool done = false; !done;) {
+            uint32_t st[kLookBack];
+#pragma unroll
+            for (int k = 0; k < kLookBack; ++k)
+                st[k] = t - k >= 0 ? ld_relaxed32(lookback + (size_t)(t - k) * kRadix + d) : kLbInc;
+            int used = 0;  // words taken: up to the first that is not published or is inclusive
+#pragma unroll
+            for (int k = 0; k < kLookBack; ++k) {
+                if (done || used < k || !(st[k] & ~kLbMask)) continue;
+                excl += st[k] & kLbMask;
+                done = (st[k] & kLbInc) != 0;
+                used = k + 1;
             }
-            excl += st & kLbMask;
-            if (flag == kLbInc) break;
-            --t;
+            t -= used;
+            if (!done && used < kLookBack && !spin_budget(budget)) {
+                atomicOr(status, RM_STATUS_SORT_TIMEOUT);
+                break;
+            }
         }
         st_relaxed32(lookback + (size_t)tile * kRadix + d, kLbInc | ((excl + vcount) & kLbMask));
         S.global_start[d] = excl;
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const int pos = i * kSortThreads + threadIdx.x;
         if (pos < valid_in_tile) {
             const uint64_t k = S.keys[pos];
@@ -331,7 +349,10 @@ int rm_sort_pairs_range(const int64_t* keys_in, const int32_t* values_in, int64_
     uint32_t* alt_v = (uint32_t*)(ws + L.alt_vals_off);
     cudaError_t e = cudaMemsetAsync(ws + 4, 0, L.memset_bytes - 4, s);
     if (e != cudaSuccess) return rm_host::fail(RM_ECUDA, "rm_sort_pairs: %s", cudaGetErrorString(e));
-    e = cudaFuncSetAttribute(onesweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PassSmem));
+    const bool large = n >= kLargeFrom;
+    const auto kernel = large ? onesweep_kernel<kLargeItems> : onesweep_kernel<kSmallItems>;
+    const size_t smem = large ? sizeof(PassSmem<kLargeItems>) : sizeof(PassSmem<kSmallItems>);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return rm_host::fail(RM_ECUDA, "rm_sort_pairs: %s", cudaGetErrorString(e));
     const int64_t tiles = sort_tiles(n);
     const int64_t runs = (n + kHistThreads * kHistRun - 1) / (kHistThreads * kHistRun);
@@ -349,7 +370,7 @@ int rm_sort_pairs_range(const int64_t* keys_in, const int32_t* values_in, int64_
         const int shift = begin_bit + 8 * p;
         const int bits = (end_bit - shift) < 8 ? (end_bit - shift) : 8;
         const uint32_t dmask = (bits >= 8) ? 255u : ((1u << bits) - 1u);
-        onesweep_kernel<<<(unsigned)tiles, kSortThreads, sizeof(PassSmem), s>>>(
+        kernel<<<(unsigned)tiles, kSortThreads, smem, s>>>(
             src_k, src_v, dk, dv, n, n_dev, p, shift, dmask, hdr, lookback + (size_t)p * tiles * kRadix,
             status_dev ? status_dev : &hdr->status, rm_host::wait_limit());
         src_k = dk;
