@@ -118,29 +118,36 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const int32_t* __res
         }
         if (lane < kScanThreads / 32) s_warp[lane] = wi - w;  // exclusive warp offsets
         const int64_t block_total = __shfl_sync(0xffffffffu, wi, kScanThreads / 32 - 1);
-        if (lane == 0) {
-            int64_t prefix = 0;
-            bool ovf = block_total > (int64_t)INT32_MAX || block_total < 0;
-            if (tile != 0) {
-                st_relaxed(&state[tile], kFlagAgg | (ovf ? kFlagOvf : 0ull) | (uint32_t)block_total);
-                int64_t t = (int64_t)tile - 1;
-                uint32_t budget = spin_limit;
-                while (t >= 0) {
-                    const uint64_t s = ld_relaxed(&state[t]);
-                    const uint64_t flag = s & (3ull << 32);
-                    if (flag == 0) {
-                        if (!spin_budget(budget)) {
-                            atomicOr(status, RM_STATUS_SCAN_TIMEOUT);
-                            break;
-                        }
-                        continue;
-                    }
-                    prefix += (int64_t)(uint32_t)s;
-                    ovf |= (s & kFlagOvf) != 0;
-                    if (flag == kFlagInc) break;
-                    --t;
+        int64_t prefix = 0;
+        bool ovf = block_total > (int64_t)INT32_MAX || block_total < 0;
+        if (tile != 0) {
+            if (lane == 0) st_relaxed(&state[tile], kFlagAgg | (ovf ? kFlagOvf : 0ull) | (uint32_t)block_total);
+            int64_t t = (int64_t)tile - 1;
+            uint32_t budget = spin_limit;
+            // The warp reads 32 predecessors at a time: one lane walking over
+            // the tiles that started together was a serial chain (1.3M tets
+            // 16.2 -> 12.3 us).
+            while (t >= 0) {
+                const uint64_t s = t - lane >= 0 ? ld_relaxed(&state[t - lane]) : kFlagInc;
+                const unsigned gap = __ballot_sync(0xffffffffu, (s & (3ull << 32)) == 0);
+                const unsigned inc = __ballot_sync(0xffffffffu, (s & kFlagInc) != 0);
+                const int ready = gap ? __ffs(gap) - 1 : 32;
+                const bool done = inc && __ffs(inc) <= ready;
+                const int take = done ? __ffs(inc) : ready;
+                int64_t part = lane < take ? (int64_t)(uint32_t)s : 0;
+#pragma unroll
+                for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+                prefix += part;
+                ovf |= __any_sync(0xffffffffu, lane < take && (s & kFlagOvf) != 0);
+                if (done) break;
+                t -= take;
+                if (take < 32 && !spin_budget(budget)) {
+                    if (lane == 0) atomicOr(status, RM_STATUS_SCAN_TIMEOUT);
+                    break;
                 }
             }
+        }
+        if (lane == 0) {
             const int64_t tile_incl = prefix + block_total;
             ovf |= tile_incl > (int64_t)INT32_MAX;
             if (ovf) atomicOr(status, RM_STATUS_OVERFLOW);
