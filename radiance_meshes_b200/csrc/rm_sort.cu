@@ -67,11 +67,14 @@ __host__ SortLayout sort_layout(int64_t n, int npasses) {
     SortLayout L;
     const int64_t tiles = sort_tiles(n) > 0 ? sort_tiles(n) : 1;
     L.lookback_off = align_up(sizeof(SortHeader), 256);
-    const size_t lb = sizeof(uint32_t) * (size_t)npasses * (size_t)tiles * kRadix;
+    // room for the small tiles at any n: the size grows with n, so that a
+    // workspace for n pairs holds any fewer
+    const int64_t room = (n + kSortThreads * kSmallItems - 1) / (kSortThreads * kSmallItems);
+    const size_t lb = sizeof(uint32_t) * (size_t)npasses * (size_t)(room > 0 ? room : 1) * kRadix;
     L.alt_keys_off = align_up(L.lookback_off + lb, 256);
     L.alt_vals_off = align_up(L.alt_keys_off + sizeof(uint64_t) * (size_t)(n > 0 ? n : 1), 256);
     L.total = align_up(L.alt_vals_off + sizeof(uint32_t) * (size_t)(n > 0 ? n : 1), 256);
-    L.memset_bytes = L.lookback_off + lb;
+    L.memset_bytes = L.lookback_off + sizeof(uint32_t) * (size_t)npasses * (size_t)tiles * kRadix;
     return L;
 }
 

@@ -286,3 +286,10 @@ def test_fine_list_entry_points_validate():
     # packed bits (no footprint) only for a 2x split
     rc = L.rm_fine_lists_multi(16, 16, 10, None, 16, None, None, 10, cams, 1, 2, 10, 16, 16, 16, 256, ws, None, None)
     assert rc == C.RM_EINVAL and "packed" in C.last_error()
+
+
+def test_sort_workspace_grows_with_size():
+    """A workspace for n pairs holds any fewer, across the change of tile size."""
+    size = C.lib().rm_sort_workspace_size
+    sizes = [size(n) for n in range(0, 8 << 20, 65_521)] + [size(1 << 29)]
+    assert all(a <= b for a, b in zip(sizes, sizes[1:]))
