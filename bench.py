@@ -55,7 +55,7 @@ def parse():
                     help="how the backward stages tet records in shared memory: per-thread loads, or bulk copies "
                          "(cp.async.bulk, two batches in flight); bulk copies only in single-GPU runs")
     ap.add_argument("--pair-ctas", type=int, default=0,
-                    help="resident CTAs per SM of the forward's pair kernel (0: the library default)")
+                    help="resident CTAs per SM of the forward (0: the library default)")
     ap.add_argument("--bwd-batch", type=int, default=0, choices=[0, 16, 32, 64],
                     help="tets per shared-memory batch of the backward (0: the library default)")
     ap.add_argument("--profile-steps", type=int, default=0, help="(profiling) run N steps after warmup, print nothing")
@@ -202,7 +202,7 @@ def issue_roofline(kernel, launch_ms, tests, clocks, **extra):
         if not model:
             return out
         warp_inst = tests * model["thread_instructions_per_test"] / model["active_lanes_per_instruction"]
-        src = "profiles/issue_model.json (instructions per test of the 50k-point capture)"
+        src = "profiles/issue_model.json (instructions per test of a capture)"
     achieved = warp_inst / (launch_ms * 1e-3) / 1e9
     peak = sms * 4 * mhz * 1e6 / 1e9
     out.update({"bound": "issue", "unit": "G warp instructions/s", "achieved": achieved, "peak": peak,
