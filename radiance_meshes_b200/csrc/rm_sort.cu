@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(kSortThreads, 1024 / kSortThreads) onesweep_ke
     // their end); the next pass may be set up once every CTA is here.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("" : "+l"(n_dev));  // its load, of a read-only parameter, must not move up past the wait
     const int64_t n = n_dev ? min(*n_dev, cap) : cap;
     if (threadIdx.x == 0) S.tile = atomicAdd(&hdr->counters[pass], 1u);
     __syncthreads();
