@@ -2404,7 +2404,8 @@ __device__ __forceinline__ void bwd_pair_item(
 constexpr int kBwdWarpsPerSm = 20;
 
 template <int PX, class V>
-__global__ void __launch_bounds__(PX < 32 ? 32 : PX, PX < 32 ? kBwdWarpsPerSm : kBwdWarpsPerSm * 32 / PX) blend_bwd_kernel(
+__global__ void __launch_bounds__(PX < 32 ? 32 : PX, PX < 32 ? kBwdWarpsPerSm : kBwdWarpsPerSm * 32 / PX)
+    blend_bwd_kernel(
     const int32_t* __restrict__ ids, const int2* __restrict__ ranges, const float4* __restrict__ recs,
     const int4* __restrict__ indices, const float2* __restrict__ jitter, const __grid_constant__ V views,
     const float4* __restrict__ img, const float* __restrict__ dist, const int32_t* __restrict__ ncs,
