@@ -314,6 +314,9 @@ RM_API size_t rm_blend_status_offset(int64_t n_tets, int64_t n_tiles);
  * from this GPU's memory into the issuing CTA, completing on an mbarrier), two
  * batches in flight, instead of per-thread loads.  Backward, 64-pixel items. */
 #define RM_BLEND_STAGE_TMA 0x4
+/* rm_calc_tet_err: the workspace beyond rm_blend_workspace_size holds no masks
+ * that a backward still needs, so the call may use it. */
+#define RM_BLEND_OWN_SCRATCH 0x8
 
 /* flags bits 8..15: log2 of the pixels per work item strip (16 or 64; 0 = 64) */
 #define RM_BLEND_STRIP_SHIFT 8
@@ -584,10 +587,12 @@ RM_API int rm_blend_bwd_multi(const int32_t* sorted_ids, const int32_t* ranges,
  * and the maximum of int(65535 * T).  Columns 3 and 4 are left untouched, as
  * in the reference, whose walk also starts from log T = 1 and stops once
  * log T < -5.5.  Workspace and flags as rm_blend_fwd (records are packed
- * unless RM_BLEND_REUSE_RECORDS).  A workspace with rm_blend_hit_mask_bytes and
- * 4 bytes per pixel (and 512) beyond rm_blend_workspace_size lets long lists be
- * taken in stretches (64-pixel strips): the same counts and maxima, several
- * times faster where a few lists are long.
+ * unless RM_BLEND_REUSE_RECORDS); a forward's hit masks in it are kept.  With
+ * RM_BLEND_OWN_SCRATCH (64-pixel strips) and a workspace of
+ * rm_blend_hit_mask_bytes and 4 bytes per pixel (and 512) beyond
+ * rm_blend_workspace_size, long lists are taken in stretches: the same counts
+ * and maxima, several times faster where a few lists are long; masks that a
+ * forward left there are then lost, and a backward tests every entry.
  */
 RM_API int rm_calc_tet_err(const int32_t* sorted_ids, const int32_t* ranges,
                            const int32_t* indices, const float* vertices,

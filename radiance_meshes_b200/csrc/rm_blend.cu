@@ -342,6 +342,7 @@ struct HitMasks {
 };
 
 constexpr uint32_t kMaskValid = 0x6d61736bu;
+constexpr uint32_t kMaskStats = 0x73746174u;  // written by the statistics' walk, of no use to a backward
 constexpr int kNoSegments = 31;   // seg_shift of a pass without checkpoints
 constexpr int kMinSegShift = 7;   // segments are whole batches (<= 64 entries) and whole mask blocks
 constexpr int kCkFloats = 6;
@@ -363,21 +364,22 @@ __device__ __forceinline__ float* ck_at(const HitMasks& hm, int64_t id, int sub,
 }
 
 // Header words of a pass with hit masks, written by the forward's order
-// kernel: [0] kMaskValid, [1] seg_shift, [2] checkpoint ids, [4..5] offset of
+// kernel: [0] kMaskValid (kMaskStats in the statistics), [1] seg_shift, [2] checkpoint ids, [4..5] offset of
 // the checkpoints in words after the mask words' start.
 struct MaskHeader {
     uint32_t state, seg_shift, ck_cap, pad;
     int64_t ck_off;
 };
 
-// The masks a kernel may use: none unless the header says the forward wrote
-// them.  hm.cap is the room in words for masks and checkpoints together.
-__device__ __forceinline__ HitMasks live_masks(HitMasks hm, int subs) {
+// The masks a kernel may use: none unless the header says that a walk of its
+// own kind wrote them.  hm.cap is the room in words for masks and checkpoints
+// together.
+__device__ __forceinline__ HitMasks live_masks(HitMasks hm, int subs, uint32_t state = kMaskValid) {
     hm.ck = nullptr;
     hm.ck_cap = 0;
     hm.seg_shift = kNoSegments;
     if (!hm.words) return hm;
-    if (!hm.header || __ldcg(hm.header) != kMaskValid) {
+    if (!hm.header || __ldcg(hm.header) != state) {
         hm.words = nullptr;
         return hm;
     }
@@ -1153,7 +1155,8 @@ __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
     const int nq = PX == 64 ? __ldg(q.info + 1) : 0;
     const int q_items = nq * q.subs * 4;
     const int n_items = q_items + (__ldg(q.info) - nq) * q.subs;
-    if (threadIdx.x == 0) hm = live_masks(q.hm, q.subs);  // seen after next_item's barriers
+    if (threadIdx.x == 0)
+        hm = live_masks(q.hm, q.subs, LOGT ? kMaskStats : kMaskValid);  // seen after next_item's barriers
     for (;;) {
         int item = next_item(q, &s_item);
         if (item >= n_items) break;
@@ -1271,7 +1274,7 @@ __global__ void __cluster_dims__(kOrderCtas, 1, 1) __launch_bounds__(1024)
         // segments per bucket of the masks' segment length (segment_item)
         int shift = kNoSegments;
         if (seg_header && __ldcg(seg_header) == kMaskValid) shift = (int)__ldcg(seg_header + 1);
-        if (mask_header && mh.state == kMaskValid) shift = (int)mh.seg_shift;
+        if (mask_header && mh.state != 0u) shift = (int)mh.seg_shift;
         if (shift >= kMinSegShift && shift < kNoSegments) {
             uint32_t at = 0;
             for (int b = 32; b > shift; --b) {
@@ -2812,7 +2815,7 @@ __global__ void __launch_bounds__(64, 12) err_seg_kernel(const int32_t* __restri
                                                          const Queue q) {
     __shared__ ErrSegSmem S;
     __shared__ HitMasks hm;
-    if (threadIdx.x == 0) hm = live_masks(q.hm, q.subs);
+    if (threadIdx.x == 0) hm = live_masks(q.hm, q.subs, kMaskStats);
     __syncthreads();
     const int64_t n_items = segment_items(q.info, q.G, hm.seg_shift) * q.subs;
     for (;;) {
@@ -3061,9 +3064,11 @@ int launch_fwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, cons
     const bool masks = tn.hit_masks && PX == 64 && w.mask_header;
     const int subs = sh.tile_px / PX;
     const int cap = tn.pair_ctas_per_sm * sm_count();
+    MaskHeader mh = {};
+    if (masks) mh = mask_header_for(w.mask_cap, G, subs);
+    if (masks && LOGT) mh.state = kMaskStats;
     int rc = launch_order(ranges, G, w, PX == 64 ? tn.heavy_shift : tn.heavy_shift == 0 ? 1 : tn.heavy_shift, s,
-                          w.mask_header, masks ? mask_header_for(w.mask_cap, G, subs) : MaskHeader{}, nullptr,
-                          PX == 64 ? (cap > subs ? cap / subs : 1) : 0);
+                          w.mask_header, mh, nullptr, PX == 64 ? (cap > subs ? cap / subs : 1) : 0);
     if (rc) return rc;
     const HitMasks hm = {masks ? w.mask_words : nullptr, w.mask_cap, w.mask_header, nullptr, 0, kNoSegments};
     const Queue q = {w.order, w.info, w.tickets + 0, G, subs, true, hm, tn.status, rm_host::wait_limit(), tn.n_recs};
@@ -3331,10 +3336,11 @@ int rm_calc_tet_err(const int32_t* sorted_ids, const int32_t* ranges, const int3
     }
     const int strip = strip_pixels(cam, flags);
     const int subs = cam->tile_width * cam->tile_height / strip;
-    // with room for hit masks and n_contributors: the forward's walk, then the
-    // statistics by stretches
+    // with room for hit masks and n_contributors that is the call's own: the
+    // forward's walk, then the statistics by stretches.  Otherwise that part of
+    // the workspace is left as it is: a backward may still need its masks.
     const size_t nc_bytes = (size_t)cam->image_height * cam->image_width * sizeof(int32_t);
-    if (strip == 64 && workspace_bytes > blend_ws_bytes(n_tets, G) + nc_bytes + 512) {
+    if ((flags & RM_BLEND_OWN_SCRATCH) && strip == 64 && workspace_bytes > blend_ws_bytes(n_tets, G) + nc_bytes + 512) {
         const size_t nc_off = (workspace_bytes - nc_bytes) / 256 * 256;
         const BlendWs wm = blend_ws(workspace, n_tets, G, nc_off);
         if (wm.mask_header && mask_header_for(wm.mask_cap, G, subs).seg_shift < (uint32_t)kNoSegments) {

@@ -718,7 +718,7 @@ def calc_tet_err(sorted_ids, ranges, indices, vertices, cell_values, cam: RMCame
     _call("rm_calc_tet_err", lambda: L.rm_calc_tet_err(
         C.ptr(sorted_ids), C.ptr(ranges), C.ptr(indices), C.ptr(vertices), C.ptr(cell_values), T, vertices.shape[0],
         C.ptr(tiles_touched), ctypes.byref(cam), C.ptr(pixel_err), C.ptr(ssim_err), C.ptr(tet_err),
-        C.ptr(tet_count), C.ptr(ws), ws.numel(), 0, _stream()))
+        C.ptr(tet_count), C.ptr(ws), ws.numel(), C.RM_BLEND_OWN_SCRATCH, _stream()))
     return tet_err, tet_count
 
 

@@ -1,0 +1,67 @@
+"""What the forward leaves in its workspace for the backward (hit masks and
+checkpoints), whichever kind of work item wrote it and whatever else ran on
+the workspace in between."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import run_gpu_forward, to_dev
+from radiance_meshes_b200 import _capi as C
+from radiance_meshes_b200 import rasterizer as R
+from radiance_meshes_b200.camera import pinhole_tcam
+from test_gpu_long_lists import _stack
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(n, density, tile=8, H=21, W=18, small=0.0):
+    verts, idx, cv = _stack(n, density, n, small)
+    tcam = pinhole_tcam((0.1, 0.0, 0.0), (0.0, 0.0, 1.0), H, W, 30.0, tile_size=tile)
+    jitter = np.random.default_rng(n).uniform(0, 1, (H, W, 2)).astype(np.float32)
+    r = run_gpu_forward(verts, idx, cv, tcam, jitter, keep_debug=False, hit_masks=True)
+    g = torch.Generator("cuda").manual_seed(n)
+    r["gimg"] = torch.randn(H, W, 4, device="cuda", generator=g)
+    r["gdist"] = 1e-3 * torch.randn(H, W, 5, device="cuda", generator=g)
+    return r
+
+
+def _bwd(r, records, hit_masks):
+    L = r["lists"]
+    out = R.blend_bwd(L.sorted_ids, L.ranges, r["i"], r["v"], r["c"], r["j"], r["cam"], r["img"], r["dist"], r["nc"],
+                      r["gimg"], r["gdist"], records, hit_masks=hit_masks)
+    torch.cuda.synchronize()
+    return out
+
+
+def _same(a, b):
+    """Equal but for the order of the sums."""
+    for x, y in zip(a, b):
+        assert torch.isfinite(x).all()
+        assert float((x - y).norm()) <= 1e-5 * float(y.norm())
+
+
+@pytest.mark.parametrize("n,density", [(33, 0.3), (400, 0.3), (400, 6.0)])
+@pytest.mark.parametrize("own", [False, True])
+def test_statistics_keep_the_forwards_masks(cuda, n, density, own):
+    """rm_blend_fwd, rm_calc_tet_err and rm_blend_bwd on one workspace, with
+    the same flags: the statistics leave the forward's masks as they are.
+    Allowed to overwrite them, they leave none that a backward would take."""
+    r = _scene(n, density)
+    L, cam = r["lists"], r["cam"]
+    whole = _bwd(r, r["records"], False)
+    before = r["records"].clone()
+    rng = np.random.default_rng(n)
+    pe, se = (to_dev(rng.uniform(0, 1, (cam.image_height, cam.image_width)).astype(np.float32)) for _ in range(2))
+    err = torch.zeros(n, 16, device="cuda")
+    cnt = torch.zeros(n, 2, dtype=torch.int32, device="cuda")
+    C.check(C.lib().rm_calc_tet_err(
+        C.ptr(L.sorted_ids), C.ptr(L.ranges), C.ptr(r["i"]), C.ptr(r["v"]), C.ptr(r["c"]), n, r["v"].shape[0], None,
+        ctypes.byref(cam), C.ptr(pe), C.ptr(se), C.ptr(err), C.ptr(cnt), C.ptr(r["records"]), r["records"].numel(),
+        C.RM_BLEND_REUSE_RECORDS | C.RM_BLEND_HIT_MASKS | (C.RM_BLEND_OWN_SCRATCH if own else 0),
+        C.stream_handle()), "rm_calc_tet_err")
+    assert int(cnt[:, 0].sum()) > 0
+    base = C.lib().rm_blend_workspace_size(n, cam.grid_width * cam.grid_height)
+    assert own or torch.equal(r["records"][base:], before[base:])
+    _same(_bwd(r, r["records"], True), whole)
