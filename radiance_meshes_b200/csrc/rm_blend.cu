@@ -790,7 +790,7 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
     using Sh = PairShape<PX, NT, B>;
     static_assert(PX <= 64 && NT >= 64, "two owner warps at most");
     static_assert(Sh::kStageWarps >= 1 && Sh::kStageWarps <= FwdPairSmem<PX, B>::kMaxStage, "staging warps");
-    constexpr bool kMasks = PX == 64 && B % 32 == 0;
+    constexpr bool kMasks = PX == 64;
     constexpr int RB = Sh::RB;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool own_warp = warp < Sh::kOwnWarps;
@@ -974,8 +974,11 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
                     }
                 }
                 if (kMasks && owner && hm.words) {
-                    const int64_t i = mask_word(gtile, rg.x, blk + w, sub, subs, p);
-                    if (i < hm.cap) __stcg(hm.words + i, hb);
+                    const int64_t i = mask_word(gtile, rg.x, (blk + w) * RB >> 5, sub, subs, p);
+                    if (i < hm.cap) {
+                        if (RB == 32) __stcg(hm.words + i, hb);
+                        else __stcg((unsigned short*)(hm.words + i) + ((blk + w) & 1), (unsigned short)hb);
+                    }
                 }
             }
             if (__any_sync(0xffffffffu, was != active))

@@ -65,3 +65,26 @@ def test_statistics_keep_the_forwards_masks(cuda, n, density, own):
     base = C.lib().rm_blend_workspace_size(n, cam.grid_width * cam.grid_height)
     assert own or torch.equal(r["records"][base:], before[base:])
     _same(_bwd(r, r["records"], True), whole)
+
+
+@pytest.mark.parametrize("batch", [16, 32, 64])
+@pytest.mark.parametrize("heavy", [0, 1, 15])  # by the lists' lengths, every tile by pair items, by warp items
+@pytest.mark.parametrize("n,density", [(33, 0.3), (400, 0.3), (400, 6.0)])
+def test_masks_of_every_batch_and_route(cuda, batch, heavy, n, density):
+    """Each kind of forward item, with each batch size, leaves masks and
+    checkpoints that give the gradients of a backward that tests every entry.
+    The pair items of batches of 16 write half a mask word a block.
+    (The workspace starts out zeroed: a mask that is not written loses hits.)"""
+    r = _scene(n, density)
+    whole = _bwd(r, r["records"], False)
+    L = r["lists"]
+    ws = torch.zeros_like(r["records"])
+    old = R.blend_tuning()
+    R.set_blend_tuning((heavy << C.RM_BLEND_HEAVY_SHIFT) | ({16: 4, 32: 5, 64: 6}[batch] << C.RM_BLEND_BATCH_SHIFT), 0)
+    try:
+        img, dist, nc, _ = R.blend_fwd(L.sorted_ids, L.ranges, r["i"], r["v"], r["c"], r["j"], r["cam"],
+                                       tiles_touched=r["tiles"], records=ws, hit_masks=True)
+    finally:
+        R.set_blend_tuning(*old)
+    assert torch.equal(img, r["img"]) and torch.equal(dist, r["dist"]) and torch.equal(nc, r["nc"])
+    _same(_bwd(r, ws, True), whole)
