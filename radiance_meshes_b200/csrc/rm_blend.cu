@@ -623,6 +623,14 @@ __device__ __forceinline__ bool entry_reaches(const float4* __restrict__ r, cons
     return reach;
 }
 
+// A ray's z (d.r2) as its bundle takes it: 0, for which entry_reaches does not
+// apply, where the ray has no place in the box.  Such a ray (a jitter or a
+// direction that is not a number) counts as a hit of every entry of positive
+// density, which the other rays of the bundle must not drop.
+__device__ __forceinline__ float bundle_z(float z, float u, float v) {
+    return fabsf(u) < 1e30f && fabsf(v) < 1e30f ? z : 0.f;
+}
+
 // 1 / (least z) of a bundle, or 0 when entry_reaches does not apply (rays
 // starting behind the camera position, axes that are no rotation, rays far
 // off the axis).
@@ -840,8 +848,10 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
             const float2 j = LOGT ? make_float2(0.5f, 0.5f) : __ldg(jitter + pix);
             make_ray(cam, px, py, j.x, j.y, o, d);
             z = dot3(mk3(M[8], M[9], M[10]), d);
-            S.uv[0][tid] = dot3(mk3(M[0], M[1], M[2]), d) / z;
-            S.uv[1][tid] = dot3(mk3(M[4], M[5], M[6]), d) / z;
+            const float u = dot3(mk3(M[0], M[1], M[2]), d) / z, v = dot3(mk3(M[4], M[5], M[6]), d) / z;
+            S.uv[0][tid] = u;
+            S.uv[1][tid] = v;
+            z = bundle_z(z, u, v);
             S.ray[0][tid] = o.x; S.ray[1][tid] = o.y; S.ray[2][tid] = o.z;
             S.ray[3][tid] = d.x; S.ray[4][tid] = d.y; S.ray[5][tid] = d.z;
         }
@@ -1047,6 +1057,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
         z = dot3(mk3(M[8], M[9], M[10]), d);
         u = dot3(mk3(M[0], M[1], M[2]), d) / z;
         v = dot3(mk3(M[4], M[5], M[6]), d) / z;
+        z = bundle_z(z, u, v);
     }
 #pragma unroll
     for (int off = 16; off; off >>= 1) z = fminf(z, __shfl_xor_sync(0xffffffffu, z, off));

@@ -88,3 +88,34 @@ def test_masks_of_every_batch_and_route(cuda, batch, heavy, n, density):
         R.set_blend_tuning(*old)
     assert torch.equal(img, r["img"]) and torch.equal(dist, r["dist"]) and torch.equal(nc, r["nc"])
     _same(_bwd(r, ws, True), whole)
+
+
+@pytest.mark.parametrize("tile,heavy", [(4, 0), (8, 1), (8, 15), (16, 0)])
+@pytest.mark.parametrize("positive", [1, 5])
+def test_nan_ray_ends_at_the_first_entry_it_meets(cuda, tile, heavy, positive):
+    """A ray that is not a number counts as a hit of every entry with a
+    positive density, whatever the other rays of its strip see; only its own
+    pixel shows it."""
+    n, size = 160, 32
+    verts, idx, cv = _stack(n, 0.3, n, 1.0)
+    cv[np.arange(n) % positive != 0, 0] = 0.0
+    tcam = pinhole_tcam((0.1, 0.0, 0.0), (0.0, 0.0, 1.0), size, size, 30.0, tile_size=tile)
+    jitter = np.random.default_rng(n).uniform(0, 1, (size, size, 2)).astype(np.float32)
+    bad = np.zeros((size, size), bool)
+    bad[3::16, 5::8] = True
+    old = R.blend_tuning()
+    R.set_blend_tuning(heavy << C.RM_BLEND_HEAVY_SHIFT, 0)
+    try:
+        clean = run_gpu_forward(verts, idx, cv, tcam, jitter, keep_debug=False)
+        jitter[bad] = np.nan
+        r = run_gpu_forward(verts, idx, cv, tcam, jitter, keep_debug=False)
+    finally:
+        R.set_blend_tuning(*old)
+    ids, ranges = r["lists"].sorted_ids.cpu().numpy(), r["lists"].ranges.cpu().numpy()
+    nc = r["nc"].cpu().numpy()[..., 0]
+    for y, x in zip(*np.nonzero(bad)):
+        x0, x1 = ranges[(y // tile) * (size // tile) + x // tile]
+        hit = np.flatnonzero(cv[ids[x0:x1], 0] > 0)
+        assert nc[y, x] == (hit[0] + 1 if len(hit) else x1 - x0)
+    ok = torch.from_numpy(~bad).cuda()
+    assert torch.equal(r["nc"][ok], clean["nc"][ok]) and torch.equal(r["img"][ok], clean["img"][ok])
