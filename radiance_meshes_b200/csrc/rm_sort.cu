@@ -196,10 +196,12 @@ struct PassSmem {
     uint32_t vals[kSortThreads * ITEMS];
 };
 
+// A pass may be resident while the pass before it still writes kin and vin, so
+// these are read past the read-only path (which asks for memory that nobody
+// writes during the kernel's lifetime); every pair is read once.
 template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads, 1024 / kSortThreads) onesweep_kernel(
-    const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
-    uint32_t* __restrict__ vout, int64_t cap, const int64_t* __restrict__ n_dev, int pass, int shift,
+    const uint64_t* kin, const uint32_t* vin, uint64_t* kout, uint32_t* vout, int64_t cap, const int64_t* __restrict__ n_dev, int pass, int shift,
     uint32_t dmask, SortHeader* hdr, uint32_t* __restrict__ lookback, uint32_t* status, uint32_t spin_limit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int kSortTile = kSortThreads * ITEMS;
@@ -229,8 +231,8 @@ __global__ void __launch_bounds__(kSortThreads, 1024 / kSortThreads) onesweep_ke
     for (int i = 0; i < ITEMS; ++i) {
         const int64_t idx = wbase + i * 32 + lane;
         const bool valid = idx < n;
-        key[i] = valid ? __ldg(kin + idx) : ~0ull;
-        val[i] = valid ? __ldg(vin + idx) : 0u;
+        key[i] = valid ? __ldcg(kin + idx) : ~0ull;
+        val[i] = valid ? __ldcg(vin + idx) : 0u;
         dig[i] = valid ? ((uint32_t)(key[i] >> shift) & dmask) : 255u;
     }
     const uint32_t lt = lanemask_lt();

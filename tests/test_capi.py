@@ -293,3 +293,15 @@ def test_sort_workspace_grows_with_size():
     size = C.lib().rm_sort_workspace_size
     sizes = [size(n) for n in range(0, 8 << 20, 65_521)] + [size(1 << 29)]
     assert all(a <= b for a, b in zip(sizes, sizes[1:]))
+
+
+def test_overlapped_sort_passes_read_past_the_read_only_path():
+    """A sort pass is launched over the end of the pass that writes its input:
+    nothing may let the compiler read that input through the read-only path."""
+    src = open(os.path.join(os.path.dirname(C.__file__), "csrc", "rm_sort.cu")).read()
+    kernel = src[src.index("onesweep_kernel("):src.index("extern \"C\"")]
+    params = kernel[:kernel.index("{")]
+    assert "griddepcontrol.wait" in kernel
+    for name in ("kin", "vin", "kout", "vout"):
+        assert re.search(rf"\* {name}\b", params), name  # no __restrict__
+        assert f"__ldg({name}" not in kernel
