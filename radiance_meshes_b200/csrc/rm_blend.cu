@@ -309,6 +309,7 @@ struct PixelState {
     float c[3];
     float logT;
     float D[5];
+    float part[5];  // what the hits since the last checkpoint added to the colour, D2 and D3
 };
 
 // ------------------------------------------------------------------ forward --
@@ -345,17 +346,22 @@ constexpr uint32_t kMaskValid = 0x6d61736bu;
 constexpr uint32_t kMaskStats = 0x73746174u;  // written by the statistics' walk, of no use to a backward
 constexpr int kNoSegments = 31;   // seg_shift of a pass without checkpoints
 constexpr int kMinSegShift = 7;   // segments are whole batches (<= 64 entries) and whole mask blocks
-constexpr int kCkFloats = 6;
+constexpr int kCkFloats = 8;
 
 // Checkpoints.  A pixel that is still active at list offset k << seg_shift
-// (k >= 1) of a tile's list stores the state it has there: log T, the
-// distortion moments D2 and D3 and the colour.  The backward pass then takes
-// each stretch of 1 << seg_shift entries as a work item of its own, starting
-// from the checkpoint at its end: the undo chains start from log T, D2 and D3
-// there, and what the later entries contribute to the adjoint state is a
-// difference of the final and the stored prefix sums (seed_segment).  Without
-// them the pixel with the longest walk bounds the launch: alone on the GPU
-// the 14,506-entry tile of a 1.3M-tet frame takes 1.74 ms, of 2.57 ms in all.
+// (k >= 1) of a tile's list stores log T, D2 and D3 as they are there, and,
+// once its walk has ended, the sums of what the entries from there on added to
+// its colour, D2 and D3.  The backward pass then takes each stretch of
+// 1 << seg_shift entries as a work item of its own, starting from the
+// checkpoint at its end: the undo chains start from log T, D2 and D3 there, and
+// what the later entries contribute to the adjoint state follows from the sums
+// (seed_segment).  These are added up from the last stretch back, each
+// stretch's own sum started at zero: a difference of the final and the earlier
+// colour would hold the rounding of the whole colour, however little is left
+// to come.  Without
+// checkpoints the pixel with the longest walk bounds the launch: alone on the
+// GPU the 14,506-entry tile of a 1.3M-tet frame takes 1.74 ms, of 2.57 ms in
+// all.
 // Ids floor(x / S) + k are distinct over the tiles because the lists do not
 // overlap and offsets k * S lie inside them.
 __device__ __forceinline__ int64_t ck_id(int x, int k, int shift) { return (int64_t)(x >> shift) + k; }
@@ -486,8 +492,9 @@ __device__ __forceinline__ float4 record_part(const float4* __restrict__ recs, i
 }
 
 // Stores the checkpoint of pixel p (p of the strip's 64) at list position
-// base, when one lies there.
-__device__ __forceinline__ void write_checkpoint(const HitMasks& hm, const PixelState& st, int x, int base, int sub,
+// base, when one lies there, with the sums of the stretch before it.
+template <bool LOGT>
+__device__ __forceinline__ void write_checkpoint(const HitMasks& hm, PixelState& st, int x, int base, int sub,
                                                  int subs, int p) {
     const int off = base - x;
     if (off == 0 || (off & ((1 << kMinSegShift) - 1))) return;  // no segment length has one here
@@ -496,11 +503,46 @@ __device__ __forceinline__ void write_checkpoint(const HitMasks& hm, const Pixel
     if (id >= hm.ck_cap) return;
     float* c = ck_at(hm, id, sub, subs, p);
     c[0 * 64] = st.logT;
+    if (LOGT) return;
     c[1 * 64] = st.D[2];
     c[2 * 64] = st.D[3];
-    c[3 * 64] = st.c[0];
-    c[4 * 64] = st.c[1];
-    c[5 * 64] = st.c[2];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        c[(3 + i) * 64] = st.part[i];
+        st.part[i] = 0.f;
+    }
+}
+
+// The sums of the stretches before the checkpoints of a pixel whose walk took
+// nc entries turned into the sums over all of its later entries, from the last
+// checkpoint (st.part: the sums after it) back.
+__device__ __forceinline__ void finish_checkpoints(const HitMasks& hm, const PixelState& st, int x, int nc, int sub,
+                                                   int subs, int p) {
+    if (!hm.ck || nc <= (1 << hm.seg_shift)) return;
+    int k = (nc - 1) >> hm.seg_shift;
+    const int64_t first = ck_id(x, 0, hm.seg_shift);
+    if (first + k >= hm.ck_cap) return;  // not all of them were stored: no pass starts from them
+    const int64_t step = (int64_t)subs * kCkFloats * 64;
+    float* c = ck_at(hm, first + k, sub, subs, p) + 3 * 64;
+    float later[5];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) later[i] = st.part[i];
+    constexpr int kAhead = 4;  // checkpoints read at a time
+    for (; k > 0; k -= kAhead) {
+        float before[kAhead][5];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+#pragma unroll
+            for (int i = 0; i < 5; ++i) before[j][i] = j < k ? c[-j * step + i * 64] : 0.f;
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+#pragma unroll
+            for (int i = 0; i < 5; ++i) {
+                if (j < k) c[-j * step + i * 64] = later[i];
+                later[i] = later[i] + before[j][i];
+            }
+        c -= kAhead * step;
+    }
 }
 
 // One hit folded into the pixel state (update_alpha_out,
@@ -509,7 +551,10 @@ __device__ __forceinline__ void write_checkpoint(const HitMasks& hm, const Pixel
 __device__ __forceinline__ void fold_hit(PixelState& st, float a, float m0, float m1, float d4, const float* rgb) {
     const float T = exp_approx(st.logT);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) st.c[k] = fmaf(rgb[k], T, st.c[k]);
+    for (int k = 0; k < 3; ++k) {
+        st.c[k] = fmaf(rgb[k], T, st.c[k]);
+        st.part[k] = fmaf(rgb[k], T, st.part[k]);
+    }
     st.logT = st.logT - a;
     const float D2 = st.D[2], D3 = st.D[3];
     st.D[0] = fmaf(2.0f * m1, D2, st.D[0]);
@@ -517,6 +562,8 @@ __device__ __forceinline__ void fold_hit(PixelState& st, float a, float m0, floa
     st.D[2] = D2 + m0;
     st.D[3] = D3 + m1;
     st.D[4] = st.D[4] + d4;
+    st.part[3] = st.part[3] + m0;
+    st.part[4] = st.part[4] + m1;
 }
 
 // Result of testing one ray against one list entry, in the exact arithmetic of
@@ -779,6 +826,9 @@ __device__ __forceinline__ void fold_any(PixelState& st, float a, float m0, floa
     st.c[0] = fmaf(r, T, st.c[0]);
     st.c[1] = fmaf(g, T, st.c[1]);
     st.c[2] = fmaf(b, T, st.c[2]);
+    st.part[0] = fmaf(r, T, st.part[0]);
+    st.part[1] = fmaf(g, T, st.part[1]);
+    st.part[2] = fmaf(b, T, st.part[2]);
     st.logT = st.logT - a;
     const float D2 = st.D[2], D3 = st.D[3];
     st.D[0] = fmaf(2.0f * m1, D2, st.D[0]);
@@ -786,6 +836,8 @@ __device__ __forceinline__ void fold_any(PixelState& st, float a, float m0, floa
     st.D[2] = D2 + m0;
     st.D[3] = D3 + m1;
     st.D[4] = st.D[4] + d4;
+    st.part[3] = st.part[3] + m0;
+    st.part[4] = st.part[4] + m1;
 }
 
 template <int PX, int NT, int B, bool LOGT>
@@ -812,7 +864,7 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
     const int px = tx * cam.tile_width + lx, py = ty * cam.tile_height + ly;
     const bool inside = owner && px < cam.image_width && py < cam.image_height;
     const int64_t pix = (int64_t)py * cam.image_width + px;
-    PixelState st = {{0.f, 0.f, 0.f}, LOGT ? 1.0f : 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}};
+    PixelState st = {{0.f, 0.f, 0.f}, LOGT ? 1.0f : 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f, 0.f}};
     int32_t nc = rg.y - rg.x;  // entries walked: all of them unless log T runs out
     bool active = inside && nc > 0;
     int rank = 0, slot = tid;  // rank among the warp's active pixels; where the pixel's ray and results lie
@@ -933,7 +985,7 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
             for (int w = 0; w < m; ++w) {
                 const int j1 = S.start[cur][w + 1];
                 uint32_t hb = 0;  // bit k: entry k of the block was a hit for this owner's pixel
-                if (kMasks && active) write_checkpoint(hm, st, rg.x, rg.x + (blk + w) * RB, sub, subs, p);
+                if (kMasks && active) write_checkpoint<LOGT>(hm, st, rg.x, rg.x + (blk + w) * RB, sub, subs, p);
                 for (int j = S.start[cur][w]; LOGT && j < j1 && active; ++j) {
                     const float a = S.res[0][j][slot];
                     st.logT = st.logT - a;
@@ -1004,6 +1056,7 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
     if (inside) {
         out_nc[pix] = nc;
         if (LOGT) return;
+        if (kMasks) finish_checkpoints(hm, st, rg.x, nc, sub, subs, p);
         out_img[pix] = make_float4(st.c[0], st.c[1], st.c[2], st.logT);
         float* dd = out_dist + 5 * pix;
 #pragma unroll
@@ -1072,7 +1125,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
                   fminf(bd.v0, __shfl_xor_sync(0xffffffffu, bd.v0, off)),
                   fmaxf(bd.v1, __shfl_xor_sync(0xffffffffu, bd.v1, off))};
     };
-    PixelState st = {{0.f, 0.f, 0.f}, LOGT ? 1.0f : 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}};
+    PixelState st = {{0.f, 0.f, 0.f}, LOGT ? 1.0f : 0.f, {0.f, 0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f, 0.f}};
     int32_t nc = rg.y - rg.x;  // entries walked: all of them unless log T runs out
     bool active = inside && nc > 0;
     bounds(active);
@@ -1091,7 +1144,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
     if (AHEAD && __any_sync(0xffffffffu, active)) fetch(0, g);
     int buf = 0;
     for (int base = rg.x; base < rg.y && __any_sync(0xffffffffu, active); base += 32) {
-        if (PX == 64 && active) write_checkpoint(hm, st, rg.x, base, sub, subs, p);
+        if (PX == 64 && active) write_checkpoint<LOGT>(hm, st, rg.x, base, sub, subs, p);
         const bool valid = g >= 0;
         if (AHEAD) {
             g = g_ahead;
@@ -1144,6 +1197,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
     if (inside) {
         out_nc[pix] = nc;
         if (LOGT) return;
+        if (PX == 64) finish_checkpoints(hm, st, rg.x, nc, sub, subs, p);
         out_img[pix] = make_float4(st.c[0], st.c[1], st.c[2], st.logT);
         float* dd = out_dist + 5 * pix;
 #pragma unroll
@@ -1628,21 +1682,19 @@ __device__ __forceinline__ void flush_entries(int n, const float4 (*srec)[kRecFl
 // The state of the reverse walk at the checkpoint at list offset s1, which the
 // pixel passed alive: log T, D2, D3 as stored, and the adjoint state after the
 // entries from s1 on.  Each of those hits adds T * dot(dL/dc, rgb) to
-// dL/dlogT, 2 m1 dL/dD0 to dL/dD2 and 2 m0 dL/dD1 to dL/dD3, and the sums of
-// T * rgb, m1 and m0 over them are what the colour, D3 and D2 still gain.
+// dL/dlogT, 2 m1 dL/dD0 to dL/dD2 and 2 m0 dL/dD1 to dL/dD3; the checkpoint
+// holds the sums of T * rgb, m0 and m1 over them.
 __device__ __forceinline__ void seed_segment(const HitMasks& hm, int x, int s1, int sub, int subs, int p,
-                                             float4 final_c, float& logT, float& D2, float& D3, const float* dS_c,
-                                             float& dS_logT, float* dS_D) {
+                                             float& logT, float& D2, float& D3, const float* dS_c, float& dS_logT,
+                                             float* dS_D) {
     const float* c = ck_at(hm, ck_id(x, s1 >> hm.seg_shift, hm.seg_shift), sub, subs, p);
     logT = __ldcg(c);
-    const float d2 = __ldcg(c + 64), d3 = __ldcg(c + 2 * 64);
-    dS_D[2] = fmaf(2.0f * dS_D[0], D3 - d3, dS_D[2]);
-    dS_D[3] = fmaf(2.0f * dS_D[1], D2 - d2, dS_D[3]);
-    D2 = d2;
-    D3 = d3;
-    dS_logT = fmaf(dS_c[0], final_c.x - __ldcg(c + 3 * 64), dS_logT);
-    dS_logT = fmaf(dS_c[1], final_c.y - __ldcg(c + 4 * 64), dS_logT);
-    dS_logT = fmaf(dS_c[2], final_c.z - __ldcg(c + 5 * 64), dS_logT);
+    D2 = __ldcg(c + 64);
+    D3 = __ldcg(c + 2 * 64);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) dS_logT = fmaf(dS_c[i], __ldcg(c + (3 + i) * 64), dS_logT);
+    dS_D[3] = fmaf(2.0f * dS_D[1], __ldcg(c + 6 * 64), dS_D[3]);
+    dS_D[2] = fmaf(2.0f * dS_D[0], __ldcg(c + 7 * 64), dS_D[2]);
 }
 
 // The lowest n bits of w (none for n <= 0).
@@ -1830,7 +1882,7 @@ __device__ __forceinline__ void bwd_item(
 #pragma unroll
         for (int k = 0; k < 5; ++k) dS_D[k] = gdist ? __ldg(gdist + 5 * pix + k) : 0.f;
         if (PX == 64 && nc > s1) {
-            seed_segment(hm, rg.x, s1, sub, subs, p, c, logT, D2, D3, dS_c, dS_logT, dS_D);
+            seed_segment(hm, rg.x, s1, sub, subs, p, logT, D2, D3, dS_c, dS_logT, dS_D);
             nc = s1;
         }
     }
@@ -2874,8 +2926,8 @@ size_t blend_ws_bytes(int64_t n_tets, int64_t n_tiles) {
 
 // Entries between two checkpoints (HitMasks) for lists of at most n_pairs
 // entries: 128, which keeps the longest stretch near 30 us, while their store
-// (12 bytes an entry and strip) stays under 200 MB; 512 up to 64M entries;
-// 4096 (0.4 bytes) for the long lists of many views, whose total work hides a
+// (16 bytes an entry and strip) stays under 270 MB; 512 up to 64M entries;
+// 4096 (0.5 bytes) for the long lists of many views, whose total work hides a
 // longer stretch.
 constexpr int kSegShifts[] = {12, 9, kMinSegShift};
 int seg_shift_for(int64_t n_pairs) {

@@ -119,3 +119,40 @@ def test_nan_ray_ends_at_the_first_entry_it_meets(cuda, tile, heavy, positive):
         assert nc[y, x] == (hit[0] + 1 if len(hit) else x1 - x0)
     ok = torch.from_numpy(~bad).cuda()
     assert torch.equal(r["nc"][ok], clean["nc"][ok]) and torch.equal(r["img"][ok], clean["img"][ok])
+
+
+@pytest.mark.parametrize("heavy", [1, 15])  # every tile by pair items, by warp items
+@pytest.mark.parametrize("n", [600, 1100])  # 4 and 8 checkpoints
+def test_stretches_hold_what_little_is_left(cuda, heavy, n):
+    """Bright entries before dark ones: what the dark ones still add to the
+    colour is far below the rounding of the colour.  A backward by stretches
+    takes it from the checkpoints, one over whole lists adds it up entry by
+    entry; each of the n additions rounds by 2^-24 at most, in both, so the
+    dark entries' gradients agree to 2n * 2^-24 (1.3e-4 for 1100)."""
+    verts, idx, cv = _stack(n, 0.2, n)
+    cv[:, 4:] = 0.0
+    cv[-100:, 1:4] *= 1e3  # the lists run from the last tets to the first
+    cv[:-100, 1:4] *= 1e-2
+    H, W = 21, 18
+    tcam = pinhole_tcam((0.1, 0.0, 0.0), (0.0, 0.0, 1.0), H, W, 30.0, tile_size=8)
+    jitter = np.random.default_rng(n).uniform(0, 1, (H, W, 2)).astype(np.float32)
+    old = R.blend_tuning()
+    R.set_blend_tuning(heavy << C.RM_BLEND_HEAVY_SHIFT, 0)
+    try:
+        r = run_gpu_forward(verts, idx, cv, tcam, jitter, keep_debug=False, hit_masks=True)
+    finally:
+        R.set_blend_tuning(*old)
+    g = torch.Generator("cuda").manual_seed(n)
+    r["gimg"] = 0.5 + 0.5 * torch.rand(H, W, 4, device="cuda", generator=g)
+    r["gimg"][..., 3] = 0.0
+    r["gdist"] = None
+    (gv0, gc0), (gv1, gc1) = _bwd(r, r["records"], False), _bwd(r, r["records"], True)
+    ids, ranges = r["lists"].sorted_ids.cpu().numpy(), r["lists"].ranges.cpu().numpy()
+    dark = np.arange(n) < 100
+    for x0, x1 in ranges:  # behind every bright one
+        bright = np.flatnonzero(ids[x0:x1] >= n - 100)
+        assert not dark[ids[x0:x0 + bright[-1] + 1]].any()
+    dark = to_dev(dark)
+    for a, b in ((gc1[dark, 0], gc0[dark, 0]), (gv1.view(n, 4, 3)[dark], gv0.view(n, 4, 3)[dark])):
+        assert float(b.norm()) > 0
+        assert float((a.double() - b.double()).norm()) <= 2 * n * 2.0**-24 * float(b.double().norm())
