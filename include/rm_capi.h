@@ -294,7 +294,9 @@ RM_API size_t rm_blend_workspace_size(int64_t n_tets, int64_t n_tiles);
  * n_tiles tiles of tile_pixels pixels: 4 bytes per 32 entries per pixel for
  * the masks, and 32 bytes per pixel at every 128th entry (512th above 16M
  * entries, 4096th above 64M) for the forward's state there, from which the
- * backward takes long lists in independent stretches. */
+ * backward takes long lists in independent stretches.  A forward goes by the
+ * entries that its lists hold: the first of these distances that they allow and
+ * whose states fit, none where not even the last one's do. */
 RM_API size_t rm_blend_hit_mask_bytes(int64_t n_pairs, int64_t n_tiles, int tile_pixels);
 /* Byte offset, inside a workspace of rm_blend_workspace_size(n_tets, n_tiles)
  * bytes, of the status word a blend pass uses when given no status_dev. */

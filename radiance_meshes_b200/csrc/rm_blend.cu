@@ -369,12 +369,45 @@ __device__ __forceinline__ float* ck_at(const HitMasks& hm, int64_t id, int sub,
     return hm.ck + ((id * subs + sub) * kCkFloats) * 64 + p;
 }
 
-// Header words of a pass with hit masks, written by the forward's order
-// kernel: [0] kMaskValid (kMaskStats in the statistics), [1] seg_shift, [2] checkpoint ids, [4..5] offset of
-// the checkpoints in words after the mask words' start.
-struct MaskHeader {
-    uint32_t state, seg_shift, ck_cap, pad;
-    int64_t ck_off;
+// Entries between two checkpoints for lists of n_pairs entries in all: 128,
+// which keeps the longest stretch near 30 us, while their store (16 bytes an
+// entry and strip) stays under 270 MB; 512 up to 64M entries; 4096 (0.5 bytes)
+// for the long lists of many views, whose total work hides a longer stretch.
+__host__ __device__ inline int seg_shift_for(int64_t n_pairs) {
+    return n_pairs <= (int64_t)16 << 20 ? kMinSegShift : n_pairs <= (int64_t)64 << 20 ? 9 : 12;
+}
+__host__ __device__ inline int64_t ck_count(int64_t n_pairs, int shift) { return (n_pairs >> shift) + 2; }
+__host__ __device__ inline int64_t ck_words(int64_t n_pairs, int64_t subs, int shift) {
+    return ck_count(n_pairs, shift) * subs * kCkFloats * 64;
+}
+__host__ __device__ inline int64_t mask_word_count(int64_t n_pairs, int64_t n_tiles, int64_t subs) {
+    return (n_pairs / 32 + n_tiles + 2) * subs * 64;
+}
+
+// Where a pass with `words` words of room keeps its checkpoints: after the
+// masks, at the end of the room.
+struct MaskPlan {
+    int shift;  // kNoSegments: nowhere
+    int64_t ck_cap, ck_off;
+};
+
+// The shortest stretch that n_pairs entries (those of this pass's lists, not
+// the most that the room was sized for) allow and whose checkpoints fit.
+__host__ __device__ inline MaskPlan mask_plan(int64_t words, int64_t n_tiles, int64_t subs, int64_t n_pairs) {
+    for (int shift = seg_shift_for(n_pairs); shift <= 12; shift += shift == kMinSegShift ? 2 : 3) {
+        const int64_t ck = ck_words(n_pairs, subs, shift);
+        if (mask_word_count(n_pairs, n_tiles, subs) + ck <= words) return {shift, ck_count(n_pairs, shift), words - ck};
+    }
+    return {kNoSegments, 0, words};
+}
+
+// The room of a forward with hit masks.  Its order kernel, which knows the
+// lists' lengths, writes the header: [0] state, [1] shift, [2] checkpoint ids,
+// [4..5] offset of the checkpoints in words after the mask words' start.
+struct MaskRoom {
+    uint32_t state;  // kMaskValid (kMaskStats in the statistics); 0: no masks
+    int subs;
+    int64_t words;
 };
 
 // The masks a kernel may use: none unless the header says that a walk of its
@@ -1272,7 +1305,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
 constexpr int kOrderCtas = 8;
 __global__ void __cluster_dims__(kOrderCtas, 1, 1) __launch_bounds__(1024)
     order_kernel(const int2* __restrict__ ranges, int G, int32_t* __restrict__ order, int32_t* info, uint32_t* tickets,
-                 int heavy_shift, uint32_t* mask_header, const MaskHeader mh, const uint32_t* seg_header,
+                 int heavy_shift, uint32_t* mask_header, const MaskRoom room, const uint32_t* seg_header,
                  int fwd_slots) {
     // Warp-aggregated counting: lanes that share a bucket elect one leader
     // (match_any) for the shared atomic, and the list-length sum and the
@@ -1342,8 +1375,16 @@ __global__ void __cluster_dims__(kOrderCtas, 1, 1) __launch_bounds__(1024)
         // segments per bucket of the masks' segment length (segment_item)
         int shift = kNoSegments;
         if (seg_header && __ldcg(seg_header) == kMaskValid) shift = (int)__ldcg(seg_header + 1);
-        if (mask_header && mh.state != 0u) shift = (int)mh.seg_shift;
-        if (shift >= kMinSegShift && shift < kNoSegments) {
+        if (mask_header) {
+            MaskPlan plan = {kNoSegments, 0, 0};
+            if (room.state != 0u) plan = mask_plan(room.words, G, room.subs, (int64_t)sum);
+            shift = plan.shift;
+            mask_header[0] = room.state;
+            mask_header[1] = (uint32_t)shift;
+            mask_header[2] = (uint32_t)plan.ck_cap;
+            *(int64_t*)(mask_header + 4) = plan.ck_off;
+        }
+        if (shift >= kMinSegShift && shift <= kNoSegments) {
             uint32_t at = 0;
             for (int b = 32; b > shift; --b) {
                 info[kSegInfoOff + 32 - b] = (int32_t)at;
@@ -1377,12 +1418,6 @@ __global__ void __cluster_dims__(kOrderCtas, 1, 1) __launch_bounds__(1024)
         }
         info[1] = min(quarters, heavy);
         for (int k = 0; k < 4; ++k) tickets[k] = 0u;
-        if (mask_header) {
-            mask_header[0] = mh.state;
-            mask_header[1] = mh.seg_shift;
-            mask_header[2] = mh.ck_cap;
-            *(int64_t*)(mask_header + 4) = mh.ck_off;
-        }
     }
     __syncthreads();
     const unsigned lt = (1u << lane) - 1u;
@@ -2739,7 +2774,7 @@ __device__ __forceinline__ void err_seg_item(int tile, int sub, int seg, const i
     const int2 rg = __ldg(ranges + tile);
     const int len = rg.y - rg.x;
     int s0 = 0, s1 = len;
-    if (len > (1 << hm.seg_shift)) {
+    if (hm.ck && len > (1 << hm.seg_shift)) {
         const int shift = hm.seg_shift;
         if (ck_id(rg.x, (len - 1) >> shift, shift) < hm.ck_cap) {
             s0 = seg << shift;
@@ -2924,46 +2959,6 @@ size_t blend_ws_bytes(int64_t n_tets, int64_t n_tiles) {
     return rec + ord + 256;
 }
 
-// Entries between two checkpoints (HitMasks) for lists of at most n_pairs
-// entries: 128, which keeps the longest stretch near 30 us, while their store
-// (16 bytes an entry and strip) stays under 270 MB; 512 up to 64M entries;
-// 4096 (0.5 bytes) for the long lists of many views, whose total work hides a
-// longer stretch.
-constexpr int kSegShifts[] = {12, 9, kMinSegShift};
-int seg_shift_for(int64_t n_pairs) {
-    return n_pairs <= (int64_t)16 << 20 ? kMinSegShift : n_pairs <= (int64_t)64 << 20 ? 9 : 12;
-}
-
-int64_t ck_count(int64_t n_pairs, int shift) { return (n_pairs >> shift) + 2; }
-int64_t ck_words(int64_t n_pairs, int64_t subs, int shift) {
-    return ck_count(n_pairs, shift) * subs * kCkFloats * 64;
-}
-int64_t mask_word_count(int64_t n_pairs, int64_t n_tiles, int64_t subs) {
-    return (n_pairs / 32 + n_tiles + 2) * subs * 64;
-}
-
-// The header of a forward with hit masks over G tiles of `subs` strips with
-// `words` words of room: the largest list size whose masks fit with their
-// checkpoints, the checkpoints after the masks.
-MaskHeader mask_header_for(int64_t words, int64_t G, int64_t subs) {
-    MaskHeader h = {kMaskValid, (uint32_t)kNoSegments, 0u, 0u, words};
-    for (int shift : kSegShifts) {
-        int64_t lo = 0, hi = words;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi + 1) / 2;
-            if (mask_word_count(mid, G, subs) + ck_words(mid, subs, shift) <= words) lo = mid;
-            else hi = mid - 1;
-        }
-        if (lo == 0) return h;  // no room
-        if (shift != kMinSegShift && seg_shift_for(lo) != shift) continue;  // the shorter segments fit too
-        h.seg_shift = (uint32_t)shift;
-        h.ck_cap = (uint32_t)ck_count(lo, shift);
-        h.ck_off = words - ck_words(lo, subs, shift);
-        break;
-    }
-    return h;
-}
-
 // Hit masks, when the caller's workspace is larger than blend_ws_bytes: a
 // 256-byte header, the mask words (mask_word), the checkpoints (ck_at).
 BlendWs blend_ws(void* base, int64_t n_tets, int64_t n_tiles, size_t workspace_bytes) {
@@ -3071,9 +3066,9 @@ int side_stream(cudaStream_t caller, SideStream** out) {
 }
 
 int launch_order(const int32_t* ranges, int G, const BlendWs& w, int heavy_shift, cudaStream_t s,
-                 uint32_t* mask_header = nullptr, MaskHeader mh = MaskHeader{}, const uint32_t* seg_header = nullptr,
+                 uint32_t* mask_header = nullptr, MaskRoom room = MaskRoom{}, const uint32_t* seg_header = nullptr,
                  int fwd_slots = 0) {
-    order_kernel<<<kOrderCtas, 1024, 0, s>>>((const int2*)ranges, G, w.order, w.info, w.tickets, heavy_shift, mask_header, mh,
+    order_kernel<<<kOrderCtas, 1024, 0, s>>>((const int2*)ranges, G, w.order, w.info, w.tickets, heavy_shift, mask_header, room,
                                     seg_header, fwd_slots);
     return rm_host::check_launch("rm_blend order");
 }
@@ -3130,11 +3125,9 @@ int launch_fwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, cons
     const bool masks = tn.hit_masks && PX == 64 && w.mask_header;
     const int subs = sh.tile_px / PX;
     const int cap = tn.pair_ctas_per_sm * sm_count();
-    MaskHeader mh = {};
-    if (masks) mh = mask_header_for(w.mask_cap, G, subs);
-    if (masks && LOGT) mh.state = kMaskStats;
+    const MaskRoom room = {!masks ? 0u : LOGT ? kMaskStats : kMaskValid, subs, w.mask_cap};
     int rc = launch_order(ranges, G, w, PX == 64 ? tn.heavy_shift : tn.heavy_shift == 0 ? 1 : tn.heavy_shift, s,
-                          w.mask_header, mh, nullptr, PX == 64 ? (cap > subs ? cap / subs : 1) : 0);
+                          w.mask_header, room, nullptr, PX == 64 ? (cap > subs ? cap / subs : 1) : 0);
     if (rc) return rc;
     const HitMasks hm = {masks ? w.mask_words : nullptr, w.mask_cap, w.mask_header, nullptr, 0, kNoSegments};
     const Queue q = {w.order, w.info, w.tickets + 0, G, subs, true, hm, tn.status, rm_host::wait_limit(), tn.n_recs};
@@ -3159,7 +3152,7 @@ int launch_bwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, cons
     const int subs = sh.tile_px / PX;
     const int subs_pair = sh.tile_px / PX_PAIR;
     const bool masks = tn.hit_masks && PX == 64 && w.mask_header;
-    int rc = launch_order(ranges, G, w, tn.heavy_shift, s, nullptr, MaskHeader{}, masks ? w.mask_header : nullptr);
+    int rc = launch_order(ranges, G, w, tn.heavy_shift, s, nullptr, MaskRoom{}, masks ? w.mask_header : nullptr);
     if (rc) return rc;
     const HitMasks hm = {masks ? w.mask_words : nullptr, w.mask_cap, w.mask_header, nullptr, 0, kNoSegments};
     const Queue qd = {w.order, w.info, w.tickets + 2, G, subs, false, hm, tn.status, rm_host::wait_limit(),
@@ -3409,7 +3402,7 @@ int rm_calc_tet_err(const int32_t* sorted_ids, const int32_t* ranges, const int3
     if ((flags & RM_BLEND_OWN_SCRATCH) && strip == 64 && workspace_bytes > blend_ws_bytes(n_tets, G) + nc_bytes + 512) {
         const size_t nc_off = (workspace_bytes - nc_bytes) / 256 * 256;
         const BlendWs wm = blend_ws(workspace, n_tets, G, nc_off);
-        if (wm.mask_header && mask_header_for(wm.mask_cap, G, subs).seg_shift < (uint32_t)kNoSegments) {
+        if (wm.mask_header) {
             int32_t* nc = (int32_t*)((char*)workspace + nc_off);
             const OneView one = {*cam};
             const Shape sh = {(int)G, cam->tile_width * cam->tile_height};

@@ -156,3 +156,87 @@ def test_stretches_hold_what_little_is_left(cuda, heavy, n):
     for a, b in ((gc1[dark, 0], gc0[dark, 0]), (gv1.view(n, 4, 3)[dark], gv0.view(n, 4, 3)[dark])):
         assert float(b.norm()) > 0
         assert float((a.double() - b.double()).norm()) <= 2 * n * 2.0**-24 * float(b.double().norm())
+
+
+def _room(n_pairs, n_tiles, subs, shift=None):
+    """Bytes for the masks of n_pairs entries, and their checkpoints every 1 << shift."""
+    words = (n_pairs // 32 + n_tiles + 2) * subs * 64
+    return 256 + 4 * (words + (0 if shift is None else ((n_pairs >> shift) + 2) * subs * 8 * 64))
+
+
+def _header(ws, n_tets, n_tiles):
+    base = C.lib().rm_blend_workspace_size(n_tets, n_tiles)
+    return ws[base:base + 12].view(torch.int32).tolist()  # state, log2 of the stretch, checkpoint ids
+
+
+def _fwd_into(r, ws):
+    L = r["lists"]
+    img, dist, nc, _ = R.blend_fwd(L.sorted_ids, L.ranges, r["i"], r["v"], r["c"], r["j"], r["cam"],
+                                   tiles_touched=r["tiles"], records=ws, hit_masks=True)
+    assert torch.equal(img, r["img"]) and torch.equal(dist, r["dist"]) and torch.equal(nc, r["nc"])
+
+
+@pytest.mark.parametrize("million", [1, 9, 12, 16, 17, 55, 65, 100])
+def test_stretch_length_is_that_of_the_lists(cuda, million):
+    """Short lists are cut every 128 entries, however many the workspace has
+    room for."""
+    r = _scene(33, 0.3)
+    G = r["cam"].grid_width * r["cam"].grid_height
+    size = C.lib().rm_blend_workspace_size(33, G) + C.lib().rm_blend_hit_mask_bytes(million * 1_000_000, G, 64)
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    _fwd_into(r, ws)
+    assert _header(ws, 33, G)[1] == 7
+
+
+@pytest.mark.parametrize("entries,shift", [(16 << 20, 7), ((16 << 20) + 1, 9), (64 << 20, 9), ((64 << 20) + 1, 12)])
+def test_stretch_length_of_long_lists(cuda, entries, shift):
+    """Above 16M entries every 512, above 64M every 4096 (rm_capi.h); the size
+    that rm_blend_hit_mask_bytes gives has room for them."""
+    verts, idx, cv = _stack(1, 400.0, 1)
+    tcam = pinhole_tcam((0.1, 0.0, 0.0), (0.0, 0.0, 1.0), 16, 16, 30.0, tile_size=8)
+    r = run_gpu_forward(verts, idx, cv, tcam, np.full((16, 16, 2), 0.5, np.float32), keep_debug=False)
+    cuts = [0, 1, entries // 2, entries // 2, entries]  # one tet over and over
+    ranges = to_dev(np.array(list(zip(cuts[:-1], cuts[1:])), np.int32))
+    ids = torch.zeros(entries, dtype=torch.int32, device="cuda")
+    _, _, _, ws = R.blend_fwd(ids, ranges, r["i"], r["v"], r["c"], r["j"], r["cam"], hit_masks=True)
+    state, got, ids_fit = _header(ws, 1, 4)
+    assert got == shift and ids_fit == (entries >> shift) + 2
+
+
+@pytest.mark.parametrize("shift", [7, 9, 12, None, "half"])
+@pytest.mark.parametrize("heavy", [0, 15])
+def test_room_for_longer_stretches_or_none(cuda, shift, heavy):
+    """A workspace too small for the shortest stretches gets the next longer
+    ones, or none where not even the masks all fit: the same image, gradients
+    and statistics."""
+    n = 9000  # three stretches of 4096
+    r = _scene(n, 0.02, H=9, W=14)
+    L, cam = r["lists"], r["cam"]
+    whole = _bwd(r, r["records"], False)
+    G, P = cam.grid_width * cam.grid_height, L.n_pairs
+    base = C.lib().rm_blend_workspace_size(n, G)
+    room = _room(P, G, 1, shift) if shift != "half" else _room(P // 2, G, 1)
+    ws = torch.zeros(base + room, dtype=torch.uint8, device="cuda")
+    old = R.blend_tuning()
+    R.set_blend_tuning(heavy << C.RM_BLEND_HEAVY_SHIFT, 0)
+    try:
+        _fwd_into(r, ws)
+    finally:
+        R.set_blend_tuning(*old)
+    assert _header(ws, n, G)[1] == (shift if isinstance(shift, int) else 31)
+    _same(_bwd(r, ws, True), whole)
+    # the statistics on the same room (and their counts, a pixel each, after it)
+    rng = np.random.default_rng(n)
+    pe, se = (to_dev(rng.uniform(0, 1, (cam.image_height, cam.image_width)).astype(np.float32)) for _ in range(2))
+    out = []
+    for size, flags in ((base + room + 512 + 4 * pe.numel(), C.RM_BLEND_OWN_SCRATCH), (base, 0)):
+        ws = torch.zeros(size, dtype=torch.uint8, device="cuda")
+        err, cnt = torch.zeros(n, 16, device="cuda"), torch.zeros(n, 2, dtype=torch.int32, device="cuda")
+        C.check(C.lib().rm_calc_tet_err(
+            C.ptr(L.sorted_ids), C.ptr(L.ranges), C.ptr(r["i"]), C.ptr(r["v"]), C.ptr(r["c"]), n, r["v"].shape[0],
+            None, ctypes.byref(cam), C.ptr(pe), C.ptr(se), C.ptr(err), C.ptr(cnt), C.ptr(ws), size, flags,
+            C.stream_handle()), "rm_calc_tet_err")
+        out.append((err, cnt))
+    (err, cnt), (err0, cnt0) = out
+    assert cnt0[:, 0].sum() > 0 and torch.equal(cnt, cnt0)
+    assert float((err - err0).norm()) <= 1e-5 * float(err0.norm())
