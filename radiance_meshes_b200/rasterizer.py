@@ -299,25 +299,28 @@ def _count_read_start(count: torch.Tensor):
     pinned host memory; the host waits in _count_read_finish for the copy
     only, while the GPU goes on with what is queued after this call.  (On a
     side stream the 16-byte copy left the frame's stream alone, and cost the
-    host two events and a stream switch: 20 us of a small frame's 445.)"""
+    host two events and a stream switch: 20 us of a small frame's 445.)
+
+    The buffer is out of the table until the read is finished: a frame that
+    fails in between leaves its copy in flight, and the next frame, maybe on
+    another stream, must not read what that copy writes."""
     dev = count.device
     key = (dev, threading.get_ident())  # threads building frames at once each read their own buffer
-    st = _COUNT_READ.get(key)
+    st = _COUNT_READ.pop(key, None)
     if st is None:
         hb = torch.zeros(2, dtype=torch.int64, pin_memory=True)
         st = (hb, hb.numpy())
-        _COUNT_READ[key] = st
-    hb, hn = st
-    hb.copy_(count, non_blocking=True)
+    st[0].copy_(count, non_blocking=True)
     done = torch.cuda.Event()
     done.record()
-    return done, hn
+    return done, key, st
 
 
 def _count_read_finish(pending) -> tuple[int, int]:
-    done, hn = pending
+    done, key, st = pending
     done.synchronize()
-    return int(hn[0]), int(hn[1]) & 0xffffffff
+    _COUNT_READ[key] = st
+    return int(st[1][0]), int(st[1][1]) & 0xffffffff
 
 
 _LISTS = {"depth_first": True}
