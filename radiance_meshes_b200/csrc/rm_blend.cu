@@ -312,6 +312,11 @@ struct PixelState {
     float part[5];  // what the hits since the last checkpoint added to the colour, D2 and D3
 };
 
+// What a forward walk forms: the image; the image and what a backward needs
+// (hit masks, checkpoints), whose five sums cost a frame 2 to 3% that has no
+// use for them; or log T from 1 with masks and checkpoints (the statistics).
+enum Walk { kImage, kImageAndMasks, kLogT };
+
 // ------------------------------------------------------------------ forward --
 template <int NT>
 struct WarpShape {
@@ -581,12 +586,13 @@ __device__ __forceinline__ void finish_checkpoints(const HitMasks& hm, const Pix
 // One hit folded into the pixel state (update_alpha_out,
 // alphablend_shader_interp.slang:84-183): colour += rgb * T, log T -= a, and
 // the five distortion moments with m0 = density, m1 = density * (a + b) / 2.
+template <bool PART>
 __device__ __forceinline__ void fold_hit(PixelState& st, float a, float m0, float m1, float d4, const float* rgb) {
     const float T = exp_approx(st.logT);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         st.c[k] = fmaf(rgb[k], T, st.c[k]);
-        st.part[k] = fmaf(rgb[k], T, st.part[k]);
+        if (PART) st.part[k] = fmaf(rgb[k], T, st.part[k]);
     }
     st.logT = st.logT - a;
     const float D2 = st.D[2], D3 = st.D[3];
@@ -595,8 +601,10 @@ __device__ __forceinline__ void fold_hit(PixelState& st, float a, float m0, floa
     st.D[2] = D2 + m0;
     st.D[3] = D3 + m1;
     st.D[4] = st.D[4] + d4;
-    st.part[3] = st.part[3] + m0;
-    st.part[4] = st.part[4] + m1;
+    if (PART) {
+        st.part[3] = st.part[3] + m0;
+        st.part[4] = st.part[4] + m1;
+    }
 }
 
 // Result of testing one ray against one list entry, in the exact arithmetic of
@@ -853,15 +861,18 @@ __device__ __forceinline__ void stage_pair_batch(FwdPairSmem<PX, B>& S, int buf,
 }
 
 // One entry of the fold, hit or miss (a = 0, every increment zero).
+template <bool PART>
 __device__ __forceinline__ void fold_any(PixelState& st, float a, float m0, float m1, float d4, float r, float g,
                                          float b) {
     const float T = exp_approx(st.logT);
     st.c[0] = fmaf(r, T, st.c[0]);
     st.c[1] = fmaf(g, T, st.c[1]);
     st.c[2] = fmaf(b, T, st.c[2]);
-    st.part[0] = fmaf(r, T, st.part[0]);
-    st.part[1] = fmaf(g, T, st.part[1]);
-    st.part[2] = fmaf(b, T, st.part[2]);
+    if (PART) {
+        st.part[0] = fmaf(r, T, st.part[0]);
+        st.part[1] = fmaf(g, T, st.part[1]);
+        st.part[2] = fmaf(b, T, st.part[2]);
+    }
     st.logT = st.logT - a;
     const float D2 = st.D[2], D3 = st.D[3];
     st.D[0] = fmaf(2.0f * m1, D2, st.D[0]);
@@ -869,11 +880,13 @@ __device__ __forceinline__ void fold_any(PixelState& st, float a, float m0, floa
     st.D[2] = D2 + m0;
     st.D[3] = D3 + m1;
     st.D[4] = st.D[4] + d4;
-    st.part[3] = st.part[3] + m0;
-    st.part[4] = st.part[4] + m1;
+    if (PART) {
+        st.part[3] = st.part[3] + m0;
+        st.part[4] = st.part[4] + m1;
+    }
 }
 
-template <int PX, int NT, int B, bool LOGT>
+template <int PX, int NT, int B, Walk WALK>
 __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, const int32_t* __restrict__ ids,
                                          const int2* __restrict__ ranges, const float4* __restrict__ recs,
                                          const float2* __restrict__ jitter, const rm_camera& cam,
@@ -883,7 +896,7 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
     using Sh = PairShape<PX, NT, B>;
     static_assert(PX <= 64 && NT >= 64, "two owner warps at most");
     static_assert(Sh::kStageWarps >= 1 && Sh::kStageWarps <= FwdPairSmem<PX, B>::kMaxStage, "staging warps");
-    constexpr bool kMasks = PX == 64;
+    constexpr bool LOGT = WALK == kLogT, kMasks = PX == 64 && WALK != kImage;
     constexpr int RB = Sh::RB;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool own_warp = warp < Sh::kOwnWarps;
@@ -1050,7 +1063,7 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
                         for (int k = 0; k < 4; ++k) {
                             const bool hit = r[0][k] > 0.f;
                             hb |= hit ? bit[k] : 0u;
-                            fold_any(st, r[0][k], hit ? dens[k] : 0.f, r[1][k], r[2][k], r[3][k], r[4][k], r[5][k]);
+                            fold_any<kMasks>(st, r[0][k], hit ? dens[k] : 0.f, r[1][k], r[2][k], r[3][k], r[4][k], r[5][k]);
                         }
                     } else {
                         for (int k = 0; k < 4 && j + k < j1; ++k) {
@@ -1058,7 +1071,7 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
                             if (!(ak > 0.f)) continue;
                             const int at = S.pos[cur][j + k];
                             hb |= 1u << at;
-                            fold_any(st, ak, S.dens[cur][j + k], S.res[1][j + k][slot], S.res[2][j + k][slot],
+                            fold_any<kMasks>(st, ak, S.dens[cur][j + k], S.res[1][j + k][slot], S.res[2][j + k][slot],
                                      S.res[3][j + k][slot], S.res[4][j + k][slot], S.res[5][j + k][slot]);
                             if (st.logT < kTermLogT) {
                                 active = false;
@@ -1118,13 +1131,14 @@ struct FwdWarpSmem {
     float4 srec[AHEAD ? 2 : 1][32][kRecFloat4 + 1];  // padded: 32 lanes read one record each without conflicts
 };
 
-template <int PX, bool LOGT, bool AHEAD>
+template <int PX, Walk WALK, bool AHEAD>
 __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const int32_t* __restrict__ ids,
                                               const int2* __restrict__ ranges, const float4* __restrict__ recs,
                                               const float2* __restrict__ jitter, const rm_camera& cam,
                                               float4* __restrict__ out_img, float* __restrict__ out_dist,
                                               int32_t* __restrict__ out_nc, FwdWarpSmem<AHEAD>& S, const HitMasks& hm,
                                               int subs, int gtile, const Queue& lq) {
+    constexpr bool LOGT = WALK == kLogT, kMasks = PX == 64 && WALK != kImage;
     const int lane = threadIdx.x & 31;
     const int2 rg = __ldg(ranges + tile);
     const int p = half * 32 + lane;
@@ -1177,7 +1191,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
     if (AHEAD && __any_sync(0xffffffffu, active)) fetch(0, g);
     int buf = 0;
     for (int base = rg.x; base < rg.y && __any_sync(0xffffffffu, active); base += 32) {
-        if (PX == 64 && active) write_checkpoint<LOGT>(hm, st, rg.x, base, sub, subs, p);
+        if (kMasks && active) write_checkpoint<LOGT>(hm, st, rg.x, base, sub, subs, p);
         const bool valid = g >= 0;
         if (AHEAD) {
             g = g_ahead;
@@ -1203,7 +1217,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
                 if (e.a > 0.f) {
                     hb |= 1u << j;
                     if (LOGT) st.logT = st.logT - e.a;
-                    else fold_hit(st, e.a, rec[j][0].w, e.m1, e.d4, e.rgb);
+                    else fold_hit<kMasks>(st, e.a, rec[j][0].w, e.m1, e.d4, e.rgb);
                     if (st.logT < kTermLogT) {
                         nc = base - rg.x + j + 1;
                         ended = true;
@@ -1212,7 +1226,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
                 }
             }
         }
-        if (PX == 64 && hm.words) {
+        if (kMasks && hm.words) {
             const int64_t i = mask_word(gtile, rg.x, (base - rg.x) >> 5, sub, subs, p);
             if (i < hm.cap) __stcg(hm.words + i, hb);
         }
@@ -1230,7 +1244,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
     if (inside) {
         out_nc[pix] = nc;
         if (LOGT) return;
-        if (PX == 64) finish_checkpoints(hm, st, rg.x, nc, sub, subs, p);
+        if (kMasks) finish_checkpoints(hm, st, rg.x, nc, sub, subs, p);
         out_img[pix] = make_float4(st.c[0], st.c[1], st.c[2], st.logT);
         float* dd = out_dist + 5 * pix;
 #pragma unroll
@@ -1242,7 +1256,7 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
 // more than the warps gain, with the little L1 that the shared memory leaves
 // (1.3M tets, 1297x840: 1461 -> 1293 and 1357 -> 1024 us; a batch of four
 // served views 4187 -> 3500 us).
-template <int PX, int NT, int B, class V, bool LOGT>
+template <int PX, int NT, int B, class V, Walk WALK>
 __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
     const int32_t* __restrict__ ids, const int2* __restrict__ ranges, const float4* __restrict__ recs,
     const float2* __restrict__ jitter, const __grid_constant__ V views, float4* __restrict__ out_img,
@@ -1257,7 +1271,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
     const int q_items = nq * q.subs * 4;
     const int n_items = q_items + (__ldg(q.info) - nq) * q.subs;
     if (threadIdx.x == 0)
-        hm = live_masks(q.hm, q.subs, LOGT ? kMaskStats : kMaskValid);  // seen after next_item's barriers
+        hm = live_masks(q.hm, q.subs, WALK == kLogT ? kMaskStats : kMaskValid);  // seen after next_item's barriers
     for (;;) {
         int item = next_item(q, &s_item);
         if (item >= n_items) break;
@@ -1272,7 +1286,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
         const int t = __ldg(q.order + at + item / q.subs), v = views.find(t);
         const int tb = views.tile_base(v);
         const int64_t pb = views.pixel_base(v);
-        fwd_pair_item<PX, NT, B, LOGT>(t - tb, item % q.subs, quarter, ids, ranges + tb, recs, jitter + pb, views.camera(v),
+        fwd_pair_item<PX, NT, B, WALK>(t - tb, item % q.subs, quarter, ids, ranges + tb, recs, jitter + pb, views.camera(v),
                                  out_img + pb, out_dist + 5 * pb, out_nc + pb, S, hm, q.subs, t, q);
     }
     constexpr int kParts = PX / 32 > 0 ? PX / 32 : 1;
@@ -1289,7 +1303,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
         const int t = __ldg(q.order + heavy + strip / q.subs), v = views.find(t);
         const int tb = views.tile_base(v);
         const int64_t pb = views.pixel_base(v);
-        fwd_warp_item<PX, LOGT, kAhead>(t - tb, strip % q.subs, part, ids, ranges + tb, recs, jitter + pb, views.camera(v),
+        fwd_warp_item<PX, WALK, kAhead>(t - tb, strip % q.subs, part, ids, ranges + tb, recs, jitter + pb, views.camera(v),
                           out_img + pb, out_dist + 5 * pb, out_nc + pb, W, hm, q.subs, t, q);
     }
 }
@@ -3116,22 +3130,22 @@ struct Shape {
 
 // Forward pass: order kernel, then one persistent kernel for the heavy tiles
 // (pair items) and the others (warp items).
-template <int PX, int NT, int B, class V, bool LOGT = false>
+template <int PX, int NT, int B, Walk WALK, class V>
 int launch_fwd(const int32_t* ids, const int32_t* ranges, const BlendWs& w, const float* jitter, const V& views,
                const Shape& sh, float* img, float* dist, int32_t* nc, const Tuning& tn, cudaStream_t s) {
     const int G = sh.G;
     // hit masks need 64-pixel items; the header records whether this forward
     // wrote them, so a backward never reads stale masks
-    const bool masks = tn.hit_masks && PX == 64 && w.mask_header;
+    const bool masks = WALK != kImage && w.mask_header;
     const int subs = sh.tile_px / PX;
     const int cap = tn.pair_ctas_per_sm * sm_count();
-    const MaskRoom room = {!masks ? 0u : LOGT ? kMaskStats : kMaskValid, subs, w.mask_cap};
+    const MaskRoom room = {!masks ? 0u : WALK == kLogT ? kMaskStats : kMaskValid, subs, w.mask_cap};
     int rc = launch_order(ranges, G, w, PX == 64 ? tn.heavy_shift : tn.heavy_shift == 0 ? 1 : tn.heavy_shift, s,
                           w.mask_header, room, nullptr, PX == 64 ? (cap > subs ? cap / subs : 1) : 0);
     if (rc) return rc;
     const HitMasks hm = {masks ? w.mask_words : nullptr, w.mask_cap, w.mask_header, nullptr, 0, kNoSegments};
     const Queue q = {w.order, w.info, w.tickets + 0, G, subs, true, hm, tn.status, rm_host::wait_limit(), tn.n_recs};
-    auto kernel = blend_fwd_kernel<PX, NT, B, V, LOGT>;
+    auto kernel = blend_fwd_kernel<PX, NT, B, V, WALK>;
     constexpr int kPairSmem = (int)sizeof(FwdPairSmem<PX, B>),
                   kWarpSmem = NT / 32 * (int)sizeof(FwdWarpSmem<(V::kViews > 1)>);
     constexpr int smem = kPairSmem > kWarpSmem ? kPairSmem : kWarpSmem;
@@ -3290,21 +3304,24 @@ int blend_fwd_any(const char* who, const int32_t* sorted_ids, const int32_t* ran
     if ((rc = pass_status(who, w, status_dev, s, &tn.status))) return rc;
     // tets per shared-memory batch of the pair items: 16, 32 (default) or 64
     const int key = strip_pixels(cam0, flags) * 1000 + batch_size(flags, 32);
-#define RM_FWD_CASE(PX, NT, BP)                                                                                  \
-    case PX * 1000 + BP:                                                                                         \
-        return launch_fwd<PX, NT, BP>(sorted_ids, ranges, w, ray_jitter, views, sh, out_img, out_distortion, \
-                                              n_contrib, tn, s);
+    const bool masks = tn.hit_masks && w.mask_header;
+#define RM_FWD_CALL(PX, NT, BP, WALK)                                                                             \
+    launch_fwd<PX, NT, BP, WALK>(sorted_ids, ranges, w, ray_jitter, views, sh, out_img, out_distortion, n_contrib, \
+                                 tn, s)
+#define RM_FWD_STRIP(BP)              \
+    case 16 * 1000 + BP:              \
+        return RM_FWD_CALL(16, 64, BP, kImage); \
+    case 64 * 1000 + BP:              \
+        return masks ? RM_FWD_CALL(64, 256, BP, kImageAndMasks) : RM_FWD_CALL(64, 256, BP, kImage);
     switch (key) {
-        RM_FWD_CASE(16, 64, 16)
-        RM_FWD_CASE(16, 64, 32)
-        RM_FWD_CASE(16, 64, 64)
-        RM_FWD_CASE(64, 256, 16)
-        RM_FWD_CASE(64, 256, 32)
-        RM_FWD_CASE(64, 256, 64)
+        RM_FWD_STRIP(16)
+        RM_FWD_STRIP(32)
+        RM_FWD_STRIP(64)
         default:
             return rm_host::fail(RM_EINVAL, "%s: tets per batch %d unsupported (16, 32 or 64)", who, key % 1000);
     }
-#undef RM_FWD_CASE
+#undef RM_FWD_STRIP
+#undef RM_FWD_CALL
 }
 
 template <class V>
@@ -3409,7 +3426,7 @@ int rm_calc_tet_err(const int32_t* sorted_ids, const int32_t* ranges, const int3
             Tuning tn = tuning_from_flags(flags, 0, 3);
             tn.hit_masks = true;
             tn.n_recs = n_tets;
-            rc = launch_fwd<64, 256, 32, OneView, true>(sorted_ids, ranges, wm, nullptr, one, sh, nullptr, nullptr, nc,
+            rc = launch_fwd<64, 256, 32, kLogT>(sorted_ids, ranges, wm, nullptr, one, sh, nullptr, nullptr, nc,
                                                         tn, s);
             if (rc) return rc;
             const HitMasks hm = {wm.mask_words, wm.mask_cap, wm.mask_header, nullptr, 0, kNoSegments};
