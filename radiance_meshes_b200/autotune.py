@@ -12,15 +12,20 @@ Knobs, all measured on the caller's own mesh and cameras:
   decide in the forward, 1 sends every tile to the CTAs), and the resident
   CTAs per SM.
 * pixels per work item (strip of 16 or 64 pixels).
-* tets per shared-memory batch (16, 32 or 64).
+* tets per shared-memory batch of the forward's CTAs (16, 32 or 64; the
+  backward has a batch with bulk-copy staging only, which no batch of views
+  uses).
 
 Each candidate is timed with CUDA events on one eager fwd / bwd pass after a
-warm-up pass.  The winner is cached in a JSON file keyed by the GPU, the mesh
+warm-up pass.  The winner is cached in a JSON file keyed by the GPU, the
+library's build (flags that suited other kernels are not kept), the mesh
 size, the views' resolutions and the tile candidates
 (``$RM_AUTOTUNE_CACHE``, default ``~/.cache/radiance_meshes_b200/autotune.json``).
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import math
 import os
@@ -31,6 +36,7 @@ import torch
 
 from . import _capi as C
 from . import batch as B
+from . import build
 from .camera import tcam_to_struct
 
 __all__ = ["flags", "tune_batch", "candidates_fwd", "candidates_bwd", "cache_path", "list_configs"]
@@ -58,18 +64,15 @@ def candidates_fwd(tile: int):
     for b in (16, 32, 64):
         for ctas in (2, 3):
             out.append(dict(strip=strip, heavy_shift=0, pair_ctas=ctas, batch=b))
-    out.append(dict(strip=strip, heavy_shift=1, pair_ctas=3, batch=32))
-    out.append(dict(strip=16, heavy_shift=1, pair_ctas=3, batch=32))
+    for px in sorted({strip, 16}, reverse=True):
+        out.append(dict(strip=px, heavy_shift=1, pair_ctas=3, batch=32))
     out.append(dict(strip=strip, heavy_shift=3, pair_ctas=2, batch=32))
     return out
 
 
 def candidates_bwd(tile: int):
-    out = []
-    for strip in ((16, 64) if tile >= 8 else (16,)):
-        for b in (16, 32, 64):
-            out.append(dict(strip=strip, heavy_shift=0, pair_ctas=1, batch=b))
-    out.append(dict(strip=64 if tile >= 8 else 16, heavy_shift=3, pair_ctas=1, batch=32))
+    out = [dict(strip=strip, heavy_shift=0, pair_ctas=1) for strip in ((16, 64) if tile >= 8 else (16,))]
+    out.append(dict(strip=64 if tile >= 8 else 16, heavy_shift=3, pair_ctas=1))
     return out
 
 
@@ -101,10 +104,16 @@ def _store_cache(key, value):
             pass
 
 
+@functools.lru_cache(maxsize=None)
+def _build_id(path: str) -> str:
+    with open(path, "rb") as f:
+        return hashlib.blake2b(f.read(), digest_size=8).hexdigest()
+
+
 def _key(device, n_tets, views, tiles, backward):
     p = torch.cuda.get_device_properties(device)
     res = ",".join(f"{v.width}x{v.height}" for v in views)
-    return (f"{p.name}|sm{p.multi_processor_count}|T{int(round(math.log2(max(n_tets, 1)) * 4))}|{res}|"
+    return (f"{p.name}|sm{p.multi_processor_count}|lib{_build_id(build.lib_path())}|T{int(round(math.log2(max(n_tets, 1)) * 4))}|{res}|"
             f"tiles{'/'.join(map(str, tiles))}|{'fwdbwd' if backward else 'fwd'}")
 
 
