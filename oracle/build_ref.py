@@ -24,6 +24,7 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 REF_DIR = os.path.join(HERE, "_ref")
+REFERENCE = os.environ.get("RM_REFERENCE_TREE", "/root/reference")
 SORT_SRC = os.path.join("delaunay_rasterization", "internal", "sort_by_keys", "sort_by_keys.cu")
 SORT_SO = os.path.join(REF_DIR, "sort_by_keys", "sort_by_keys.so")
 
@@ -60,7 +61,7 @@ def load_sort():
 
 def main(argv=None):
     ap = argparse.ArgumentParser()
-    ap.add_argument("--reference", default=os.environ.get("RM_REFERENCE_TREE", "/root/reference"))
+    ap.add_argument("--reference", default=REFERENCE)
     ap.add_argument("--verbose", action="store_true")
     a = ap.parse_args(argv)
     print(build_sort(a.reference, a.verbose))
