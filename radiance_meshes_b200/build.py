@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 LIBNAME = "librm_b200.so"
 SOURCES = ["rm_capi.cu", "rm_project.cu", "rm_scan.cu", "rm_sort.cu", "rm_blend.cu", "rm_fine.cu", "rm_features.cu", "rm_tets.cu", "rm_ssim.cu"]
-HEADERS = ["rm_internal.cuh", os.path.join("..", "..", "include", "rm_capi.h")]
+HEADERS = ["rm_internal.cuh", "rm_approx.cuh", os.path.join("..", "..", "include", "rm_capi.h")]
 
 # --fmad=false: every fused multiply-add in the kernels is written explicitly
 # (fmaf), which keeps the integer outputs reproducible (see rm_internal.cuh).

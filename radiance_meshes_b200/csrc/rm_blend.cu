@@ -33,6 +33,7 @@
 #include <cooperative_groups.h>
 
 #include "rm_internal.cuh"
+#include "rm_approx.cuh"
 
 namespace rm {
 namespace {
@@ -200,20 +201,6 @@ __device__ __forceinline__ Isect intersect(const float4* __restrict__ q, f3 o, f
 struct Weights {
     float alpha, w0, w1;
 };
-
-// exp(x) for x <= 0 and 1 / x by the approximate instructions alone: __expf and
-// __fdividef add range handling (six instructions each time) for results
-// below 2^-126 and divisors above 2^126, and are equal to these elsewhere.
-__device__ __forceinline__ float exp_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.44269504f));
-    return y;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 // FUSED: the series with fused operations, for gradients.  The forward rounds
 // each product and sum, as it always has: a last bit of the image decides the
@@ -614,16 +601,6 @@ struct EntryResult {
     float a, m1, d4;
     float rgb[3];
 };
-
-// x / 3 correctly rounded for every x >= 0 (one residual correction of the
-// product with the rounded reciprocal; equal to the division on all
-// non-negative floats, checked exhaustively), a third of its instructions.
-__device__ __forceinline__ float third(float x) {
-    const float r3 = 1.0f / 3.0f;
-    const float q = x * r3;
-    const float y = fmaf(fmaf(-3.0f, q, x), r3, q);
-    return x <= 3.402823466e38f ? y : x;
-}
 
 // LOGT: a only (the statistics' walk).
 template <bool LOGT>
@@ -1121,11 +1098,12 @@ __device__ __forceinline__ void fwd_pair_item(int tile, int sub, int quarter, co
 // only lists that many other warps outlast come here (order_kernel).
 //
 // AHEAD: the next block's records are copied while this one is walked, into a
-// second buffer.  Launches of several views take it: 16 views of a million
-// tets 34.8 -> 33.6 ms, 4 views of 250k 3840 -> 3713 us.  One view's launch,
-// whose walks are fewer and shorter, loses more by what the second buffers
-// (110 KB an SM) take from the L1: 1297x840 1041 -> 1065 us, 1920x1080 1496 ->
-// 1530, 640x481 738 -> 752.
+// second buffer.  The batch launches take it, of one view too: 16 views of a
+// million tets 33.6 ms (34.8 without), 4 views of 250k 3713 us (3840), one
+// served view of 1.6M tets at 1297x840 1336 (1374), at 1920x1080 2174 (2225).
+// rm_blend_fwd, whose walks keep what a backward needs, loses more by what the
+// second buffers (110 KB an SM) take from the L1: 1297x840 1041 us (1065 with),
+// 640x481 738 (752).
 template <bool AHEAD>
 struct FwdWarpSmem {
     float4 srec[AHEAD ? 2 : 1][32][kRecFloat4 + 1];  // padded: 32 lanes read one record each without conflicts
