@@ -1484,36 +1484,11 @@ __device__ __forceinline__ void warp_sum_columns(const float* red, int lane, flo
     __syncwarp();
 }
 
-// Rows of hit_grads_planes' output: gl[12..25) and the two planes' normal
-// gradients, stored at the planes' columns (ie, ix: -1 for none or a lane
-// without a hit, whose gl[12..25) are zero).
-// As warp_sum_columns for a warp that walked two entries at once: the rows
-// of the lanes in bal_a go to acc_a, the others to acc_b.
-__device__ __forceinline__ void warp_sum_columns_split(const float* red, int lane, uint32_t bal_a,
-                                                       float* __restrict__ acc_a, float* __restrict__ acc_b) {
-    __syncwarp();
-    if (lane < kNGrad) {
-        float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
-#pragma unroll
-        for (int r = 0; r < 32; r += 2) {
-            const float v0 = red[r * kRedStride + lane], v1 = red[(r + 1) * kRedStride + lane];
-            const bool in0 = (bal_a >> r) & 1u, in1 = (bal_a >> (r + 1)) & 1u;
-            a0 += in0 ? v0 : 0.f;
-            b0 += in0 ? 0.f : v0;
-            a1 += in1 ? v1 : 0.f;
-            b1 += in1 ? 0.f : v1;
-        }
-        const float sa = a0 + a1, sb = b0 + b1;
-        if (sa != 0.f) atomicAdd(acc_a + lane, sa);
-        if (sb != 0.f) atomicAdd(acc_b + lane, sb);
-    }
-    __syncwarp();
-}
-
-// acc_b != nullptr: the rows of the lanes outside bal_a go to acc_b.
+// As warp_sum_columns, from hit_grads_planes' output: gl[12..25) and the two
+// planes' normal gradients, stored at the planes' columns (ie, ix: -1 for none
+// or a lane without a hit, whose gl[12..25) are zero).
 __device__ __forceinline__ void warp_sum_rows_planes(float* __restrict__ red, const float* gl, f3 dne, f3 dnx,
-                                                     int ie, int ix, int lane, float* __restrict__ acc,
-                                                     uint32_t bal_a = 0u, float* __restrict__ acc_b = nullptr) {
+                                                     int ie, int ix, int lane, float* __restrict__ acc) {
     float* rowf = red + lane * kRedStride;
     float4* row = reinterpret_cast<float4*>(rowf);
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1533,10 +1508,7 @@ __device__ __forceinline__ void warp_sum_rows_planes(float* __restrict__ red, co
         rowf[3 * ix + 1] = dnx.y;
         rowf[3 * ix + 2] = dnx.z;
     }
-    if (acc_b)
-        warp_sum_columns_split(red, lane, bal_a, acc, acc_b);
-    else
-        warp_sum_columns(red, lane, acc);
+    warp_sum_columns(red, lane, acc);
 }
 
 // Adjoint of one hit (the Slang autodiff of update_alpha_out,

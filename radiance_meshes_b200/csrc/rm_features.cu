@@ -332,12 +332,22 @@ int launch_features(int deg, const int32_t* indices, const float* vertices, int6
     switch (deg) {
         case 0: RM_FEAT(0, false); break;
         case 1:
-            if (staged) RM_FEAT(1, true);
-            else RM_FEAT(1, false);
+            if constexpr (BWD) {
+                if (staged) {
+                    RM_FEAT(1, true);
+                    break;
+                }
+            }
+            RM_FEAT(1, false);
             break;
         case 2:
-            if (staged) RM_FEAT(2, true);
-            else RM_FEAT(2, false);
+            if constexpr (BWD) {
+                if (staged) {
+                    RM_FEAT(2, true);
+                    break;
+                }
+            }
+            RM_FEAT(2, false);
             break;
         case 3:
             if (staged) RM_FEAT(3, true);
