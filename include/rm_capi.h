@@ -330,8 +330,8 @@ RM_API size_t rm_blend_status_offset(int64_t n_tets, int64_t n_tiles);
 #define RM_BLEND_HEAVY_SHIFT 16
 #define RM_BLEND_PAIR_CTAS_SHIFT 20
 /* flags bits 24..27: log2 of the tets staged per shared-memory batch by the
- * pass's main kernel (forward: the pair items, backward: bulk-copy staging);
- * 4, 5 or 6 (0 = default 32) */
+ * forward's pair items (0 = default 32) or the backward's bulk-copy staging
+ * (0 = default 64; its other kernels have no batch); 4, 5 or 6 */
 #define RM_BLEND_BATCH_SHIFT 24
 
 /*

@@ -20,14 +20,16 @@
 //     walk (log T, termination, distortion moments) is a few adds per entry
 //     by one owner thread per pixel, in the same arithmetic, so results do
 //     not depend on which kind of item ran a tile;
-//   * backward: strips of 64 pixels, one thread per pixel, long lists in
-//     stretches that start from states the forward left (checkpoints).
-// The backward's pair kernel (4 threads per pixel) runs on request only.
+//   * backward: strips of 64 pixels, a warp per half, one pixel per lane, long
+//     lists in stretches that start from states the forward left
+//     (checkpoints).
+// The backward's pair kernel (4 threads per pixel) and its staging by bulk
+// copies run on request only.
 // Per-tet records (128 B, packed once per frame by pack_kernel) are staged in
-// shared memory per block of list entries.  Backward gradients are summed per
-// list entry across the pixels of a CTA (warp sums, then shared-memory
-// atomics) and converted to vertex gradients once per (CTA, entry) before the
-// global atomics.
+// shared memory per block of list entries.  Each backward warp adds up an
+// entry's partials over its pixels; both warps' sums are turned into vertex and
+// cell-value gradients once per (strip, stretch, entry) and added to global
+// memory.
 #include <mutex>
 
 #include <cooperative_groups.h>
@@ -428,7 +430,7 @@ __device__ __forceinline__ HitMasks live_masks(HitMasks hm, int subs, uint32_t s
 // Work queue shared by the kernels of one pass.  order[] lists the tiles
 // heaviest first; info[0] is the number of heavy tiles (the first entries of
 // order[]), which go by pair items, the rest by warp items (forward) or to the
-// dense kernel (backward).
+// kernels that take whole or cut lists (backward).
 struct Queue {
     const int32_t* order;
     const int32_t* info;
@@ -594,8 +596,8 @@ __device__ __forceinline__ void fold_hit(PixelState& st, float a, float m0, floa
     }
 }
 
-// Result of testing one ray against one list entry, in the exact arithmetic of
-// the dense path: a = density * dt (0 for a miss), m1, the D4 increment
+// Result of testing one ray against one list entry, the same for every kind of
+// item: a = density * dt (0 for a miss), m1, the D4 increment
 // density^2 * dt / 3 and the segment colour.
 struct EntryResult {
     float a, m1, d4;
@@ -1232,8 +1234,8 @@ __device__ __forceinline__ void fwd_warp_item(int tile, int sub, int half, const
 
 // 768 threads per SM (80 registers): at 1024 (64 registers) the spills cost
 // more than the warps gain, with the little L1 that the shared memory leaves
-// (1.3M tets, 1297x840: 1461 -> 1293 and 1357 -> 1024 us; a batch of four
-// served views 4187 -> 3500 us).
+// (1.3M tets, 1297x840: 1357 us at 1024, 1024 at 768; a batch of four served
+// views 4187 and 3500).
 template <int PX, int NT, int B, class V, Walk WALK>
 __global__ void __launch_bounds__(NT, 768 / NT) blend_fwd_kernel(
     const int32_t* __restrict__ ids, const int2* __restrict__ ranges, const float4* __restrict__ recs,
@@ -2051,8 +2053,8 @@ __device__ __forceinline__ void bwd_item(
 }
 
 // Dense backward with the records staged by bulk copies (RM_BLEND_STAGE_TMA;
-// 64-pixel items).  The walk and its arithmetic are bwd_dense_item's; what
-// changes is the staging.  Each batch is planned one batch ahead: its hit
+// 64-pixel items): one thread per pixel, whole lists, sums over the CTA by
+// shared-memory atomics (flush_entries).  Each batch is planned one batch ahead: its hit
 // masks are OR-ed over the item, the entries some pixel hit are listed, their
 // tet ids loaded, and warp 0 starts one 128-byte cp.async.bulk per entry
 // (global -> this CTA's shared memory, completing on the buffer's mbarrier).
@@ -3299,12 +3301,12 @@ int blend_bwd_any(const char* who, const int32_t* sorted_ids, const int32_t* ran
         rc = pack(indices, vertices, n_verts, cell_values, n_tets, tiles_touched, w.recs, s);
         if (rc) return rc;
     }
-    // measured: the one-thread-per-pixel backward alone is fastest; its long
-    // lists are cut at the checkpoints, so no tile is heavy unless asked for
+    // no tile is heavy unless asked for: long lists are cut at the checkpoints
+    // (the pair kernel, for all tiles or the longest ones, measured slower)
     Tuning tn = tuning_from_flags(flags, 0, 1);
     tn.n_recs = n_tets;
     if ((rc = pass_status(who, w, status_dev, s, &tn.status))) return rc;
-    // tets per shared-memory batch of the dense kernel: 16, 32 or 64 (default)
+    // tets per shared-memory batch of the bulk-copy staging: 16, 32 or 64 (default)
     const int key = strip_pixels(cam0, flags) * 1000 + batch_size(flags, 64);
 #define RM_BWD_CASE(PX, NT, BD)                                                                                  \
     case PX * 1000 + BD:                                                                                         \
