@@ -292,8 +292,8 @@ RM_API int rm_tile_ranges(const int64_t* sorted_keys, int64_t n, const int64_t* 
 RM_API size_t rm_blend_workspace_size(int64_t n_tets, int64_t n_tiles);
 /* Extra workspace bytes for RM_BLEND_HIT_MASKS over n_pairs list entries in
  * n_tiles tiles of tile_pixels pixels: 4 bytes per 32 entries per pixel for
- * the masks, and 32 bytes per pixel at every 128th entry (512th above 16M
- * entries, 4096th above 64M) for the forward's state there, from which the
+ * the masks, and 32 bytes per pixel at every 128th entry (512th above half a
+ * million entries, 4096th above 64M, and no less than fewer entries need) for the forward's state there, from which the
  * backward takes long lists in independent stretches.  A forward goes by the
  * entries that its lists hold: the first of these distances that they allow and
  * whose states fit, none where not even the last one's do. */

@@ -363,12 +363,16 @@ __device__ __forceinline__ float* ck_at(const HitMasks& hm, int64_t id, int sub,
     return hm.ck + ((id * subs + sub) * kCkFloats) * 64 + p;
 }
 
-// Entries between two checkpoints for lists of n_pairs entries in all: 128,
-// which keeps the longest stretch near 30 us, while their store (16 bytes an
-// entry and strip) stays under 270 MB; 512 up to 64M entries; 4096 (0.5 bytes)
-// for the long lists of many views, whose total work hides a longer stretch.
+// Entries between two checkpoints for lists of n_pairs entries in all: 128
+// where the stretches are what fills the GPU, 512 above half a million entries
+// and 4096 above 64M, where there are enough of them and each one's start (its
+// rays, its state) and each pixel's state are what counts.  Backward, us, at 128
+// and 512: 0.03M entries 87 and 211, 0.28M 188 and 332, 0.44M 284 and 285, 1.3M
+// 514 and 507, 3.9M 1661 and 1614, 13.7M (2% hits) 1166 and 771; at 128, 512
+// and 4096: 115M 8104, 4781 and 3943.
+constexpr int64_t kShortLists = (int64_t)1 << 19, kLongLists = (int64_t)64 << 20;
 __host__ __device__ inline int seg_shift_for(int64_t n_pairs) {
-    return n_pairs <= (int64_t)16 << 20 ? kMinSegShift : n_pairs <= (int64_t)64 << 20 ? 9 : 12;
+    return n_pairs <= kShortLists ? kMinSegShift : n_pairs <= kLongLists ? 9 : 12;
 }
 __host__ __device__ inline int64_t ck_count(int64_t n_pairs, int shift) { return (n_pairs >> shift) + 2; }
 __host__ __device__ inline int64_t ck_words(int64_t n_pairs, int64_t subs, int shift) {
@@ -3340,7 +3344,13 @@ size_t rm_blend_status_offset(int64_t n_tets, int64_t n_tiles) {
 size_t rm_blend_hit_mask_bytes(int64_t n_pairs, int64_t n_tiles, int tile_pixels) {
     const int64_t subs = tile_pixels > 64 ? tile_pixels / 64 : 1;
     const int64_t P = n_pairs > 0 ? n_pairs : 0, G = n_tiles > 0 ? n_tiles : 0;
-    return 256 + (size_t)(rm::mask_word_count(P, G, subs) + rm::ck_words(P, subs, rm::seg_shift_for(P))) * sizeof(uint32_t);
+    // no less than any shorter lists need
+    int64_t words = 0;
+    for (int64_t n : {P < rm::kShortLists ? P : rm::kShortLists, P < rm::kLongLists ? P : rm::kLongLists, P}) {
+        const int64_t w = rm::mask_word_count(n, G, subs) + rm::ck_words(n, subs, rm::seg_shift_for(n));
+        words = w > words ? w : words;
+    }
+    return 256 + (size_t)words * sizeof(uint32_t);
 }
 
 int rm_calc_tet_err(const int32_t* sorted_ids, const int32_t* ranges, const int32_t* indices, const float* vertices,

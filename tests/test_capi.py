@@ -305,3 +305,17 @@ def test_overlapped_sort_passes_read_past_the_read_only_path():
     for name in ("kin", "vin", "kout", "vout"):
         assert re.search(rf"\* {name}\b", params), name  # no __restrict__
         assert f"__ldg({name}" not in kernel
+
+
+@pytest.mark.parametrize("tile_pixels", [64, 256, 1024])
+def test_hit_mask_room_grows_with_the_lists(tile_pixels):
+    """Room for n list entries holds any fewer, whatever the distance of the
+    checkpoints that each number has."""
+    L, G, subs = C.lib(), 1000, tile_pixels // 64
+    sizes = []
+    for n in (0, 1, 1000, 1 << 19, (1 << 19) + 1, 1 << 20, 1 << 24, 64 << 20, (64 << 20) + 1, 1 << 27, 1 << 28):
+        shift = 7 if n <= 1 << 19 else 9 if n <= 64 << 20 else 12
+        need = 256 + 4 * 64 * subs * (n // 32 + G + 2 + 8 * ((n >> shift) + 2))
+        sizes.append(L.rm_blend_hit_mask_bytes(n, G, tile_pixels))
+        assert sizes[-1] >= need
+    assert sizes == sorted(sizes)
